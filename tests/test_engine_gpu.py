@@ -127,6 +127,78 @@ def test_device_sampler_matches_plain_chain():
             assert got[i] == want, (trial, c, u)
 
 
+def _chain64(l, t, k, p, mp):
+    """(ids, cumulative weights) that the draw walks, in float64, and how near a filter's edge was."""
+    ids = np.arange(len(l))
+    l = l.astype(np.float64)
+    near, is_sorted = 1.0, False
+    rank = lambda: np.lexsort((ids, -l))  # noqa: E731
+    if 0 < k < len(l):
+        ids, is_sorted = rank()[:k], True
+    if p < 1.0 and k != 1:
+        ids, is_sorted = (ids if is_sorted else rank()), True
+        w = np.exp(l[ids] - l.max())
+        cum = np.cumsum(w) / w.sum()
+        near = np.abs(cum - p).min()
+        ids = ids[:np.searchsorted(cum, p) + 1]
+    if mp > 0:
+        floor = l.max() + np.log(mp)
+        near = min(near, np.abs(l[ids] - floor).min())
+        ids = ids[l[ids] >= floor]
+    w = np.exp((l[ids] - l.max()) / t)
+    return ids, np.cumsum(w), near
+
+
+@pytest.mark.parametrize("vocab,stride", [(1, 1), (7, 7), (333, 333), (2049, 2052), (8191, 8191),
+                                          (8192, 8192), (8197, 8197), (40961, 40964),
+                                          (151936, 151936)])
+def test_sample_kernel_over_sizes_and_shapes_of_distributions(vocab, stride):
+    """One block below 8,192 logits, a cluster of eight from there; rows whose survivors fit the
+    sorted list and rows whose do not (flat, tied, no filter); rows that are not aligned to 16 bytes;
+    masked tokens (-inf).  Against the chain in float64: the drawn token's stretch of the cumulative
+    weights holds the uniform.  The kernel's 32-bit weights sum to within vocab * 2**-24 of Z in the
+    worst order, and each is within 2**-22 of the true one: 1e-3 * Z is above both."""
+    from llmario_b200 import kernels
+    g = torch.Generator().manual_seed(vocab)
+    options = [(1.0, 0, 1.0, 0.0), (0.7, 40, 0.9, 0.0), (1.0, 40, 0.95, 0.05), (0.8, 0, 1.0, 0.1),
+               (1.3, 0, 0.5, 0.0), (0.9, 0, 0.97, 0.02), (1.0, vocab - 1, 1.0, 0.0),
+               (1.0, 3000, 0.99, 0.0), (30.0, 0, 1.0, 0.0), (1.0, 1, 0.5, 0.0), (0.0, 0, 1.0, 0.0),
+               (0.6, vocab + 3, 0.8, 0.3)]
+    kinds = {"wide": lambda: 2.5 * torch.randn(vocab, generator=g),
+             "flat": lambda: 0.001 * torch.randn(vocab, generator=g),
+             "tied": lambda: torch.randint(-2, 3, (vocab,), generator=g).float(),
+             "peaked": lambda: torch.where(torch.rand(vocab, generator=g) < 20.0 / vocab, 30.0, -30.0)
+             + torch.randn(vocab, generator=g)}
+    rows = []
+    for name, make in kinds.items():
+        for j, o in enumerate(options):
+            l = make()
+            if j % 3 == 1:
+                l[torch.rand(vocab, generator=g) < 0.5] = -float("inf")
+                l[vocab // 2] = 3.0
+            rows.append((name, o, l))
+    n = len(rows)
+    wide = torch.full((n, stride), float("nan"))
+    wide[:, :vocab] = torch.stack([r[2] for r in rows])
+    u = torch.rand(n, generator=g, dtype=torch.float64)
+    col = lambda i, dt: torch.tensor([r[1][i] for r in rows], dtype=dt, device=DEV)  # noqa: E731
+    out = torch.full((n,), -7, dtype=torch.int32, device=DEV)
+    kernels.sample(wide.to(DEV)[:, :vocab], col(0, torch.float32), col(1, torch.int32),
+                   col(2, torch.float32), col(3, torch.float32), u.to(DEV), out)
+    for (name, (t, k, p, mp), l), ui, got in zip(rows, u.tolist(), out.tolist()):
+        l = l.numpy()
+        if t == 0.0:
+            assert got == int(np.argmax(l)), (name, t, k, p, mp)
+            continue
+        ids, cum, near = _chain64(l, t, k, p, mp)
+        if near < 1e-5:
+            continue          # a filter's edge lies within the rounding of 32-bit sums
+        at = np.flatnonzero(ids == got)
+        assert len(at) == 1, (name, t, k, p, mp, got)
+        lo, hi = (cum[at[0] - 1] if at[0] else 0.0), cum[at[0]]
+        assert lo - 1e-3 * cum[-1] <= ui * cum[-1] <= hi + 1e-3 * cum[-1], (name, t, k, p, mp)
+
+
 def test_device_sampler_penalties_and_streams():
     from llmario_b200.sampling import DeviceSampler, RequestSampler, SamplingParams
     V = 64
