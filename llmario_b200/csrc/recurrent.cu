@@ -11,8 +11,9 @@
 // Everything here is 32-bit: the inputs are the 32-bit results of the projections, the state
 // lives in 32-bit floats in the request's state slot, decays and step sizes are made here from
 // the projected values.  The tokens of a request are visited one after the other and every sum
-// has a fixed order, so the result for a token is the same bits however the prompt was cut into
-// steps and whatever else is in the batch.
+// has a fixed order.  The diagonal recurrence cuts long portions into runs that are walked at the
+// same time (recurrence_runs_kernel), so how a prompt was cut into steps changes a token's result by
+// the rounding of 32-bit sums; the other recurrences, and its short portions, give the same bits.
 //
 // Which rows of a step belong to which request is read on the device: either every row is a
 // request of its own (`single`: slot = row_slot[row]), or a table of (first row, end row) per
@@ -79,6 +80,9 @@ struct ScanArgs {
   // `unit`: q and k of every head are divided by sqrt(sum of squares + unit_floor) first
   const float* beta; int beta_stride;
   int unit; float unit_floor;
+  int parts, part_rows;                  // runs a request's rows are cut into, and their length
+  float* part_state;                     // [request of the step][run][H][V][K]
+  float* part_decay;                     // [request of the step][run][H][K] (one number with a scalar decay)
   int tail_only;        // only the last (rows of the request) % 4 rows: the others went in groups of four
 };
 
@@ -384,6 +388,324 @@ __global__ void __launch_bounds__(SCAN_THREADS) linear_recurrence_kernel(const S
       }
     }
   }
+}
+
+
+// ---- long portions in runs.  The walk above is one chain per block: a token's shared-memory reads
+// and shuffles, some 450 cycles, with one or two warps per scheduler (a prompt of 2,048 tokens on 4
+// heads of 128 x 256: 64 blocks on 148 SMs, 436 us; on 32 heads of 128 x 64 492 us).  The recurrence is a
+// diagonal map, so a portion can be cut into runs of part_rows that are walked at the same time:
+//   FOLD    each run but the last from a zero state, no outputs: what the run adds to the state,
+//           and the product of its decays;
+//   carry   (scan_carry_kernel) the states that enter the runs, one after the other;
+//   RUNS    each run from the state that enters it; the last one leaves the request's state.
+// That is half as much arithmetic again, but warps enough to hide the chain: 124 and 228 us.  What is
+// left goes to issue slots and latencies, hence eight columns per lane in place of four (q, k and
+// the decay are read from shared memory once for thirty-two state elements, nine shuffles for
+// eight outputs; with four columns 134 and 253 us), and multiply-adds on pairs (fma.rn.f32x2: rows
+// e and e + 1 of a column, which lie as the reads leave them; the values stand twice in shared memory).
+typedef unsigned long long pair_f32;
+__device__ __forceinline__ pair_f32 pair_fma(pair_f32 a, pair_f32 b, pair_f32 c) {
+  pair_f32 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ pair_f32 pair_mul(pair_f32 a, pair_f32 b) {
+  pair_f32 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ pair_f32 pair_of(float lo, float hi) {
+  return (pair_f32)__float_as_uint(lo) | ((pair_f32)__float_as_uint(hi) << 32);
+}
+__device__ __forceinline__ float pair_lo(pair_f32 v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float pair_hi(pair_f32 v) { return __uint_as_float((uint32_t)(v >> 32)); }
+
+constexpr int RUN_COLS = 8;      // columns per lane
+
+template <int L, int NF, bool VEC, bool FOLD>
+__global__ void __launch_bounds__(SCAN_THREADS) recurrence_runs_kernel(const ScanArgs a) {
+  constexpr int KP = 4 * L * NF;                                 // key channels, padded
+  constexpr int GROUPS = 32 / L;                                 // column groups of a warp
+  constexpr int COLS = RUN_COLS * GROUPS * (SCAN_THREADS / 32);  // value channels of a block
+  constexpr int TC = KP >= 256 ? 4 : (KP >= 128 ? 8 : 16);       // tokens of a chunk
+  __shared__ __align__(16) float q_s[FOLD ? 1 : 2][FOLD ? 1 : TC][FOLD ? 4 : KP];
+  __shared__ __align__(16) float k_s[2][TC][KP];
+  __shared__ __align__(16) float a_s[2][VEC ? TC : 1][VEC ? KP : 4];
+  __shared__ __align__(16) float v_s[2][TC][COLS][2];            // every value twice
+  __shared__ float d_s[2][TC];          // scalar decay: its argument, then the decay itself
+  __shared__ float w_s[2][TC];          // the weight of the values: the input weight, the step
+  pdl_trigger();
+  pdl_wait();
+  const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int request = blockIdx.x / a.parts, run = blockIdx.x - request * a.parts;
+  const int slot = a.seg[SEG * request + 2];
+  if (slot < 0) return;
+  const int first = a.seg[SEG * slot] + run * a.part_rows;
+  int end = a.seg[SEG * slot + 1];
+  if (end <= first) return;
+  const bool last_run = end - first <= a.part_rows;
+  if (FOLD && last_run) return;
+  if (!last_run) end = first + a.part_rows;
+  const int K = a.K, V = a.V, g = h / (a.H / a.G);
+  const int j0 = blockIdx.z * COLS;
+  const int li = lane % L;
+  const int c0 = (warp * GROUPS + lane / L) * RUN_COLS, jc = j0 + c0;     // this lane's eight columns
+  float* const part = a.part_state + ((size_t)blockIdx.x * a.H + h) * V * K;
+  float* const send = FOLD ? part : a.state + (size_t)slot * a.state_stride + (size_t)h * V * K;
+  const bool k4 = (K & 3) == 0 && (((uintptr_t)part | (uintptr_t)send) & 15) == 0;
+
+  // key channels beyond K: they hold nothing and must stay that way
+  for (int idx = tid; idx < 2 * TC * (KP - K); idx += SCAN_THREADS) {
+    const int st = idx / (TC * (KP - K)), rem = idx - st * TC * (KP - K);
+    const int tt = rem / (KP - K), i = K + rem - tt * (KP - K);
+    if (!FOLD) q_s[st][tt][i] = 0.f;
+    k_s[st][tt][i] = 0.f;
+    if (VEC) a_s[st][tt][i] = 1.f;
+  }
+  const bool wide = (K & 3) == 0 && !((a.q_stride | a.k_stride | (VEC ? a.d_stride : 0)) & 3) &&
+                    !(((uintptr_t)(a.q + g * K) | (uintptr_t)(a.k + g * K) |
+                       (VEC ? (uintptr_t)(a.d + h * K) : 0)) & 15);
+  auto fetch = [&](int st, int t0) {
+    const int n_tok = min(TC, end - t0);
+    if (wide) {
+      const int k4n = K >> 2;
+      for (int idx = tid; idx < n_tok * k4n; idx += SCAN_THREADS) {
+        const int tt = idx / k4n, i = (idx - tt * k4n) << 2;
+        const size_t row = (size_t)(t0 + tt);
+        if (!FOLD) cp_async16(&q_s[st][tt][i], a.q + row * a.q_stride + g * K + i);
+        cp_async16(&k_s[st][tt][i], a.k + row * a.k_stride + g * K + i);
+        if (VEC) cp_async16(&a_s[st][tt][i], a.d + row * a.d_stride + h * K + i);
+      }
+    } else {
+      for (int idx = tid; idx < n_tok * K; idx += SCAN_THREADS) {
+        const int tt = idx / K, i = idx - tt * K;
+        const size_t row = (size_t)(t0 + tt);
+        if (!FOLD) cp_async4(&q_s[st][tt][i], a.q + row * a.q_stride + g * K + i);
+        cp_async4(&k_s[st][tt][i], a.k + row * a.k_stride + g * K + i);
+        if (VEC) cp_async4(&a_s[st][tt][i], a.d + row * a.d_stride + h * K + i);
+      }
+    }
+    for (int idx = tid; idx < n_tok * COLS; idx += SCAN_THREADS) {
+      const int tt = idx / COLS, cc = idx - tt * COLS;
+      if (j0 + cc < a.v_cols) {
+        const float* src = a.v + (size_t)(t0 + tt) * a.v_stride + h * a.v_cols + j0 + cc;
+        cp_async4(&v_s[st][tt][cc][0], src);
+        cp_async4(&v_s[st][tt][cc][1], src);
+      } else {
+        v_s[st][tt][cc][0] = v_s[st][tt][cc][1] = (a.ones && j0 + cc == V - 1) ? 1.f : 0.f;
+      }
+    }
+    if (!VEC)
+      for (int tt = tid; tt < n_tok; tt += SCAN_THREADS) {
+        cp_async4(&d_s[st][tt], a.d + (size_t)(t0 + tt) * a.d_stride + h);
+        if (a.kind == DECAY_SCALAR_INPUT) cp_async4(&w_s[st][tt], a.d2 + (size_t)(t0 + tt) * a.d_stride + h);
+      }
+    cp_async_commit();
+  };
+
+  fetch(0, first);
+  pair_f32 s[NF][2][RUN_COLS];       // [n][rows 2 r, 2 r + 1][column]
+#pragma unroll
+  for (int c = 0; c < RUN_COLS; ++c) {
+    const bool live = !FOLD && jc + c < V;
+    const float* srow = part + (size_t)(live ? jc + c : 0) * K;
+#pragma unroll
+    for (int n = 0; n < NF; ++n) {
+      const int i0 = 4 * (li + L * n);
+      float t[4];
+      if (live && k4 && i0 + 3 < K) {
+        const float4 f = *reinterpret_cast<const float4*>(srow + i0);
+        t[0] = f.x, t[1] = f.y, t[2] = f.z, t[3] = f.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) t[e] = (live && i0 + e < K) ? srow[i0 + e] : 0.f;
+      }
+      s[n][0][c] = pair_of(t[0], t[1]), s[n][1][c] = pair_of(t[2], t[3]);
+    }
+  }
+  pair_f32 through[VEC ? NF : 1][2];      // FOLD: the product of the run's decays
+#pragma unroll
+  for (int n = 0; n < (VEC ? NF : 1); ++n) through[n][0] = through[n][1] = pair_of(1.f, 1.f);
+
+  const float rate = a.kind == DECAY_RATE_STEP ? expf(a.p0[h]) : 0.f;
+  const float bias = a.kind == DECAY_RATE_STEP ? a.p1[h] : 0.f;
+  const float q_scale = a.q_scale;
+  const bool up1 = (li & (L / 2)) != 0, up2 = (li & (L / 4)) != 0, up3 = (li & (L / 8)) != 0;
+  const int my_col = jc + 4 * (up1 ? 1 : 0) + 2 * (up2 ? 1 : 0) + (up3 ? 1 : 0);
+  const bool writer = (li & (L / 8 - 1)) == 0 && my_col < V;
+  int st = 0;
+  for (int t0 = first; t0 < end; t0 += TC, st ^= 1) {
+    const int n_tok = min(TC, end - t0);
+    if (t0 + TC < end) {
+      fetch(st ^ 1, t0 + TC);       // (its stage was walked two chunks ago; a barrier lies between)
+      cp_async_wait<1>();
+    } else {
+      cp_async_wait<0>();
+    }
+    __syncthreads();
+    // ---- the decay from its argument and the values' weights, once per token
+    float* v_flat = &v_s[st][0][0][0];
+    if (VEC) {
+      if (a.kind == DECAY_SIGMOID_POW)
+        for (int idx = tid; idx < n_tok * K; idx += SCAN_THREADS) {
+          const int tt = idx / K, i = idx - tt * K;
+          a_s[st][tt][i] = expf(-a.c * softplus_f(-a_s[st][tt][i]));
+        }
+    } else if (a.kind == DECAY_SCALAR_INPUT) {
+      for (int idx = tid; idx < n_tok * COLS * 2; idx += SCAN_THREADS) v_flat[idx] *= w_s[st][idx / (COLS * 2)];
+    } else {
+      for (int tt = tid; tt < n_tok; tt += SCAN_THREADS) {
+        const float step = softplus_f(d_s[st][tt] + bias);
+        w_s[st][tt] = step;
+        d_s[st][tt] = expf(-rate * step);
+      }
+      __syncthreads();
+      for (int idx = tid; idx < n_tok * COLS * 2; idx += SCAN_THREADS) v_flat[idx] *= w_s[st][idx / (COLS * 2)];
+    }
+    __syncthreads();
+    // ---- the tokens of the chunk, one after the other
+#pragma unroll 2
+    for (int tt = 0; tt < n_tok; ++tt) {
+      pair_f32 vv[RUN_COLS], acc[RUN_COLS];
+#pragma unroll
+      for (int c = 0; c < RUN_COLS; c += 2) {
+        const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(&v_s[st][tt][c0 + c][0]);
+        vv[c] = t.x, vv[c + 1] = t.y;
+      }
+#pragma unroll
+      for (int c = 0; c < RUN_COLS; ++c) acc[c] = 0ull;
+      const float a1 = VEC ? 1.f : d_s[st][tt];
+      if (FOLD && !VEC) through[0][0] = pair_mul(through[0][0], pair_of(a1, a1));
+#pragma unroll
+      for (int n = 0; n < NF; ++n) {
+        const ulonglong2 kk = *reinterpret_cast<const ulonglong2*>(&k_s[st][tt][4 * (li + L * n)]);
+        ulonglong2 aa, qq = make_ulonglong2(0ull, 0ull);
+        if (VEC) aa = *reinterpret_cast<const ulonglong2*>(&a_s[st][tt][4 * (li + L * n)]);
+        else aa.x = aa.y = pair_of(a1, a1);
+        if (!FOLD) qq = *reinterpret_cast<const ulonglong2*>(&q_s[st][tt][4 * (li + L * n)]);
+        if (FOLD && VEC) {
+          through[VEC ? n : 0][0] = pair_mul(through[VEC ? n : 0][0], aa.x);
+          through[VEC ? n : 0][1] = pair_mul(through[VEC ? n : 0][1], aa.y);
+        }
+#pragma unroll
+        for (int c = 0; c < RUN_COLS; ++c) {
+          s[n][0][c] = pair_fma(aa.x, s[n][0][c], pair_mul(kk.x, vv[c]));
+          s[n][1][c] = pair_fma(aa.y, s[n][1][c], pair_mul(kk.y, vv[c]));
+          if (!FOLD) {
+            acc[c] = pair_fma(s[n][0][c], qq.x, acc[c]);
+            acc[c] = pair_fma(s[n][1][c], qq.y, acc[c]);
+          }
+        }
+      }
+      if (FOLD) continue;
+      // sum over the L lanes of the group: hand four columns to the partner, then two, then one,
+      // then a plain butterfly over what is left
+      float o8[8], o4[4], o2[2];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) o8[c] = pair_lo(acc[c]) + pair_hi(acc[c]);
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        o4[c] = (up1 ? o8[4 + c] : o8[c]) + __shfl_xor_sync(0xffffffffu, up1 ? o8[c] : o8[4 + c], L / 2);
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+        o2[c] = (up2 ? o4[2 + c] : o4[c]) + __shfl_xor_sync(0xffffffffu, up2 ? o4[c] : o4[2 + c], L / 4);
+      float sum = (up3 ? o2[1] : o2[0]) + __shfl_xor_sync(0xffffffffu, up3 ? o2[0] : o2[1], L / 8);
+#pragma unroll
+      for (int o = L / 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (writer) a.out[(size_t)(t0 + tt) * a.out_stride + h * V + my_col] = sum * q_scale;
+    }
+    __syncthreads();
+  }
+  if (FOLD && blockIdx.z == 0 && warp == 0 && lane < L) {
+    float* to = a.part_decay + ((size_t)blockIdx.x * a.H + h) * (VEC ? K : 1);
+    if (!VEC) {
+      if (lane == 0) to[0] = pair_lo(through[0][0]);
+    } else {
+#pragma unroll
+      for (int n = 0; n < NF; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const pair_f32 t = through[VEC ? n : 0][e >> 1];
+          if (4 * (li + L * n) + e < K) to[4 * (li + L * n) + e] = e & 1 ? pair_hi(t) : pair_lo(t);
+        }
+    }
+  }
+  if (!FOLD && !last_run) return;
+#pragma unroll
+  for (int c = 0; c < RUN_COLS; ++c) {
+    if (jc + c >= V) continue;
+    float* srow = send + (size_t)(jc + c) * K;
+#pragma unroll
+    for (int n = 0; n < NF; ++n) {
+      const int i0 = 4 * (li + L * n);
+      const float t[4] = {pair_lo(s[n][0][c]), pair_hi(s[n][0][c]), pair_lo(s[n][1][c]), pair_hi(s[n][1][c])};
+      if (k4 && i0 + 3 < K) {
+        *reinterpret_cast<float4*>(srow + i0) = make_float4(t[0], t[1], t[2], t[3]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (i0 + e < K) srow[i0 + e] = t[e];
+      }
+    }
+  }
+}
+
+// The states that enter the runs of a request, in place of what the runs add: a thread per state
+// element walks the runs.
+__global__ void __launch_bounds__(256) scan_carry_kernel(const ScanArgs a, int per_channel) {
+  pdl_trigger();
+  pdl_wait();
+  const int slot = a.seg[SEG * blockIdx.y + 2];
+  if (slot < 0) return;
+  const int rows = a.seg[SEG * slot + 1] - a.seg[SEG * slot];
+  const int runs = (rows + a.part_rows - 1) / a.part_rows;
+  const long long size = (long long)a.H * a.V * a.K;
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= size) return;
+  const int h = (int)(i / ((long long)a.V * a.K)), ch = (int)(i % a.K);
+  float s = a.state[(size_t)slot * a.state_stride + i];
+  float* part = a.part_state + (size_t)blockIdx.y * a.parts * size + i;
+  const float* decay = per_channel ? a.part_decay + ((size_t)blockIdx.y * a.parts * a.H + h) * a.K + ch
+                                   : a.part_decay + (size_t)blockIdx.y * a.parts * a.H + h;
+  const size_t step = (size_t)a.H * (per_channel ? a.K : 1);
+  for (int r = 0; r < runs; r += 4) {      // four runs' loads are under way together
+    float add[4], keep[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      add[j] = 0.f, keep[j] = 0.f;
+      if (r + j + 1 < runs) add[j] = part[(size_t)(r + j) * size], keep[j] = decay[(size_t)(r + j) * step];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (r + j < runs) {
+        part[(size_t)(r + j) * size] = s;
+        s = fmaf(keep[j], s, add[j]);
+      }
+  }
+}
+
+template <int L, int NF, bool VEC>
+int launch_runs(const ScanArgs& a, int n_requests, cudaStream_t stream) {
+  constexpr int COLS = RUN_COLS * (32 / L) * (SCAN_THREADS / 32);
+  const dim3 grid(n_requests * a.parts, a.H, (a.V + COLS - 1) / COLS);
+  int rc = launch_pdl(recurrence_runs_kernel<L, NF, VEC, true>, grid, SCAN_THREADS, 0, stream, a);
+  if (rc) return rc;
+  next_launch_plain();      // (blocks that wait would take the fold's places)
+  const long long size = (long long)a.H * a.V * a.K;
+  rc = launch_pdl(scan_carry_kernel, dim3((unsigned)((size + 255) / 256), n_requests), 256, 0, stream, a, (int)VEC);
+  if (rc) return rc;
+  return launch_pdl(recurrence_runs_kernel<L, NF, VEC, false>, grid, SCAN_THREADS, 0, stream, a);
+}
+
+static int run_in_runs(const ScanArgs& a, int n_requests, cudaStream_t stream) {
+  const bool scalar = a.kind == DECAY_RATE_STEP || a.kind == DECAY_SCALAR_INPUT;
+#define RUNS(L, NF) return scalar ? launch_runs<L, NF, false>(a, n_requests, stream) : launch_runs<L, NF, true>(a, n_requests, stream)
+  if (a.K <= 32) RUNS(8, 1);
+  if (a.K <= 64) RUNS(16, 1);
+  if (a.K <= 128) RUNS(32, 1);
+  RUNS(32, 2);
+#undef RUNS
 }
 
 template <int L, int NF>
@@ -1093,13 +1415,17 @@ static int run_scan(ScanArgs& a, int rows, int n_requests, cudaStream_t stream) 
 // channel fastest.  `ones`: v has V - 1 channels per head and the state's last column is fed the
 // constant 1, so that it holds the decayed sum of the keys alone and the last output channel is
 // its product with the query (the normaliser of a matrix memory).
+// parts > 1 (K up to 256): every request's rows are cut into runs of part_rows, at most `parts` of
+// them, which are walked at the same time; `work` holds n_requests * parts * H * (V + 1) * K floats.
 LLM_EXPORT int llm_linear_recurrence(const float* q, int q_stride, const float* k, int k_stride, const float* v,
                                      int v_stride, const float* d, int d_stride, const float* d2, int ones,
                                      const float* p0, const float* p1, float c, float q_scale, float* state,
                                      long long state_stride, float* out, int out_stride, const int* seg,
                                      const int* row_slot, int rows, int n_requests, int single, int H, int G,
-                                     int K, int V, int kind, cudaStream_t stream) {
+                                     int K, int V, int kind, int parts, int part_rows, float* work,
+                                     cudaStream_t stream) {
   if (rows <= 0) return 0;
+  if (parts > 1 && (single || !work || part_rows <= 0 || n_requests > 65535 || K > 256)) return LLM_ERR_ARGUMENT;
   if (H <= 0 || G <= 0 || H % G || K <= 0 || V <= 0 || kind < 0 || kind > 3) return LLM_ERR_ARGUMENT;
   if (kind == DECAY_RATE_STEP && (!p0 || !p1)) return LLM_ERR_ARGUMENT;
   if (kind == DECAY_SCALAR_INPUT && !d2) return LLM_ERR_ARGUMENT;
@@ -1114,7 +1440,9 @@ LLM_EXPORT int llm_linear_recurrence(const float* q, int q_stride, const float* 
   a.seg = seg, a.row_slot = row_slot;
   a.single = single, a.H = H, a.G = G, a.K = K, a.V = V, a.kind = kind;
   a.beta = nullptr, a.beta_stride = 0, a.unit = 0, a.unit_floor = 0.f, a.tail_only = 0;
-  const int rc = run_scan(a, rows, n_requests, stream);
+  a.parts = parts > 1 ? parts : 1, a.part_rows = part_rows, a.part_state = work;
+  a.part_decay = parts > 1 ? work + (size_t)n_requests * parts * H * V * K : nullptr;
+  const int rc = parts > 1 ? run_in_runs(a, n_requests, stream) : run_scan(a, rows, n_requests, stream);
   if (!single) next_launch_plain();      // (whatever follows the walk of a portion)
   return rc;
 }
@@ -1149,6 +1477,7 @@ LLM_EXPORT int llm_delta_recurrence_grouped(const float* q, int q_stride, const 
   a.seg = seg, a.row_slot = row_slot;
   a.single = single, a.H = H, a.G = G, a.K = K, a.V = V, a.kind = kind;
   a.beta = beta, a.beta_stride = beta_stride, a.unit = unit ? 1 : 0, a.unit_floor = unit_floor, a.tail_only = 0;
+  a.parts = 1, a.part_rows = 0, a.part_state = a.part_decay = nullptr;
   // Portions of prompts with 68 to 256 key channels go four tokens at a time: what a group needs
   // is prepared once per head in parallel over the tokens, the walk takes a group per round, and
   // the token-by-token kernel takes the rows that are left (fewer than four a request).

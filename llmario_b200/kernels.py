@@ -98,7 +98,7 @@ def _signatures():
         "llm_segment_table": [P, I, P, I, P],
         "llm_bias_sigmoid_pow": [P, P, I, I, F, P],
         "llm_linear_recurrence": [P, I, P, I, P, I, P, I, P, I, P, P, F, F, P, L, P, I, P, P, I, I,
-                                  I, I, I, I, I, I, P],
+                                  I, I, I, I, I, I, I, I, P, P],
         "llm_log_gate_scan": [P, P, I, P, P, F, P, L, P, I, P, P, I, I, I, I, P],
         "llm_memory_out_norm": [P, I, P, I, P, I, P, P, I, I, I, I, I, F, F, P],
         "llm_stream_step": [P, L, I, P, P, P, I, I, P, P, F, P, I, P, I, I, P],
@@ -495,7 +495,8 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, d: torc
                       value_dim: int, kind: int, q_scale: float = 1.0, exponent: float = 1.0,
                       rate_log: Optional[torch.Tensor] = None,
                       step_bias: Optional[torch.Tensor] = None, n_requests: int = 0,
-                      input_weight: Optional[torch.Tensor] = None, ones: bool = False) -> None:
+                      input_weight: Optional[torch.Tensor] = None, ones: bool = False,
+                      work: Optional[torch.Tensor] = None) -> None:
     """Per request and head ``S <- diag(a_t) S + k_t v_t^T``, ``o_t = S^T (q_scale q_t)`` over
     the rows of the step in order.  q, k float32 [rows, groups * key_dim], v and out float32
     [rows, heads * value_dim] (column slices of wider matrices are fine); head h uses group
@@ -510,20 +511,60 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, d: torc
     holds the decayed sum of the keys, and the last output channel its product with q).
     ``seg``: the table of :func:`segment_table` with ``n_requests`` the
     number of requests that have rows in the step, or None when every row is a request of its
-    own."""
-    _cuda(q, k, v, d, state, out, row_slot, seg, rate_log, step_bias, input_weight)
+    own.  ``work`` (float32, at least :func:`recurrence_work_floats` elements): room for the
+    states between the runs that :func:`recurrence_runs` cuts long portions into; without it
+    every portion is walked as a whole.  The two ways differ by rounding only."""
+    _cuda(q, k, v, d, state, out, row_slot, seg, rate_log, step_bias, input_weight, work)
+    assert work is None or (work.dtype == torch.float32 and work.is_contiguous())
     for t in (q, k, v, d, state, out):
         assert t.dtype == torch.float32 and t.stride(-1) == 1
     rows = out.shape[0]
     assert state.dim() == 2 and state.shape[1] >= heads * value_dim * key_dim
     if input_weight is not None:
         assert input_weight.dtype == torch.float32 and input_weight.stride(0) == d.stride(0)
+    parts, part_rows = 1, 0
+    if work is not None and seg is not None:
+        parts, part_rows = recurrence_runs(rows, n_requests, heads, key_dim, value_dim)
+        need = recurrence_work_floats(rows, n_requests, heads, key_dim, value_dim)
+        if work.numel() < need:
+            raise KernelError(f"linear_recurrence: {need} floats of work are needed, "
+                              f"{work.numel()} given")
     _check(lib().llm_linear_recurrence(
         _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(d), d.stride(0),
         _ptr(input_weight), int(ones), _ptr(rate_log), _ptr(step_bias), float(exponent), float(q_scale), _ptr(state),
         state.stride(0), _ptr(out), out.stride(0), _ptr(seg), _ptr(row_slot), rows,
-        int(n_requests), int(seg is None), heads, groups, key_dim, value_dim, kind, _stream()),
+        int(n_requests), int(seg is None), heads, groups, key_dim, value_dim, kind, parts,
+        part_rows, _ptr(work) if parts > 1 else None, _stream()),
         f"linear_recurrence (key_dim {key_dim})")
+    global launches
+    launches += 2 * int(parts > 1)      # the folds and the states between the runs
+
+
+def recurrence_runs(rows: int, n_requests: int, heads: int, key_dim: int,
+                    value_dim: int) -> Tuple[int, int]:
+    """Into how many runs of how many rows the portions of a step's requests are cut for
+    :func:`linear_recurrence`, (1, 0) for none.  A block of the runs has 128, 64 or 32 value
+    channels of a head; portions are cut so that about 2,000 blocks run (three to four rounds).
+    The runs cost half as much arithmetic again: with up to 64 blocks to the whole walk (one or
+    two warps per scheduler) they pay from 192 rows a request on (4 heads of 128 x 256, 192 / 512 /
+    2,048 rows: 47 / 115 / 436 -> 42 / 50 / 124 us; 32 heads of 128 x 64: 53 / 129 / 492 -> 50 / 81 / 228),
+    with up to 128 from 1,024 rows on (16 heads of 128 x 256, 512 / 1,024 / 2,048 rows: 136 / 265 / 522
+    -> 130 / 218 / 402), beyond that not (128 heads of 128 x 64, 2,048 rows: 739 -> 775)."""
+    columns = 128 if key_dim <= 32 else 64 if key_dim <= 64 else 32
+    blocks = max(1, n_requests) * heads * -(-value_dim // columns)
+    if key_dim > 256 or blocks > 128 or rows < (192 if blocks <= 64 else 1024) * n_requests:
+        return 1, 0
+    parts = min(32, -(-2000 // blocks))
+    part_rows = max(32, -(-rows // (16 * parts)) * 16)
+    return -(-rows // part_rows), part_rows
+
+
+def recurrence_work_floats(rows: int, n_requests: int, heads: int, key_dim: int,
+                           value_dim: int) -> int:
+    """Elements of ``work`` with which :func:`linear_recurrence` cuts portions into runs, 0 when
+    it would not cut them."""
+    parts, _ = recurrence_runs(rows, n_requests, heads, key_dim, value_dim)
+    return n_requests * parts * heads * (value_dim + 1) * key_dim if parts > 1 else 0
 
 
 def bias_sigmoid_pow(z: torch.Tensor, bias: Optional[torch.Tensor], exponent: float) -> None:

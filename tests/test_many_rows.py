@@ -3,6 +3,8 @@ wrong, against float64 statements and against the kernels for few rows."""
 import pytest
 import torch
 
+from llmario_b200.kernels import recurrence_runs, recurrence_work_floats
+
 gpu = pytest.mark.gpu
 DEV = "cuda:0"
 
@@ -38,3 +40,87 @@ def test_gemm_float32(M, N, K, pad, accumulate):
             few = c0[:rows].clone()
             kernels.gemm_simt(a[:rows], w, few, accumulate)
             assert torch.equal(few, out[:rows])
+
+
+def test_runs_cover_the_rows_and_fit_their_work():
+    for rows in (1, 100, 192, 193, 1000, 2048, 8191):
+        for n in (1, 2, 7, 40):
+            for H, K, V in ((4, 128, 256), (32, 128, 64), (1, 30, 7), (16, 250, 33)):
+                parts, run = recurrence_runs(rows, n, H, K, V)
+                floats = recurrence_work_floats(rows, n, H, K, V)
+                if parts == 1:
+                    assert floats == 0
+                else:
+                    assert parts * run >= rows and (parts - 1) * run < rows and run % 16 == 0
+                    assert floats == n * parts * H * (V + 1) * K and floats < 2 ** 27
+
+
+@gpu
+@pytest.mark.parametrize("H,G,K,V,lengths", [(2, 1, 128, 64, [2048]), (4, 4, 128, 256, [193]), (3, 3, 30, 7, [500, 3, 1, 290]),
+                                             (2, 2, 72, 20, [96, 480]), (1, 1, 256, 16, [320, 64]),
+                                             (2, 1, 200, 40, [288, 111])])
+@pytest.mark.parametrize("kind", (0, 1, 2, 3))
+def test_recurrence_in_runs(kind, H, G, K, V, lengths):
+    """Long portions in runs against the formula in float64 and against the whole walk, states that
+    carry on from an earlier step, requests that end in their first run."""
+    from llmario_b200 import kernels
+    if kind in (0, 1) and G != H:
+        G = H
+    rows, n_slots = sum(lengths), len(lengths) + 2
+    assert recurrence_runs(rows, len(lengths), H, K, V)[0] > 1
+    slots = list(range(n_slots - 1, n_slots - 1 - len(lengths), -1))
+    row_slot = torch.tensor(sum(([s] * n for s, n in zip(slots, lengths)), []), dtype=torch.int32, device=DEV)
+    seg = torch.empty(n_slots, 3, dtype=torch.int32, device=DEV)
+    kernels.segment_table(row_slot, seg)
+    q, k, v = rnd(rows, G * K, seed=1), rnd(rows, G * K, seed=2, scale=0.3), rnd(rows, H * V - (H if kind == 3 else 0), seed=3)
+    d = rnd(rows, H if kind >= 2 else H * K, seed=4) + 2
+    d2 = None
+    if kind in (0, 3):
+        d = torch.sigmoid(d + 2)
+    if kind == 3:
+        d2 = rnd(rows, H, seed=5).abs()
+    p0, p1 = rnd(H, seed=6) - 2, rnd(H, seed=7)
+    start = rnd(n_slots, H * V * K + 3, seed=8)
+
+    def go(work):
+        state = start.clone()
+        out = torch.full((rows, H * V), float("nan"), device=DEV)
+        kernels.linear_recurrence(q, k, v, d, state, out, row_slot, seg, H, G, K, V, kind, q_scale=0.5, exponent=0.25,
+                                  rate_log=p0, step_bias=p1, n_requests=len(lengths), input_weight=d2, ones=kind == 3,
+                                  work=work)
+        return state, out
+
+    work = torch.full((recurrence_work_floats(rows, len(lengths), H, K, V),), float("nan"), device=DEV)
+    state, out = go(work)
+    state_w, out_w = go(None)
+    S = start[:, :H * V * K].double().view(n_slots, H, V, K).clone()
+    ref = torch.zeros(rows, H, V, dtype=torch.float64, device=DEV)
+    vd = v.double().view(rows, H, -1)
+    if kind == 3:
+        vd = torch.cat([vd, torch.ones(rows, H, 1, dtype=torch.float64, device=DEV)], -1) * d2.double()[..., None]
+    if kind == 2:
+        dt = torch.nn.functional.softplus(d.double() + p1.double())
+        a = torch.exp(-torch.exp(p0.double()) * dt)[..., None].expand(rows, H, K)
+        vd = vd * dt[..., None]
+    elif kind == 3:
+        a = d.double()[..., None].expand(rows, H, K)
+    else:
+        a = d.double().view(rows, H, K)
+        if kind == 1:
+            a = torch.sigmoid(a) ** 0.25
+    kd = k.double().view(rows, G, K).repeat_interleave(H // G, 1)
+    qd = 0.5 * q.double().view(rows, G, K).repeat_interleave(H // G, 1)
+    r = 0
+    for s, n in zip(slots, lengths):
+        for _ in range(n):
+            S[s] = S[s] * a[r][:, None, :] + vd[r][:, :, None] * kd[r][:, None, :]
+            ref[r] = (S[s] * qd[r][:, None, :]).sum(-1)
+            r += 1
+    err = lambda x, y: float((x.double() - y).norm() / y.norm())  # noqa: E731
+    e_out, e_whole = err(out, ref.view(rows, -1)), err(out_w, ref.view(rows, -1))
+    got, whole = (t[:, :H * V * K].reshape(S.shape) for t in (state, state_w))
+    # 32-bit sums: the runs may not be further off than the whole walk by more than a rounding
+    assert e_out <= 1.2 * e_whole + 2 ** -22 and e_out < 1e-5
+    assert err(got, S) <= 1.2 * err(whole, S) + 2 ** -22
+    assert torch.equal(state[:, H * V * K:], start[:, H * V * K:])
+    assert torch.equal(state[:2], start[:2])                  # slots without rows
