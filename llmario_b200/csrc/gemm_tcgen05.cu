@@ -30,6 +30,7 @@
 #include "tcgen05.cuh"
 
 int llm_zero_f32(float* p, int rows, int cols, int ld, cudaStream_t stream);   // elementwise.cu
+int llm_pair_store_way(int T, int N, int K, int splits);                       // gemm_tcgen05_pair.cu
 int llm_gemm_tcgen05_pair(const void* X, const void* W, void* C, int c_dtype, int T, int N, int K, int lda,
                           int ldw, int ldc, int mode, int half, float limit, int* status, cudaStream_t stream);
 int llm_gemm_tcgen05_persistent(const void* X, const void* W, void* C, int c_dtype, int T, int N, int K,
@@ -465,6 +466,17 @@ static int gemm_any(const void* X, const void* W, void* C, int c_dtype, int T, i
     // one-tile kernel with 128 tokens
     // (the pair kernel cuts K itself where its adding epilogue allows, so it also takes the
     // products for which the caller asked for a split)
+    const int way = mode == 0 && splits > 1 && c_dtype == LLM_F32 ? llm_pair_store_way(T, N, K, splits) : 2;
+    if (way < 2) {
+      if (way == 1 && !out_is_zero) {
+        const int z = llm_zero_f32((float*)C, T, N, ldc, stream);
+        if (z != 0) return z;
+        g_llm_after_rotation = 1;      // (a kernel of many blocks: see launched_many_blocks)
+      }
+      int r = llm_gemm_tcgen05_pair(X, W, C, c_dtype, T, N, K, lda, ldw, ldc, way, half, limit, status, stream);
+      if (r != LLM_ERR_UNSUPPORTED) return r;
+      if (way == 1) out_is_zero = 1;
+    }
     if (splits == 1 || mode == 1) {
       int r = llm_gemm_tcgen05_pair(X, W, C, c_dtype, T, N, K, lda, ldw, ldc, mode, half, limit, status, stream);
       if (r != LLM_ERR_UNSUPPORTED) return r;

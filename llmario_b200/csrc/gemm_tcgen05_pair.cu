@@ -312,6 +312,23 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
   }
 }
 
+// The adding epilogue lets K be cut.  With few tiles to a pair the last round of tiles leaves
+// most pairs idle (160 tiles on 74 pairs: three rounds for the work of 2.2), and with fewer
+// tiles than pairs some never work.  A work item costs its 64-wide blocks of K plus about six
+// blocks' worth of start and epilogue (fitted to measured times of seven shapes); K is cut into
+// the number of ranges, each of at least eight blocks, for which the rounds cost least.
+int cheapest_cut(int tiles, int nkb, int pairs, double* cost_of_it) {
+  int ksplits = 1;
+  double best = 0;
+  for (int s = 1; s <= 8 && (s == 1 || nkb / s >= 8); ++s) {
+    const int rounds = (tiles * s + pairs - 1) / pairs;
+    const double cost = rounds * ((double)nkb / s + 6.0);
+    if (s == 1 || cost < best * 0.99) best = cost, ksplits = s;
+  }
+  *cost_of_it = best;
+  return ksplits;
+}
+
 template <int STAGES, int EPI, typename TC>
 int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mc, int T, int N, int K, int half,
            int sm_count, int* status, cudaStream_t stream, float act_limit = 0.f) {
@@ -352,20 +369,11 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mc, 
     }
     resident_pairs = n < sm_count / 2 ? n : sm_count / 2;
   }
-  // The adding epilogue lets K be cut.  With few tiles to a pair the last round of tiles leaves
-  // most pairs idle (160 tiles on 74 pairs: three rounds for the work of 2.2), and with fewer
-  // tiles than pairs some never work.  A work item costs its 64-wide blocks of K plus about six
-  // blocks' worth of start and epilogue (fitted to measured times of seven shapes); K is cut into
-  // the number of ranges, each of at least eight blocks, for which the rounds cost least.
   int ksplits = 1;
   if (EPI == EPI_ACCUM) {
-    const int tiles = m_tiles * n_tiles, nkb = (K + TILE_K - 1) / TILE_K;
-    double best = 0;
-    for (int s = 1; s <= 8 && nkb / s >= 8; ++s) {
-      const int rounds = (tiles * s + resident_pairs - 1) / resident_pairs;
-      const double cost = rounds * ((double)nkb / s + 6.0);
-      if (s == 1 || cost < best * 0.99) best = cost, ksplits = s;
-    }
+    const int nkb = (K + TILE_K - 1) / TILE_K;
+    double cost;
+    ksplits = cheapest_cut(m_tiles * n_tiles, nkb, resident_pairs, &cost);
     if (g_llm_pair_ksplits > 0 && nkb / g_llm_pair_ksplits >= 1) ksplits = g_llm_pair_ksplits;
   }
   const int works = m_tiles * n_tiles * ksplits;
@@ -377,6 +385,28 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mc, 
   return (int)cudaLaunchKernelEx(&cfg, kernel, mw, mx, mc, T, N, K, half, m_tiles, n_tiles, ksplits, act_limit, status);
 }
 }  // namespace
+
+// How a 32-bit product of many rows with few tiles, for which the caller asked for a split of K, is
+// made soonest: 0 whole sums on pairs, 1 the output cleared and ranges of K added into it on pairs,
+// 2 the same on lone CTAs with tiles of 128 x 128 in `splits` ranges.  In units of one 64-wide block
+// of K of a pair's tile (0.39 us): clearing is a launch and a pass over the output (2.5 us, then
+// 3 TB/s with the additions' own traffic); a lone CTA's block is 1.4 units with two CTAs to an SM.
+// Measured, lone CTAs against the choice made here, with weights from memory: 777 x 4,096 x 1,024
+// (rows x N x K) 29.7 -> 18.4 us, 2,048 x 1,024 x 3,072 39.6 -> 27.4 (ranges of K), 1,501 x 4,096 x 4,096
+// 70.5 -> 56.3, 512 x 6,144 x 4,096 46.1 -> 37.7; 513 x 1,024 x 1,024 stays on lone CTAs (15.4 against
+// 18.4 on pairs).
+int llm_pair_store_way(int T, int N, int K, int splits) {
+  const int pairs = 74, nkb = (K + TILE_K - 1) / TILE_K;
+  const int tiles = ((N + 2 * TILE_M - 1) / (2 * TILE_M)) * ((T + BN - 1) / BN);
+  const double clear = (2.5 + (double)T * N * 4 / 3e6) / 0.39;
+  const double whole = ((tiles + pairs - 1) / pairs) * (nkb + 6.0);
+  double cut;
+  if (cheapest_cut(tiles, nkb, pairs, &cut) == 1) cut = 1e30;
+  const long long lone = (long long)((N + TILE_M - 1) / TILE_M) * ((T + 127) / 128) * splits;
+  const double alone = (double)((lone + 4 * pairs - 1) / (4 * pairs)) * (1.4 * nkb / splits + 6.0) + clear;
+  if (alone < whole && alone < cut + clear) return 2;
+  return cut + clear < whole ? 1 : 0;
+}
 
 // The pair kernel for bfloat16 X [T][K], W [N][K]; modes 0, 1, 3 and 4 of llm_gemm_tcgen05 (no K
 // split; the gated form only with interleaved rows).  Returns LLM_ERR_UNSUPPORTED when the output

@@ -124,3 +124,20 @@ def test_recurrence_in_runs(kind, H, G, K, V, lengths):
     assert err(got, S) <= 1.2 * err(whole, S) + 2 ** -22
     assert torch.equal(state[:, H * V * K:], start[:, H * V * K:])
     assert torch.equal(state[:2], start[:2])                  # slots without rows
+
+
+@gpu
+@pytest.mark.parametrize("T,N,K", [(777, 4096, 1024), (1024, 520, 72), (543, 6144, 200), (2048, 1024, 3072),
+                                   (513, 264, 512), (1500, 136, 4096), (600, 4096, 2056), (2049, 520, 1024)])
+def test_linear_many_rows_few_tiles(T, N, K):
+    """Products with fewer tiles than CTAs, stored whole or added in ranges of K."""
+    from llmario_b200 import kernels
+    a, w = rnd(T, K, dtype=torch.bfloat16, seed=1), rnd(N, K, dtype=torch.bfloat16, seed=2)
+    wide = torch.full((T, N + 8), float("nan"), device=DEV)
+    kernels.linear(a, w, wide[:, :N])
+    ref = a.double() @ w.double().T
+    # 32-bit sums of exact products of 16-bit operands
+    bound = (K + 10) * 2 ** -23 * (a.abs().double() @ w.abs().double().T)
+    assert bool(((wide[:, :N].double() - ref).abs() <= bound).all())
+    assert bool(torch.isnan(wide[:, N:]).all())
+    kernels.check_tc_status(torch.device(DEV))
