@@ -43,8 +43,17 @@ template <> struct Vec8<bf16> {
   }
 };
 
-// VEC: the head size is a multiple of 8, so a key row is read in 16-byte (32-byte) pieces.
-// NACC: 32-channel pieces of a value row that a lane sums (vd <= 32 * NACC)
+// Whether the rows of block b of R rows (R <= 32, a power of two) are consecutive tokens of one
+// request: a whole warp asks.  The tiled kernel takes such blocks and the kernel of one warp per
+// (row, head) the others, so both have to agree.
+template <int R>
+__device__ __forceinline__ bool consecutive_rows(int b, int rows, const int* __restrict__ row_slot,
+                                                 const int* __restrict__ row_pos, int lane) {
+  const int r0 = b * R, n = min(R, rows - r0);
+  const int r = r0 + min(lane, n - 1);
+  return __all_sync(0xffffffffu, row_slot[r] == row_slot[r0] && row_pos[r] == row_pos[r0] + (r - r0));
+}
+
 // the second cache of a layer with pooled blocks (null k: none)
 struct PooledSource {
   const void *k, *v;
@@ -55,11 +64,13 @@ struct PooledSource {
 
 // VEC: the head size is a multiple of 8, so a key row is read in 16-byte (32-byte) pieces.
 // NACC: 32-channel pieces of a value row that a lane sums (vd <= 32 * NACC)
+// SKIP > 0: rows whose block of SKIP rows the tiled kernel below takes are left out (see
+// consecutive_rows).
 // EXTRAS: only what lies outside the window (pooled blocks, kept first keys, the sink) is summed,
 // and the result is left as a part for a merge with the window's keys, which another kernel sums:
 // part_o [rows][Hq][hd] the weighted values without the division, part_ml [rows][Hq][2] the
 // maximum as a base-2 logarithm (score times log2 e) and the sum of the weights.
-template <typename T, bool VEC, int NACC, bool EXTRAS>
+template <typename T, bool VEC, int NACC, bool EXTRAS, int SKIP = 0>
 __global__ void __launch_bounds__(WARPS * 32) attention_generic_kernel(
     const T* __restrict__ q, T* __restrict__ out, const T* __restrict__ k_cache,
     const T* __restrict__ v_cache, long long page_stride, const int* __restrict__ block_table,
@@ -71,6 +82,7 @@ __global__ void __launch_bounds__(WARPS * 32) attention_generic_kernel(
   const long long item = (long long)blockIdx.x * WARPS + warp_in_block;
   if (item >= (long long)rows * Hq) return;
   const int t = (int)(item / Hq), h = (int)(item % Hq);
+  if (SKIP > 0 && consecutive_rows<SKIP>(t / (SKIP > 0 ? SKIP : 1), rows, row_slot, row_pos, lane)) return;
   const int kvh = h / (Hq / Hkv);
   const int pos = row_pos[t];
   const int* table = block_table + (size_t)row_slot[t] * table_stride;
@@ -187,6 +199,198 @@ __global__ void __launch_bounds__(WARPS * 32) attention_generic_kernel(
     const int d = lane + 32 * i;
     if (d < vd) orow[d] = from_f32<T>(acc[i] * inv);
   }
+}
+
+// ---- the same for prompts in 32-bit: a block owns 32 queries (TILE_Q / GROUP consecutive tokens,
+// the GROUP heads that share a key head) and brings every tile of 32 keys and values into shared
+// memory once for all of them (cp.async, two tiles in flight), where the kernel above reads it
+// again for each query, a lane per key row.  Warp w has the queries 4 w .. 4 w + 3; a lane scores
+// its key of the tile against the four, then sums its channels of the values for the four.  Every
+// sum has the order of the kernel above (a dot product over ascending channels, the butterfly over
+// 32 keys aligned to absolute positions, ascending keys), so both give the same bits.
+// Bound by the 16-byte reads of shared memory (five per sixteen multiply-adds of the scores).  16
+// heads of 128 on 8 key heads, 64 / 211 / 512 rows of a prompt: 43 / 138 / 420 -> 28 / 48 / 118 us.
+constexpr int TILE_Q = 32, TILE_WARPS = 8;
+template <int HD, int GROUP>
+__global__ void __launch_bounds__(TILE_WARPS * 32, 2) attention_tile_f32_kernel(
+    const float* __restrict__ q, float* __restrict__ out, const float* __restrict__ k_cache,
+    const float* __restrict__ v_cache, long long page_stride, const int* __restrict__ block_table,
+    int table_stride, const int* __restrict__ row_slot, const int* __restrict__ row_pos, int rows, int Hq,
+    int page_size, float scale, int window) {
+  constexpr int R = TILE_Q / GROUP, LD = HD + 4, CH = HD / 32;      // CH channels per lane
+  extern __shared__ __align__(16) float t_smem[];
+  float* q_s = t_smem;                                 // [32 queries][LD]
+  float* w_s = q_s + TILE_Q * LD;                      // [warp][key][its four queries]
+  float* kv_s = w_s + TILE_WARPS * 32 * 4;             // two stages of keys [32][LD] and values [32][LD]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int b = (int)(gridDim.x - 1 - blockIdx.x), kvh = blockIdx.y;      // (the longest rows first)
+  if (!consecutive_rows<R>(b, rows, row_slot, row_pos, lane)) return;
+  const int r0 = b * R, n_rows = min(R, rows - r0);
+  const int pos0 = row_pos[r0], last = pos0 + n_rows - 1;
+  const int* table = block_table + (size_t)row_slot[r0] * table_stride;
+  const int low = first_key(pos0, window);
+  // eight threads bring a key and its value; where the row of the tile behind the one that is
+  // asked for lies is looked up a tile ahead, so that no copy waits for the block table
+  const int fj = tid >> 3, fc = (tid & 7) * 4;
+  auto locate = [&](int base) {
+    const int p = base + fj;
+    return p >= low && p <= last
+               ? (long long)table[p / page_size] * page_stride + ((long long)kvh * page_size + p % page_size) * HD
+               : -1LL;
+  };
+  auto fetch = [&](long long at, int stage) {
+    float* ks = kv_s + stage * 2 * 32 * LD + fj * LD + fc;
+    const bool there = at >= 0;
+    const float *kp = k_cache + (there ? at + fc : 0), *vp = v_cache + (there ? at + fc : 0);
+#pragma unroll
+    for (int c = 0; c < HD; c += 32) {
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(ks + c)), "l"(kp + (there ? c : 0)),
+                   "r"(there ? 16 : 0)
+                   : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(ks + 32 * LD + c)),
+                   "l"(vp + (there ? c : 0)), "r"(there ? 16 : 0)
+                   : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const int first = low / 32 * 32;
+  fetch(locate(first), 0);
+  long long next_at = locate(first + 32);
+  // query g * R + r of the block is head g of token r0 + r: a warp's four share a head (R >= 4)
+  for (int idx = tid; idx < TILE_Q * HD; idx += TILE_WARPS * 32) {
+    const int i = idx / HD, c = idx % HD, r = i % R;
+    q_s[i * LD + c] = r < n_rows ? q[((size_t)(r0 + r) * Hq + kvh * GROUP + i / R) * HD + c] : 0.f;
+  }
+  float m[4], l[4], acc[4][CH];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m[i] = -INFINITY, l[i] = 0.f;
+#pragma unroll
+    for (int c = 0; c < CH; ++c) acc[i][c] = 0.f;
+  }
+  float* my_w = w_s + warp * 32 * 4;
+  int stage = 0;
+  for (int base = first; base <= last; base += 32, stage ^= 1) {
+    if (base + 32 <= last) {
+      fetch(next_at, stage ^ 1);
+      next_at = locate(base + 64);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    const float* ks = kv_s + stage * 2 * 32 * LD;
+    const float* vs = ks + 32 * LD;
+    float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int c = 0; c < HD; c += 4) {
+      const float4 kk = *reinterpret_cast<const float4*>(ks + lane * LD + c);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 qq = *reinterpret_cast<const float4*>(q_s + (warp * 4 + i) * LD + c);
+        d[i] = fmaf(qq.x, kk.x, d[i]), d[i] = fmaf(qq.y, kk.y, d[i]);
+        d[i] = fmaf(qq.z, kk.z, d[i]), d[i] = fmaf(qq.w, kk.w, d[i]);
+      }
+    }
+    // the four queries' butterflies side by side.  (A query that sees no key of the tile keeps its
+    // sums: the maximum stays, so the correction is exactly 1, or 0 for sums that are still 0.)
+    unsigned mask[4];
+    float w[4], top[4], s[4], corr[4], sum[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int pos = pos0 + (warp * 4 + i) % R, p = base + lane;
+      const bool valid = p >= first_key(pos, window) && p <= pos;
+      mask[i] = __ballot_sync(0xffffffffu, valid);
+      // (a rounded product, as above, not one half of a multiply-add)
+      top[i] = s[i] = valid ? __fmul_rn(d[i], scale) : -INFINITY;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) top[i] = fmaxf(top[i], __shfl_xor_sync(0xffffffffu, top[i], o));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float m_new = fmaxf(m[i], top[i]);
+      sum[i] = w[i] = (mask[i] >> lane) & 1u ? expf(s[i] - m_new) : 0.f;
+      corr[i] = (m[i] == -INFINITY) ? 0.f : expf(m[i] - m_new);
+      m[i] = m_new;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], o);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      l[i] = l[i] * corr[i] + sum[i];
+#pragma unroll
+      for (int c = 0; c < CH; ++c) acc[i][c] *= corr[i];
+    }
+    *reinterpret_cast<float4*>(my_w + lane * 4) = make_float4(w[0], w[1], w[2], w[3]);
+    __syncwarp();
+    const bool whole = (mask[0] & mask[1] & mask[2] & mask[3]) == 0xffffffffu;
+    const unsigned any = mask[0] | mask[1] | mask[2] | mask[3];
+    auto values = [&](int j, float (&v)[CH]) {
+      if (CH == 4) {
+        const float4 t = *reinterpret_cast<const float4*>(vs + j * LD + 4 * lane);
+        v[0] = t.x, v[1] = t.y, v[CH - 2] = t.z, v[CH - 1] = t.w;
+      } else {
+        const float2 t = *reinterpret_cast<const float2*>(vs + j * LD + 2 * lane);
+        v[0] = t.x, v[1] = t.y;
+      }
+    };
+    if (whole) {
+#pragma unroll 4
+      for (int j = 0; j < 32; ++j) {
+        const float4 wj = *reinterpret_cast<const float4*>(my_w + j * 4);
+        float v[CH];
+        values(j, v);
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+          acc[0][c] = fmaf(wj.x, v[c], acc[0][c]), acc[1][c] = fmaf(wj.y, v[c], acc[1][c]);
+          acc[2][c] = fmaf(wj.z, v[c], acc[2][c]), acc[3][c] = fmaf(wj.w, v[c], acc[3][c]);
+        }
+      }
+    } else {
+      // (a key that a query does not see adds nothing, whatever its value is)
+      for (int j = 0; j < 32; ++j) {
+        if (!((any >> j) & 1u)) continue;
+        const float4 wj = *reinterpret_cast<const float4*>(my_w + j * 4);
+        const float we[4] = {wj.x, wj.y, wj.z, wj.w};
+        float v[CH];
+        values(j, v);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if ((mask[i] >> j) & 1u) {
+#pragma unroll
+            for (int c = 0; c < CH; ++c) acc[i][c] = fmaf(we[i], v[c], acc[i][c]);
+          }
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int at = warp * 4 + i, r = at % R;
+    if (r >= n_rows) continue;
+    const float inv = 1.0f / l[i];
+    float* o = out + ((size_t)(r0 + r) * Hq + kvh * GROUP + at / R) * HD + CH * lane;
+#pragma unroll
+    for (int c = 0; c < CH; ++c) o[c] = acc[i][c] * inv;
+  }
+}
+
+template <int HD, int GROUP>
+int launch_tile_f32(const float* q, float* out, const float* k, const float* v, long long page_stride,
+                    const int* block_table, int table_stride, const int* row_slot, const int* row_pos, int rows, int Hq,
+                    int Hkv, int page_size, float scale, int window, cudaStream_t stream) {
+  constexpr int R = TILE_Q / GROUP, LD = HD + 4;
+  constexpr int SMEM = (TILE_Q * LD + TILE_WARPS * 32 * 4 + 4 * 32 * LD) * 4;
+  auto kernel = attention_tile_f32_kernel<HD, GROUP>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+  if (e != cudaSuccess) return (int)e;
+  kernel<<<dim3((rows + R - 1) / R, Hkv), TILE_WARPS * 32, SMEM, stream>>>(
+      q, out, k, v, page_stride, block_table, table_stride, row_slot, row_pos, rows, Hq, page_size, scale, window);
+  return launch_status();
 }
 
 // What lies outside the window for all heads of a group at once: one warp per (row, key head).
@@ -323,14 +527,12 @@ __global__ void __launch_bounds__(WARPS * 32) attention_outside_kernel(
 }
 }  // namespace
 
-// keep_first and the pooled cache (pk_cache null: none) as described at the top of this file
-LLM_EXPORT int llm_attention_generic_ext(const void* q, void* out, const void* k_cache, const void* v_cache,
-                                         int dtype, long long page_stride, const int* block_table,
-                                         int table_stride, const int* row_slot, const int* row_pos, int rows,
-                                         int Hq, int Hkv, int hd, int page_size, float scale, int window,
-                                         const float* sink, int vd, int keep_first, const void* pk_cache,
-                                         const void* pv_cache, long long p_page_stride, const int* p_table,
-                                         int p_table_stride, int pool, cudaStream_t stream) {
+static int attention_generic(const void* q, void* out, const void* k_cache, const void* v_cache, int dtype,
+                             long long page_stride, const int* block_table, int table_stride, const int* row_slot,
+                             const int* row_pos, int rows, int Hq, int Hkv, int hd, int page_size, float scale,
+                             int window, const float* sink, int vd, int keep_first, const void* pk_cache,
+                             const void* pv_cache, long long p_page_stride, const int* p_table, int p_table_stride,
+                             int pool, bool single, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (vd <= 0) vd = hd;
   if (hd > MAX_HD || hd <= 0 || vd > hd || Hkv <= 0 || Hq % Hkv != 0) return LLM_ERR_UNSUPPORTED;
@@ -345,6 +547,38 @@ LLM_EXPORT int llm_attention_generic_ext(const void* q, void* out, const void* k
                     ((p_page_stride % 8) == 0 && (((uintptr_t)pk_cache | (uintptr_t)pv_cache) & 31) == 0));
   const long long items = (long long)rows * Hq;
   const int blocks = (int)((items + WARPS - 1) / WARPS);
+  // Prompts in 32-bit: blocks of consecutive tokens by tiles, the rest by the kernel of one warp
+  // per (row, head), which leaves those out.  Both find the blocks on the device, from row_slot and
+  // row_pos, so no list of items is needed; a caller that knows that every row is a request of its
+  // own (`single`) gets the second kernel alone, and so do steps of fewer than 16 rows (16 rows of
+  // one prompt: 19 us row by row, 23 by tiles; 64: 43 and 28).
+  const int group = Hq / Hkv;
+  if (dtype == LLM_F32 && vec && !single && vd == hd && (hd == 64 || hd == 128) && !sink && keep_first == 0 &&
+      pk_cache == nullptr && (group == 1 || group == 2 || group == 4 || group == 8) && rows >= 16 && Hkv <= 65535 &&
+      (((uintptr_t)q | (uintptr_t)out) & 15) == 0) {
+    int rc = LLM_ERR_UNSUPPORTED;
+#define TILED(D, G)                                                                                              \
+  do {                                                                                                           \
+    rc = launch_tile_f32<D, G>((const float*)q, (float*)out, (const float*)k_cache, (const float*)v_cache,       \
+                               page_stride, block_table, table_stride, row_slot, row_pos, rows, Hq, Hkv,         \
+                               page_size, scale, window, stream);                                                \
+    if (rc) return rc;                                                                                           \
+    attention_generic_kernel<float, true, 4, false, TILE_Q / G><<<blocks, WARPS * 32, 0, stream>>>(              \
+        (const float*)q, (float*)out, (const float*)k_cache, (const float*)v_cache, page_stride, block_table,    \
+        table_stride, row_slot, row_pos, rows, Hq, Hkv, hd, page_size, scale, window, sink, vd, keep_first,      \
+        pooled, nullptr, nullptr);                                                                               \
+    return launch_status();                                                                                      \
+  } while (0)
+#define TILED_G(D)            \
+  if (group == 1) TILED(D, 1); \
+  if (group == 2) TILED(D, 2); \
+  if (group == 4) TILED(D, 4); \
+  TILED(D, 8)
+    if (hd == 64) { TILED_G(64); }
+    TILED_G(128);
+#undef TILED_G
+#undef TILED
+  }
 #define GENERIC(T, V, N)                                                                            \
   attention_generic_kernel<T, V, N, false><<<blocks, WARPS * 32, 0, stream>>>(                      \
       (const T*)q, (T*)out, (const T*)k_cache, (const T*)v_cache, page_stride, block_table,         \
@@ -368,15 +602,40 @@ LLM_EXPORT int llm_attention_generic_ext(const void* q, void* out, const void* k
   return launch_status();
 }
 
+// keep_first and the pooled cache (pk_cache null: none) as described at the top of this file
+LLM_EXPORT int llm_attention_generic_ext(const void* q, void* out, const void* k_cache, const void* v_cache,
+                                         int dtype, long long page_stride, const int* block_table,
+                                         int table_stride, const int* row_slot, const int* row_pos, int rows,
+                                         int Hq, int Hkv, int hd, int page_size, float scale, int window,
+                                         const float* sink, int vd, int keep_first, const void* pk_cache,
+                                         const void* pv_cache, long long p_page_stride, const int* p_table,
+                                         int p_table_stride, int pool, cudaStream_t stream) {
+  return attention_generic(q, out, k_cache, v_cache, dtype, page_stride, block_table, table_stride, row_slot, row_pos,
+                           rows, Hq, Hkv, hd, page_size, scale, window, sink, vd, keep_first, pk_cache, pv_cache,
+                           p_page_stride, p_table, p_table_stride, pool, false, stream);
+}
+
 LLM_EXPORT int llm_attention_generic(const void* q, void* out, const void* k_cache,
                                      const void* v_cache, int dtype, long long page_stride,
                                      const int* block_table, int table_stride, const int* row_slot,
                                      const int* row_pos, int rows, int Hq, int Hkv, int hd,
                                      int page_size, float scale, int window, const float* sink, int vd,
                                      cudaStream_t stream) {
-  return llm_attention_generic_ext(q, out, k_cache, v_cache, dtype, page_stride, block_table, table_stride,
-                                   row_slot, row_pos, rows, Hq, Hkv, hd, page_size, scale, window, sink, vd, 0,
-                                   nullptr, nullptr, 0, nullptr, 0, 0, stream);
+  return attention_generic(q, out, k_cache, v_cache, dtype, page_stride, block_table, table_stride, row_slot, row_pos,
+                           rows, Hq, Hkv, hd, page_size, scale, window, sink, vd, 0, nullptr, nullptr, 0, nullptr, 0,
+                           0, false, stream);
+}
+
+// The same for a step whose rows are known to be one token each of as many requests (the result
+// is the same bits; only the way to it differs).
+LLM_EXPORT int llm_attention_generic_single(const void* q, void* out, const void* k_cache, const void* v_cache,
+                                            int dtype, long long page_stride, const int* block_table,
+                                            int table_stride, const int* row_slot, const int* row_pos, int rows,
+                                            int Hq, int Hkv, int hd, int page_size, float scale, int window,
+                                            const float* sink, int vd, cudaStream_t stream) {
+  return attention_generic(q, out, k_cache, v_cache, dtype, page_stride, block_table, table_stride, row_slot, row_pos,
+                           rows, Hq, Hkv, hd, page_size, scale, window, sink, vd, 0, nullptr, nullptr, 0, nullptr, 0,
+                           0, true, stream);
 }
 
 // Only what a row sees outside its window: the pooled blocks that lie behind it, the kept first

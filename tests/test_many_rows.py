@@ -141,3 +141,48 @@ def test_linear_many_rows_few_tiles(T, N, K):
     assert bool(((wide[:, :N].double() - ref).abs() <= bound).all())
     assert bool(torch.isnan(wide[:, N:]).all())
     kernels.check_tc_status(torch.device(DEV))
+
+
+@gpu
+@pytest.mark.parametrize("group,hd,window,page", [(1, 64, 0, 16), (2, 128, 0, 64), (4, 128, 50, 16), (8, 64, 33, 4),
+                                                  (2, 64, -48, 32), (8, 128, 0, 8)])
+def test_attention_float32_tiles_give_the_bits_of_single_rows(group, hd, window, page):
+    """Blocks of consecutive tokens go by tiles, the rest row by row: both give the same bits,
+    whatever is in the step (a request's end inside a block, single tokens between portions, values
+    that are not finite at positions a row does not see)."""
+    from llmario_b200 import kernels
+    Hkv = 2
+    Hq = Hkv * group
+    segments = [(0, 37), (900, 1), (5, 70), (3, 3), (64, 16), (0, 1), (31, 45)]      # (first position, rows)
+    slots = [4, 0, 6, 1, 3, 2, 5]
+    n_pages = sum(-(-(p + n) // page) for p, n in segments)
+    storage = rnd(n_pages, 2, Hkv, page, hd, seed=5)
+    table = torch.full((7, 1024 // page), -1, dtype=torch.int32)
+    used = 0
+    row_slot, row_pos = [], []
+    for (p, n), slot in zip(segments, slots):
+        need = -(-(p + n) // page)
+        table[slot, :need] = torch.randperm(need, generator=torch.Generator().manual_seed(slot)).int() + used
+        used += need
+        row_slot += [slot] * n
+        row_pos += list(range(p, p + n))
+    # the last position of the first request holds values that no other row may meet
+    last = segments[0][1] - 1
+    storage[int(table[4, last // page]), 1, :, last % page] = float("inf")
+    rs = torch.tensor(row_slot, dtype=torch.int32, device=DEV)
+    rp = torch.tensor(row_pos, dtype=torch.int32, device=DEV)
+    table = table.to(DEV)
+    q = rnd(len(row_slot), Hq * hd, seed=7)
+
+    def run(rows):
+        out = torch.full((len(rows), Hq * hd), float("nan"), device=DEV)
+        kernels.attention_generic(q[rows].contiguous(), out, storage[:, 0], storage[:, 1], storage.stride(0), table,
+                                  rs[rows].contiguous(), rp[rows].contiguous(), Hq, Hkv, hd, page, hd ** -0.5, window)
+        return out
+
+    everything = run(list(range(len(row_slot))))
+    # eight rows are fewer than a block: row by row
+    alone = torch.cat([run(list(range(i, min(i + 8, len(row_slot))))) for i in range(0, len(row_slot), 8)])
+    finite = [i for i in range(len(row_slot)) if i != last]
+    assert bool(torch.isfinite(everything[finite]).all())
+    assert torch.equal(everything[finite], alone[finite])
