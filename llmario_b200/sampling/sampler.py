@@ -17,7 +17,7 @@ import torch
 
 from .. import kernels
 from .params import SamplingParams
-from .rng import Xoshiro256StarStar
+from .rng import Xoshiro256StarStar, next_uniforms
 
 
 _serials = itertools.count(1)
@@ -183,9 +183,9 @@ class DeviceSampler:
                                                  p.presence_penalty)
                     k[r] = p.top_k
                 self._host_key[i] = key
-            u = h[8 * c:10 * c].view(np.float64)
-            for r, s in enumerate(samplers):
-                u[r] = s.next_uniform()
+            # (greedy rows do not advance their streams)
+            next_uniforms([None if s.params.greedy else s.rng for s in samplers],
+                          self._host[i].data_ptr() + 8 * c * 4)
             self._dev.copy_(self._host[i], non_blocking=True)
             self.h2d_bytes += self._host[i].numel() * 4
             self._host_event[i] = torch.cuda.Event()

@@ -186,3 +186,15 @@ def test_attention_float32_tiles_give_the_bits_of_single_rows(group, hd, window,
     finite = [i for i in range(len(row_slot)) if i != last]
     assert bool(torch.isfinite(everything[finite]).all())
     assert torch.equal(everything[finite], alone[finite])
+
+
+def test_uniforms_of_many_streams():
+    """The native draw: every stream's own next number, in order, nothing for streams left out."""
+    import ctypes
+    from llmario_b200.sampling.rng import Xoshiro256StarStar, next_uniforms
+    mine, alone = ([Xoshiro256StarStar(s) for s in (0, 1, 2 ** 64 - 1, 7)] for _ in range(2))
+    out = (ctypes.c_double * 5)(*[9.0] * 5)
+    for _ in range(3):
+        next_uniforms([mine[0], None, mine[1], mine[2], mine[0]], ctypes.addressof(out))
+        assert list(out) == [alone[0].next_f64(), 0.0, alone[1].next_f64(), alone[2].next_f64(), alone[0].next_f64()]
+    assert mine[3].next_u64() == alone[3].next_u64()
