@@ -976,6 +976,64 @@ __global__ void __launch_bounds__(THREADS) gated_group_norm_vec_kernel(
   }
 }
 
+// The same for groups of up to 256 channels, a warp per (row, group) and eight of them to a block
+// (a block of one warp each: 1,501 rows of 32 groups of 128 took 51 us, mostly the start of 48,032
+// blocks; now 16.5, the bytes take 11).  The sum has the same order, so the result is the same bits.
+template <typename TOut>
+__global__ void __launch_bounds__(256) gated_group_norm_warp_kernel(
+    const float* __restrict__ o, int o_stride, const float* __restrict__ x, int x_stride,
+    const float* __restrict__ skip, int head, const float* __restrict__ g, int g_stride,
+    const float* __restrict__ w, int w_period, TOut* __restrict__ out, int out_stride, int groups, int group,
+    float eps, int gate_first, int gate_sigmoid, int items) {
+  constexpr int KEEP = 2;
+  pdl_trigger();
+  pdl_wait();
+  const int item = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (item >= items) return;
+  const int r = item / groups, gi = item - r * groups;
+  const int c0 = gi * group, n4 = group >> 2;
+  float4 y[KEEP], gate[KEEP];
+  float ss = 0.f;
+#pragma unroll
+  for (int n = 0; n < KEEP; ++n) {
+    const int i = lane + n * 32, ch = c0 + 4 * i;
+    if (i >= n4) continue;
+    float4 v = *reinterpret_cast<const float4*>(o + (size_t)r * o_stride + ch);
+    if (skip) {
+      const float d = skip[ch / head];
+      const float4 xv = *reinterpret_cast<const float4*>(x + (size_t)r * x_stride + ch);
+      v.x = fmaf(d, xv.x, v.x), v.y = fmaf(d, xv.y, v.y), v.z = fmaf(d, xv.z, v.z), v.w = fmaf(d, xv.w, v.w);
+    }
+    const float4 gv = *reinterpret_cast<const float4*>(g + (size_t)r * g_stride + ch);
+    gate[n] = make_float4(gate_f(gv.x, gate_sigmoid), gate_f(gv.y, gate_sigmoid), gate_f(gv.z, gate_sigmoid),
+                          gate_f(gv.w, gate_sigmoid));
+    if (gate_first) v.x *= gate[n].x, v.y *= gate[n].y, v.z *= gate[n].z, v.w *= gate[n].w;
+    y[n] = v;
+    ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+  }
+  ss = warp_sum(ss);
+  const float scale = 1.0f / sqrtf(ss / (float)group + eps);
+#pragma unroll
+  for (int n = 0; n < KEEP; ++n) {
+    const int i = lane + n * 32, ch = c0 + 4 * i;
+    if (i >= n4) continue;
+    const float4 wv = *reinterpret_cast<const float4*>(w + ch % w_period);
+    float4 v = y[n];
+    v.x = v.x * scale * wv.x, v.y = v.y * scale * wv.y, v.z = v.z * scale * wv.z, v.w = v.w * scale * wv.w;
+    if (!gate_first) v.x *= gate[n].x, v.y *= gate[n].y, v.z *= gate[n].z, v.w *= gate[n].w;
+    TOut* dst = out + (size_t)r * out_stride + ch;
+    if (sizeof(TOut) == 4) {
+      *reinterpret_cast<float4*>(dst) = v;
+    } else {
+      __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+      uint2 packed;
+      packed.x = *reinterpret_cast<uint32_t*>(&lo);
+      packed.y = *reinterpret_cast<uint32_t*>(&hi);
+      *reinterpret_cast<uint2*>(dst) = packed;
+    }
+  }
+}
+
 // ---- exponential gates kept in range by a running maximum (the gates of a matrix memory)
 //   i_t = cap tanh((zi_t + bi) / cap),  f_t = log sigmoid(cap tanh((zf_t + bf) / cap))
 //   m_t = max(f_t + m_{t-1}, i_t),  keep_t = exp(f_t + m_{t-1} - m_t),  take_t = exp(i_t - m_t)
@@ -1725,6 +1783,16 @@ static int gated_group_norm_launch(const float* o, int o_stride, const float* x,
   return launch_pdl(gated_group_norm_vec_kernel<T, TH>, blocks, TH, 0, stream, o, o_stride, x, x_stride, skip,  \
                     head, g, g_stride, w, w_period, (T*)out, out_stride, groups, group, eps, gate_first,   \
                     gate_sigmoid)
+#define GNW(T)                                                                                                  \
+  return launch_pdl(gated_group_norm_warp_kernel<T>, (blocks + 7) / 8, 256, 0, stream, o, o_stride, x, x_stride, \
+                    skip, head, g, g_stride, w, w_period, (T*)out, out_stride, groups, group, eps, gate_first,   \
+                    gate_sigmoid, blocks)
+  // (few groups: a block each spreads them over the SMs)
+  if (vec && group <= 256 && items >= 2048) {
+    if (out_dtype == LLM_F32) GNW(float);
+    if (out_dtype == LLM_BF16) GNW(bf16);
+  }
+#undef GNW
   if (vec && out_dtype == LLM_F32) {
     if (group <= 256) GNV(float, 32);
     if (group <= 512) GNV(float, 64);
