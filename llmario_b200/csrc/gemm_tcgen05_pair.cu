@@ -16,8 +16,17 @@
 //              multiplied: TMEM -> registers -> shared memory in chunks of 32 tokens -> TMA store or
 //              TMA add-reduction; the leader learns from both CTAs when an accumulator is drained
 //
-// Epilogues: store, residual add, gated silu(g) * u with gate and up rows interleaved in blocks of
-// 16.  The output must be reachable by TMA.  Every wait is bounded: a CTA that gives up sets
+// The grouped form (GROUPED): X's rows lie in tiles of bn rows, tile i multiplied with matrix
+// tile_group[i] of W (a feed-forward of routed experts, the tokens sorted by expert).  Neighbouring
+// tiles of one matrix are taken together, up to 256 rows, and the MMA is as wide as what was
+// taken (N = bn, 2 bn, ... 256), so that only the padding of an expert's last bn rows is multiplied for
+// nothing.  1,501 tokens with two of eight experts of 6,144 x 4,096, lone CTAs with tiles of 128 rows ->
+// pairs: up with its squared rectifier 241 -> 163 us (one kernel instead of two), gated 183 -> 164, down
+// 165 -> 165 (3,072 tokens: 299 -> 288).  (Dealing the pieces by length, the longest first, took 199 us: a matrix's pieces then are
+// not neighbours in time and its rows come from memory twice.)
+//
+// Epilogues: store, residual add, squared rectifier, gated silu(g) * u with gate and up rows
+// interleaved in blocks of 16.  The output must be reachable by TMA.  Every wait is bounded: a CTA that gives up sets
 // *status and walks to the final cluster barrier, where its peer (whose own waits run out in
 // turn) meets it before tensor memory is freed.  No load is multicast.
 #include "tcgen05.cuh"
@@ -30,7 +39,9 @@ constexpr int BN = 256;          // tokens per pair tile
 constexpr int HALF_N = 128;      // tokens this CTA loads
 constexpr int CH = 32;           // tokens per epilogue chunk
 
-template <int STAGES, int FEAT, typename TC>
+constexpr int MAX_SMALL = 512;   // tiles of bn rows that the grouped form takes
+
+template <int STAGES, int FEAT, typename TC, bool GROUPED>
 struct alignas(1024) PairStorage {
   uint8_t a[STAGES][TILE_M * TILE_K * 2];      // this CTA's 128 weight rows
   uint8_t b[STAGES][HALF_N * TILE_K * 2];      // this CTA's 128 tokens
@@ -41,6 +52,9 @@ struct alignas(1024) PairStorage {
   uint64_t acc_empty[2];        // leader: both CTAs have drained the accumulator
   uint32_t tmem_base;
   int dead;
+  int n_list;                                      // grouped form: what is multiplied together,
+  int list[GROUPED ? MAX_SMALL : 1];               // first tile + (tiles << 16),
+  int group[GROUPED ? MAX_SMALL : 1];              // and every tile's matrix
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -102,6 +116,10 @@ __device__ __forceinline__ void pair_mma(uint32_t tmem_d, uint64_t desc_a, uint6
       ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+__device__ __forceinline__ float relu_squared(float z) {
+  const float r = fmaxf(z, 0.f);
+  return r * r;
+}
 // when the MMAs issued so far are done, arrive on the barrier at this offset in both CTAs
 __device__ __forceinline__ void pair_commit(uint64_t* bar) {
   const uint16_t both = 3;
@@ -111,29 +129,40 @@ __device__ __forceinline__ void pair_commit(uint64_t* bar) {
       : "memory");
 }
 
-template <int STAGES, int EPI, typename TC>
+// the grouped form's operands: n_small tiles of bn rows, tile i with matrix tile_group[i] (negative:
+// left out), matrices group_rows rows of W apart; row_scale (clamped epilogue): a factor per row of X
+struct Grouping {
+  const int* tile_group;
+  int bn, n_small, group_rows;
+  const float* row_scale;
+};
+
+// What a tile holds: 256 tokens always; 256 or, at the end of T, fewer; or the grouped form's pieces.
+// (A variant of its own for the first: with a width read at run time it lost 1 % on prompts of 2,048
+// and 8,192 tokens.)
+enum Form : int { WHOLE_TILES = 0, LAST_TOKENS = 1, GROUPED_TILES = 2 };
+
+// map_x: boxes of 128 tokens, map_xs: of 64
+template <int STAGES, int EPI, typename TC, int FORM>
 __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
     const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-    const __grid_constant__ CUtensorMap map_c, int T, int N, int K, int half, int m_tiles, int n_tiles,
-    int ksplits, float act_limit, int* __restrict__ status) {
-  constexpr bool GATED = gated_epilogue(EPI);
+    const __grid_constant__ CUtensorMap map_xs, const __grid_constant__ CUtensorMap map_c, int T, int N, int K, int half,
+    int m_tiles, int n_tiles, int ksplits, float act_limit, int* __restrict__ status, const Grouping grouping) {
+  constexpr bool GATED = gated_epilogue(EPI), GROUPED = FORM == GROUPED_TILES;
   constexpr int FEAT = GATED ? 64 : TILE_M;     // output features of this CTA per tile
   extern __shared__ uint8_t raw[];
-  auto& sm = *reinterpret_cast<PairStorage<STAGES, FEAT, TC>*>(
+  auto& sm = *reinterpret_cast<PairStorage<STAGES, FEAT, TC, GROUPED>*>(
       (reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
   const bool leader = rank == 0;
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const int nkb = (K + TILE_K - 1) / TILE_K;
-  const int tiles = m_tiles * n_tiles;
   // A work item is a tile and one of `ksplits` ranges of K (more than one only with the adding
-  // epilogue, whose partial sums meet in memory): item w is tile w % tiles, range w / tiles.
-  const int works = tiles * ksplits;
-  constexpr uint32_t STAGE_BYTES = TILE_M * TILE_K * 2 + HALF_N * TILE_K * 2;
-  // float32 accumulator, bf16 A and B, both K-major, N = 256, M = 256 over the pair
-  constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
-                             ((uint32_t)((2 * TILE_M) >> 4) << 24);
+  // epilogue, whose partial sums meet in memory).
+  int works = m_tiles * n_tiles * ksplits;
+  // float32 accumulator, bf16 A and B, both K-major, M = 256 over the pair; N as the tile has tokens
+  constexpr uint32_t idesc_0 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)((2 * TILE_M) >> 4) << 24);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -159,6 +188,59 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
   pdl_trigger();             // after the allocation, as in the one-CTA kernel
+  if (GROUPED) {
+    // (the tiles' matrices come from a kernel before this one, and the weights depend on them)
+    pdl_wait();
+    for (int i = threadIdx.x; i < grouping.n_small; i += 192) sm.group[i] = grouping.tile_group[i];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const int most = BN / grouping.bn;
+      int n = 0, len = 0, last = -1;
+      for (int i = 0; i < grouping.n_small; ++i) {
+        const int g = sm.group[i];
+        if (g >= 0) {
+          if (g == last && len < most) ++len, sm.list[n - 1] += 1 << 16;
+          else len = 1, sm.list[n++] = i | (1 << 16);
+        }
+        last = g;
+      }
+      sm.n_list = n;
+    }
+    __syncthreads();
+    n_tiles = sm.n_list;
+    works = m_tiles * n_tiles;
+  }
+  // the tile and the range of K of a work item: items of whole tiles before those of the last tokens
+  const int n_whole = GROUPED ? 0 : m_tiles * (T / BN);
+  auto item = [&](int work, int& tile, int& ks) {
+    if (GROUPED) {
+      tile = work, ks = 0;
+    } else if (FORM == WHOLE_TILES) {
+      tile = work % n_whole, ks = work / n_whole;
+    } else if (work < n_whole * ksplits) {
+      tile = work % n_whole, ks = work / n_whole;
+    } else {
+      const int rest = work - n_whole * ksplits;
+      tile = n_whole + rest % m_tiles, ks = rest / m_tiles;
+    }
+  };
+  // a tile's place among the tiles of weight rows, its first row of X, its rows, and the row of W
+  // where its matrix starts
+  auto place = [&](int tile, int& m, int& t0, int& n, int& w0) {
+    if (GROUPED) {
+      const int e = sm.list[tile % n_tiles], i = e & 0xffff;
+      m = tile / n_tiles, t0 = i * grouping.bn, n = (e >> 16) * grouping.bn, w0 = sm.group[i] * grouping.group_rows;
+    } else if (FORM == WHOLE_TILES) {
+      m = tile / n_tiles, t0 = (tile % n_tiles) * BN, n = BN, w0 = 0;
+    } else {
+      // the whole tiles of tokens first, then, if T is not a multiple of 256, the last tokens, with
+      // an MMA as wide as they are (in steps of 32)
+      const int whole = T / BN;
+      w0 = 0;
+      if (tile < n_whole) m = tile / whole, t0 = (tile % whole) * BN, n = BN;
+      else m = tile - n_whole, t0 = whole * BN, n = (T - t0 + 31) & ~31;
+    }
+  };
 
   if (warp == 0 && lane == 0) {
     // ------------------------------------------------------------------ producer (both CTAs)
@@ -167,26 +249,35 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
     // before that arrival: the count is signed).
     uint32_t full_addr[STAGES];
     for (int s = 0; s < STAGES; ++s) full_addr[s] = in_cta(&sm.full[s], 0);
-    auto load_w = [&](int s, int row0, int k) {
-      if (leader) mbar_expect_tx(&sm.full[s], 2 * STAGE_BYTES);
+    // A tile of up to 128 tokens brings half a box of them (both operands come from the L2 at some 10
+    // TB/s over all pairs, which is what holds this kernel; several smaller boxes cost the TMA unit
+    // more than they save: 165 -> 181 us for the grouped products above).
+    auto load_w = [&](int s, int row0, int k, int n) {
+      const int b_rows = FORM == WHOLE_TILES || n > HALF_N ? HALF_N : HALF_N / 2;
+      if (leader) mbar_expect_tx(&sm.full[s], 2 * (uint32_t)((TILE_M + b_rows) * TILE_K * 2));
       tma_load_2d_pair(sm.a[s], &map_w, k, row0, full_addr[s]);
+    };
+    auto load_x = [&](int s, int t0, int k, int n) {
+      tma_load_2d_pair(sm.b[s], FORM == WHOLE_TILES || n > HALF_N ? &map_x : &map_xs, k, t0, full_addr[s]);
     };
     long long it = 0;
     bool ok = true;
     bool first = true;
     for (int work = pair; work < works && ok; work += n_pairs) {
-      const int tile = work % tiles, ks = work / tiles;
+      int tile, ks, m, t0, n, w0;
+      item(work, tile, ks);
+      place(tile, m, t0, n, w0);
       const int kb0 = (int)((long long)ks * nkb / ksplits), kb1 = (int)((long long)(ks + 1) * nkb / ksplits);
-      const int f0 = (tile / n_tiles) * (2 * FEAT) + (int)rank * FEAT;      // first output feature
-      const int row0 = GATED ? 2 * f0 : f0;                      // first weight row
-      const int t0 = (tile % n_tiles) * BN + (int)rank * HALF_N;
+      const int f0 = m * (2 * FEAT) + (int)rank * FEAT;          // first output feature
+      const int row0 = w0 + (GATED ? 2 * f0 : f0);               // first weight row
+      t0 += (int)rank * (n >> 1);                                // (this CTA's half of the tokens)
       int kb = kb0;
-      if (first) {
+      if (!GROUPED && first) {
         // weights do not depend on earlier kernels: fetch a ring of them before waiting
         const int head = min(kb1 - kb0, STAGES);
-        for (int i = 0; i < head; ++i) load_w(i, row0, (kb0 + i) * TILE_K);
+        for (int i = 0; i < head; ++i) load_w(i, row0, (kb0 + i) * TILE_K, n);
         pdl_wait();
-        for (int i = 0; i < head; ++i) tma_load_2d_pair(sm.b[i], &map_x, (kb0 + i) * TILE_K, t0, full_addr[i]);
+        for (int i = 0; i < head; ++i) load_x(i, t0, (kb0 + i) * TILE_K, n);
         it = head;
         kb = kb0 + head;
         first = false;
@@ -195,8 +286,8 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
         const int s = (int)(it % STAGES);
         ok = mbar_wait_pair(&sm.empty[s], (uint32_t)((it / STAGES) & 1) ^ 1);
         if (!ok) { atomicExch(status, 1); sm.dead = 1; break; }
-        load_w(s, row0, kb * TILE_K);
-        tma_load_2d_pair(sm.b[s], &map_x, kb * TILE_K, t0, full_addr[s]);
+        load_w(s, row0, kb * TILE_K, n);
+        load_x(s, t0, kb * TILE_K, n);
       }
     }
     // A producer gives up only after a wait of about two seconds, far longer than any load it
@@ -207,7 +298,10 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
     int local = 0;
     bool ok = true;
     for (int work = pair; work < works && ok; work += n_pairs, ++local) {
-      const int ks = work / tiles;
+      int tile, ks, m, t0, n, w0;
+      item(work, tile, ks);
+      place(tile, m, t0, n, w0);
+      const uint32_t idesc = idesc_0 | ((uint32_t)(n >> 3) << 17);
       const int kb0 = (int)((long long)ks * nkb / ksplits), kb1 = (int)((long long)(ks + 1) * nkb / ksplits);
       const int buf = local & 1;
       ok = mbar_wait_pair(&sm.acc_empty[buf], (uint32_t)((local >> 1) & 1) ^ 1);
@@ -238,8 +332,10 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
     int local = 0;
     int chunk_no = 0;
     for (int work = pair; work < works; work += n_pairs, ++local) {
-      const int tile = work % tiles;
-      const int n0 = (tile / n_tiles) * (2 * FEAT) + (int)rank * FEAT, t0 = (tile % n_tiles) * BN;
+      int tile, ks, m, t0, n_cols, w0;
+      item(work, tile, ks);
+      place(tile, m, t0, n_cols, w0);
+      const int n0 = m * (2 * FEAT) + (int)rank * FEAT;
       const int buf = local & 1;
       bool ok = mbar_wait_pair(&sm.acc_full[buf], (uint32_t)((local >> 1) & 1));
       if (!ok) { if (lane == 0) atomicExch(status, 3); sm.dead = 1; }
@@ -249,7 +345,7 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
       tc_fence_after();
       const uint32_t acc = tmem + (uint32_t)buf * BN + ((uint32_t)(q * 32) << 16);
 #pragma unroll 1
-      for (int c = 0; c < BN; c += CH, ++chunk_no) {
+      for (int c = 0; c < n_cols; c += CH, ++chunk_no) {
         TC* stage_out = sm.out[chunk_no & 1];
         // the store that last used this buffer (two chunks ago) must have read it
         if (issuer) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
@@ -264,8 +360,11 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
             const int col0 = h * 16 + (lane < 16 ? 0 : 8);
             float r[8];
             if (EPI == EPI_CLAMPED) {
-              const float one[8] = {1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f};
-              clamped_columns<TC>(v, lane, act_limit, one, r);
+              float sc[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i)
+                sc[i] = GROUPED && grouping.row_scale ? grouping.row_scale[min(t0 + c + col0 + i, T - 1)] : 1.f;
+              clamped_columns<TC>(v, lane, act_limit, sc, r);
             } else {
               gated_columns<TC>(v, lane, r);
             }
@@ -273,11 +372,14 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
             for (int i = 0; i < 8; ++i) stage_out[(col0 + i) * FEAT + f] = from_f32<TC>(r[i]);
           } else {
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-              stage_out[(h * 16 + j) * FEAT + row] = from_f32<TC>(__uint_as_float(v[j]));
+            for (int j = 0; j < 16; ++j) {
+              float z = __uint_as_float(v[j]);
+              if (EPI == EPI_RELU2) z = relu_squared(z);
+              stage_out[(h * 16 + j) * FEAT + row] = from_f32<TC>(z);
+            }
           }
         }
-        if (c + CH >= BN) {           // this accumulator has been read completely
+        if (c + CH >= n_cols) {           // this accumulator has been read completely
           tc_fence_before();
           __syncwarp();
           if (lane == 0) {
@@ -317,25 +419,31 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
 // tiles than pairs some never work.  A work item costs its 64-wide blocks of K plus about six
 // blocks' worth of start and epilogue (fitted to measured times of seven shapes); K is cut into
 // the number of ranges, each of at least eight blocks, for which the rounds cost least.
-int cheapest_cut(int tiles, int nkb, int pairs, double* cost_of_it) {
+// The last tokens of a T that is not a multiple of 256 make shorter items, dealt last.
+double rounds_cost(int m_tiles, int T, int nkb, int pairs, int s) {
+  const int whole = m_tiles * (T / BN) * s, rest = T % BN ? m_tiles * s : 0;
+  const int first = (whole + pairs - 1) / pairs, all = (whole + rest + pairs - 1) / pairs;
+  return first * ((double)nkb / s + 6.0) + (all - first) * ((double)nkb / s * (0.25 + 0.75 * (T % BN) / BN) + 5.0);
+}
+int cheapest_cut(int m_tiles, int T, int nkb, int pairs, double* cost_of_it) {
   int ksplits = 1;
   double best = 0;
   for (int s = 1; s <= 8 && (s == 1 || nkb / s >= 8); ++s) {
-    const int rounds = (tiles * s + pairs - 1) / pairs;
-    const double cost = rounds * ((double)nkb / s + 6.0);
+    const double cost = rounds_cost(m_tiles, T, nkb, pairs, s);
     if (s == 1 || cost < best * 0.99) best = cost, ksplits = s;
   }
   *cost_of_it = best;
   return ksplits;
 }
 
-template <int STAGES, int EPI, typename TC>
-int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mc, int T, int N, int K, int half,
-           int sm_count, int* status, cudaStream_t stream, float act_limit = 0.f) {
-  constexpr bool GATED = gated_epilogue(EPI);
+template <int STAGES, int EPI, typename TC, int FORM>
+int launch_form(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mxs, const CUtensorMap& mc, int T, int N,
+           int K, int half, int sm_count, int* status, cudaStream_t stream, float act_limit = 0.f,
+           const Grouping& grouping = Grouping()) {
+  constexpr bool GATED = gated_epilogue(EPI), GROUPED = FORM == GROUPED_TILES;
   constexpr int FEAT = GATED ? 64 : TILE_M;
-  auto kernel = gemm_pair_kernel<STAGES, EPI, TC>;
-  constexpr int smem = (int)sizeof(PairStorage<STAGES, FEAT, TC>) + 1024;
+  auto kernel = gemm_pair_kernel<STAGES, EPI, TC, FORM>;
+  constexpr int smem = (int)sizeof(PairStorage<STAGES, FEAT, TC, GROUPED>) + 1024;
   static_assert(smem <= 227 * 1024, "the stages and output chunks fit one SM");
   static bool configured = false;
   if (!configured) {
@@ -344,7 +452,7 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mc, 
     configured = true;
   }
   const int limit = GATED ? half : N;
-  const int m_tiles = (limit + 2 * FEAT - 1) / (2 * FEAT), n_tiles = (T + BN - 1) / BN;
+  const int m_tiles = (limit + 2 * FEAT - 1) / (2 * FEAT), n_tiles = GROUPED ? grouping.n_small : (T + BN - 1) / BN;
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(192);
   cfg.dynamicSmemBytes = smem;
@@ -373,7 +481,7 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mc, 
   if (EPI == EPI_ACCUM) {
     const int nkb = (K + TILE_K - 1) / TILE_K;
     double cost;
-    ksplits = cheapest_cut(m_tiles * n_tiles, nkb, resident_pairs, &cost);
+    ksplits = cheapest_cut(m_tiles, T, nkb, resident_pairs, &cost);
     if (g_llm_pair_ksplits > 0 && nkb / g_llm_pair_ksplits >= 1) ksplits = g_llm_pair_ksplits;
   }
   const int works = m_tiles * n_tiles * ksplits;
@@ -382,7 +490,16 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mc, 
   // directly behind the rotation kernel the pair kernel starts only when that kernel is done
   cfg.numAttrs = (g_llm_pdl && !g_llm_after_rotation) ? 2 : 1;
   g_llm_after_rotation = 0;
-  return (int)cudaLaunchKernelEx(&cfg, kernel, mw, mx, mc, T, N, K, half, m_tiles, n_tiles, ksplits, act_limit, status);
+  return (int)cudaLaunchKernelEx(&cfg, kernel, mw, mx, mxs, mc, T, N, K, half, m_tiles, n_tiles, ksplits, act_limit, status,
+                                 grouping);
+}
+
+template <int STAGES, int EPI, typename TC>
+int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mxs, const CUtensorMap& mc, int T, int N,
+           int K, int half, int sm_count, int* status, cudaStream_t stream, float act_limit = 0.f) {
+  if (T % BN)
+    return launch_form<STAGES, EPI, TC, LAST_TOKENS>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream, act_limit);
+  return launch_form<STAGES, EPI, TC, WHOLE_TILES>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream, act_limit);
 }
 }  // namespace
 
@@ -397,11 +514,11 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mc, 
 // 18.4 on pairs).
 int llm_pair_store_way(int T, int N, int K, int splits) {
   const int pairs = 74, nkb = (K + TILE_K - 1) / TILE_K;
-  const int tiles = ((N + 2 * TILE_M - 1) / (2 * TILE_M)) * ((T + BN - 1) / BN);
+  const int m_tiles = (N + 2 * TILE_M - 1) / (2 * TILE_M);
   const double clear = (2.5 + (double)T * N * 4 / 3e6) / 0.39;
-  const double whole = ((tiles + pairs - 1) / pairs) * (nkb + 6.0);
+  const double whole = rounds_cost(m_tiles, T, nkb, pairs, 1);
   double cut;
-  if (cheapest_cut(tiles, nkb, pairs, &cut) == 1) cut = 1e30;
+  if (cheapest_cut(m_tiles, T, nkb, pairs, &cut) == 1) cut = 1e30;
   const long long lone = (long long)((N + TILE_M - 1) / TILE_M) * ((T + 127) / 128) * splits;
   const double alone = (double)((lone + 4 * pairs - 1) / (4 * pairs)) * (1.4 * nkb / splits + 6.0) + clear;
   if (alone < whole && alone < cut + clear) return 2;
@@ -416,9 +533,7 @@ int g_llm_pair_ksplits = 0;   // > 0: this many ranges of K in the adding epilog
 LLM_EXPORT void llm_set_pair_ksplits(int n) { g_llm_pair_ksplits = n; }
 LLM_EXPORT void llm_set_pair(int on) { g_llm_pair = on ? 1 : 0; }
 
-int llm_gemm_tcgen05_pair(const void* X, const void* W, void* C, int c_dtype, int T, int N, int K, int lda,
-                          int ldw, int ldc, int mode, int half, float limit, int* status, cudaStream_t stream) {
-  if (!g_llm_pair) return LLM_ERR_UNSUPPORTED;
+static int pair_sm_count() {
   static int sm_count = 0;
   if (!sm_count) {
     int dev = 0;
@@ -426,27 +541,67 @@ int llm_gemm_tcgen05_pair(const void* X, const void* W, void* C, int c_dtype, in
     cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
     if (sm_count <= 0) sm_count = 148;
   }
+  return sm_count;
+}
+
+int llm_gemm_tcgen05_pair(const void* X, const void* W, void* C, int c_dtype, int T, int N, int K, int lda,
+                          int ldw, int ldc, int mode, int half, float limit, int* status, cudaStream_t stream) {
+  if (!g_llm_pair) return LLM_ERR_UNSUPPORTED;
+  const int sm_count = pair_sm_count();
   if (mode != 0 && mode != 1 && mode != 3 && mode != 4) return LLM_ERR_UNSUPPORTED;
   const int esize = c_dtype == LLM_F32 ? 4 : 2;
   if (((uintptr_t)C & 15) || ((size_t)ldc * esize) % 16) return LLM_ERR_UNSUPPORTED;
-  CUtensorMap mw, mx, mc;
+  CUtensorMap mw, mx, mxs, mc;
   if (!llm_tensor_map(W, N, K, ldw, TILE_M, TILE_K, 0, &mw)) return LLM_ERR_UNSUPPORTED;
   if (!llm_tensor_map(X, T, K, lda, HALF_N, TILE_K, 0, &mx)) return LLM_ERR_UNSUPPORTED;
+  if (!llm_tensor_map(X, T, K, lda, HALF_N / 2, TILE_K, 0, &mxs)) return LLM_ERR_UNSUPPORTED;
   const int out_cols = mode >= 3 ? half : N;
   if (!llm_tensor_map(C, T, out_cols, ldc, CH, mode >= 3 ? 64 : TILE_M, c_dtype == LLM_F32 ? 2 : 1, &mc))
     return LLM_ERR_UNSUPPORTED;
   if (mode == 0) {
-    if (c_dtype == LLM_F32) return launch<5, EPI_STORE, float>(mw, mx, mc, T, N, K, half, sm_count, status, stream);
-    if (c_dtype == LLM_BF16) return launch<6, EPI_STORE, bf16>(mw, mx, mc, T, N, K, half, sm_count, status, stream);
+    if (c_dtype == LLM_F32) return launch<5, EPI_STORE, float>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream);
+    if (c_dtype == LLM_BF16) return launch<6, EPI_STORE, bf16>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream);
   } else if (mode == 1) {
-    if (c_dtype == LLM_F32) return launch<5, EPI_ACCUM, float>(mw, mx, mc, T, N, K, half, sm_count, status, stream);
+    if (c_dtype == LLM_F32) return launch<5, EPI_ACCUM, float>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream);
   } else {
     if (N != 2 * half || half % 16) return LLM_ERR_ARGUMENT;
     if (mode == 4)
-      return c_dtype == LLM_BF16 ? launch<6, EPI_CLAMPED, bf16>(mw, mx, mc, T, N, K, half, sm_count, status, stream, limit)
+      return c_dtype == LLM_BF16 ? launch<6, EPI_CLAMPED, bf16>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream, limit)
                                  : LLM_ERR_UNSUPPORTED;
-    if (c_dtype == LLM_BF16) return launch<6, EPI_GATED, bf16>(mw, mx, mc, T, N, K, half, sm_count, status, stream);
-    if (c_dtype == LLM_F32) return launch<6, EPI_GATED, float>(mw, mx, mc, T, N, K, half, sm_count, status, stream);
+    if (c_dtype == LLM_BF16) return launch<6, EPI_GATED, bf16>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream);
+    if (c_dtype == LLM_F32) return launch<6, EPI_GATED, float>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream);
   }
   return LLM_ERR_UNSUPPORTED;
+}
+
+// The grouped product of llm_gemm_tcgen05_grouped on CTA pairs: tile i of bn rows of X (32, 64 or 128)
+// with matrix tile_group[i] of W, at most 512 tiles.  mode 0: C f32; 3 and 4: the gated forms with
+// interleaved rows, C bf16 [T][half]; 5: C = max(X W_g^T, 0)^2, bf16.
+LLM_EXPORT int llm_gemm_tcgen05_grouped_pair(const void* X, const void* W, void* C, int c_dtype, int T, int N, int K,
+                                             int lda, int ldw, int ldc, int mode, int half, int bn, int groups,
+                                             const int* tile_group, float limit, const float* row_scale, int* status,
+                                             cudaStream_t stream) {
+  if (T <= 0 || N <= 0 || groups <= 0) return 0;
+  if (!tile_group || (mode != 0 && mode != 3 && mode != 4 && mode != 5)) return LLM_ERR_ARGUMENT;
+  const bool gated = mode == 3 || mode == 4;
+  if (gated && (N != 2 * half || half % 16)) return LLM_ERR_ARGUMENT;
+  if (bn != 32 && bn != 64 && bn != 128) return LLM_ERR_UNSUPPORTED;
+  if (K <= 0 || K % 8 || lda % 8 || ldw % 8 || (((uintptr_t)X | (uintptr_t)W) & 15)) return LLM_ERR_UNSUPPORTED;
+  if ((long long)groups * N > 0x7fffffffLL || (mode == 0) != (c_dtype == LLM_F32)) return LLM_ERR_UNSUPPORTED;
+  const int esize = c_dtype == LLM_F32 ? 4 : 2;
+  if (((uintptr_t)C & 15) || ((size_t)ldc * esize) % 16) return LLM_ERR_UNSUPPORTED;
+  Grouping g;
+  g.tile_group = tile_group, g.bn = bn, g.n_small = (T + bn - 1) / bn, g.group_rows = N, g.row_scale = row_scale;
+  if (g.n_small > MAX_SMALL) return LLM_ERR_UNSUPPORTED;
+  CUtensorMap mw, mx, mxs, mc;
+  if (!llm_tensor_map(W, (long long)groups * N, K, ldw, TILE_M, TILE_K, 0, &mw)) return LLM_ERR_UNSUPPORTED;
+  if (!llm_tensor_map(X, T, K, lda, HALF_N, TILE_K, 0, &mx)) return LLM_ERR_UNSUPPORTED;
+  if (!llm_tensor_map(X, T, K, lda, HALF_N / 2, TILE_K, 0, &mxs)) return LLM_ERR_UNSUPPORTED;
+  if (!llm_tensor_map(C, T, gated ? half : N, ldc, CH, gated ? 64 : TILE_M, c_dtype == LLM_F32 ? 2 : 1, &mc))
+    return LLM_ERR_UNSUPPORTED;
+  const int sms = pair_sm_count();
+  if (mode == 0) return launch_form<5, EPI_STORE, float, GROUPED_TILES>(mw, mx, mxs, mc, T, N, K, half, sms, status, stream, 0.f, g);
+  if (mode == 3) return launch_form<6, EPI_GATED, bf16, GROUPED_TILES>(mw, mx, mxs, mc, T, N, K, half, sms, status, stream, 0.f, g);
+  if (mode == 4) return launch_form<6, EPI_CLAMPED, bf16, GROUPED_TILES>(mw, mx, mxs, mc, T, N, K, half, sms, status, stream, limit, g);
+  return launch_form<6, EPI_RELU2, bf16, GROUPED_TILES>(mw, mx, mxs, mc, T, N, K, half, sms, status, stream, 0.f, g);
 }

@@ -116,6 +116,7 @@ def _signatures():
         "llm_moe_gather": [P, P, P, I, I, I, I, P, I, P, P, P],
         "llm_moe_combine": [P, P, P, P, P, I, P, I, I, I, I, I, P, I, P, I, I, P],
         "llm_gemm_tcgen05_grouped": [P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, F, P, P, P],
+        "llm_gemm_tcgen05_grouped_pair": [P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, F, P, P, P],
         "llm_gemm_tcgen05_clamped": [P, P, P, I, I, I, I, I, I, I, F, P, P],
         "llm_gemm_tcgen05_batched": [P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P],
         "llm_moe_gate_up_rows": [P, P, P, P, I, I, I, I, I, I, I, F, P, I, P],
@@ -914,6 +915,9 @@ def _tc_ok(a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None)
             and w.stride(1) == 1 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
+_cta_pairs = True
+
+
 def use_cta_pairs(on: bool) -> None:
     """Whether products of many rows run on CTA pairs (tcgen05 cta_group::2; the default) or on
     the one-CTA persistent kernel.  For comparisons."""
@@ -921,6 +925,8 @@ def use_cta_pairs(on: bool) -> None:
     l.llm_set_pair.argtypes = [c_int]
     l.llm_set_pair.restype = None
     l.llm_set_pair(int(on))
+    global _cta_pairs
+    _cta_pairs = bool(on)
 
 
 def force_pair_k_ranges(n: int) -> None:
@@ -1731,6 +1737,19 @@ def moe_tile(pairs: int, experts: int) -> int:
     return 128
 
 
+MOE_PAIR_TILE = 64       # rows of a tile for the grouped products on CTA pairs
+
+
+def moe_pairs(pairs: int, experts: int) -> bool:
+    """Whether the grouped products of so many (token, expert) pairs run on CTA pairs
+    (:func:`gemm_grouped` with ``paired``), in tiles of MOE_PAIR_TILE rows that the kernel joins
+    to as many as 256: once an expert's average share fills half of that (1,024 pairs on eight
+    experts of 6,144 x 4,096: 126 -> 107 us for the first product with its activation), and while
+    its list of tiles has room."""
+    return (_cta_pairs and pairs >= 128 * experts
+            and -(-pairs // MOE_PAIR_TILE) + experts <= 512)
+
+
 def moe_align(ids: torch.Tensor, experts: int, bn: int, pos: torch.Tensor,
               tile_group: torch.Tensor) -> None:
     """Sort the (row, choice) pairs of ``ids`` by expert: ``pos`` (int32 [pairs]) is each pair's
@@ -1791,17 +1810,23 @@ def moe_combine(d: torch.Tensor, pos: torch.Tensor, wts: Optional[torch.Tensor],
 
 def gemm_grouped(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tile_group: torch.Tensor,
                  bn: int, gated: bool, interleaved: bool = False, activation: str = "silu",
-                 limit: float = 0.0, row_scale: Optional[torch.Tensor] = None) -> None:
+                 limit: float = 0.0, row_scale: Optional[torch.Tensor] = None,
+                 paired: bool = False) -> None:
     """The tensor-core product with a matrix per tile of ``bn`` rows of ``a``: tile t uses
     ``w[tile_group[t]]`` (w [groups, N, K] bfloat16; a negative entry leaves the tile out).
     ``gated``: w[g] = [gate; up] and out = silu(a gate^T) * (a up^T) ([rows, N / 2]);
     ``interleaved``: w[g] has its rows as 16 gate rows, their 16 up rows, ...; with interleaved
     rows ``activation="clamped_swish"`` (``limit``; see :func:`gated_act`) and ``row_scale``
-    (float32 [rows], a factor per row on both products in front of it) are there as well."""
+    (float32 [rows], a factor per row on both products in front of it) are there as well.
+    ``paired``: on CTA pairs, which join neighbouring tiles of one matrix (bn 32, 64 or 128, at
+    most 512 tiles; float32 ``out``, or interleaved rows, or without a gate
+    ``activation="relu_squared"`` and bfloat16 ``out``: the square of the positive part)."""
     _cuda(a, w, out, tile_group, row_scale)
     mode = 0 if not gated else 2
     if gated and interleaved:
         mode = {"silu": 3, "clamped_swish": 4}[activation]
+    elif paired and not gated and activation == "relu_squared":
+        mode = 5
     elif activation != "silu":
         raise KernelError(f"the grouped product with rows [gate; up] has no '{activation}'")
     assert row_scale is None or (mode == 4 and row_scale.dtype == torch.float32
@@ -1810,8 +1835,8 @@ def gemm_grouped(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tile_group
     G, N, _ = w.shape
     assert a.dtype == w.dtype == torch.bfloat16 and a.is_contiguous() and w.is_contiguous()
     assert out.stride(1) == 1 and tile_group.numel() * bn >= T
-    _check(lib().llm_gemm_tcgen05_grouped(_ptr(a), _ptr(w), _ptr(out), _dt(out), T, N, K,
-                                          a.stride(0), K, out.stride(0), mode,
-                                          N // 2 if gated else 0, bn, G, _ptr(tile_group),
-                                          float(limit), _ptr(row_scale),
-                                          _ptr(tc_status(a.device)), _stream()), "gemm_grouped")
+    l = lib()
+    _check((l.llm_gemm_tcgen05_grouped_pair if paired else l.llm_gemm_tcgen05_grouped)(
+        _ptr(a), _ptr(w), _ptr(out), _dt(out), T, N, K, a.stride(0), K, out.stride(0), mode,
+        N // 2 if gated else 0, bn, G, _ptr(tile_group), float(limit), _ptr(row_scale),
+        _ptr(tc_status(a.device)), _stream()), "gemm_grouped")

@@ -299,7 +299,8 @@ class RoutedExperts:
         if kernels.moe_grouped_ok(h.dtype, self.hidden, self.ff) and self.grouped:
             # sorted by expert into tiles of rows, two grouped tensor-core products, one sum
             pairs = rows * top
-            bn = kernels.moe_tile(pairs, E)
+            paired = kernels.moe_pairs(pairs, E) and (self.interleaved or not self.gated)
+            bn = kernels.MOE_PAIR_TILE if paired else kernels.moe_tile(pairs, E)
             tiles = -(-pairs // bn) + E
             pos = ctx.buffer("moe.pos", (pairs,), torch.int32)
             tile_group = ctx.buffer("moe.tiles", (tiles,), torch.int32)
@@ -314,13 +315,16 @@ class RoutedExperts:
             if self.gated:
                 kernels.gemm_grouped(xp, self.gate_up, act, tile_group, bn, gated=True,
                                      interleaved=True, activation=self.activation,
-                                     limit=self.limit, row_scale=scale)
+                                     limit=self.limit, row_scale=scale, paired=paired)
+            elif paired:
+                kernels.gemm_grouped(xp, self.gate_up, act, tile_group, bn, gated=False,
+                                     activation=self.activation, paired=True)
             else:
                 u = ctx.buffer("moe.up", (tiles * bn, self.ff), torch.float32)
                 kernels.gemm_grouped(xp, self.gate_up, u, tile_group, bn, gated=False)
                 kernels.act_rows(u, act, self.activation)
             d = ctx.buffer("moe.down", (tiles * bn, self.hidden), torch.float32)
-            kernels.gemm_grouped(act, self.down, d, tile_group, bn, gated=False)
+            kernels.gemm_grouped(act, self.down, d, tile_group, bn, gated=False, paired=paired)
             kernels.moe_combine(d, pos, wts if scale is None else None, x, accumulate, shared, gate, clear_shared=kept_zero,
                                 ids=ids if self.identity else None, experts=E,
                                 identity_input=ident)

@@ -198,3 +198,66 @@ def test_uniforms_of_many_streams():
         next_uniforms([mine[0], None, mine[1], mine[2], mine[0]], ctypes.addressof(out))
         assert list(out) == [alone[0].next_f64(), 0.0, alone[1].next_f64(), alone[2].next_f64(), alone[0].next_f64()]
     assert mine[3].next_u64() == alone[3].next_u64()
+
+
+@gpu
+@pytest.mark.parametrize("bn", (32, 64, 128))
+@pytest.mark.parametrize("counts,N,K", [([300, 0, 1, 129, 256, 64], 512, 256), ([700, 33, 32], 272, 72),
+                                        ([0, 0, 5], 96, 200), ([64] * 40, 64, 64)])
+def test_grouped_products_on_cta_pairs(counts, N, K, bn):
+    """Tiles of one matrix joined to as many as 256 rows, matrices without rows, ragged N and K, every
+    epilogue; padding rows hold NaN and rows of matrices without tiles are not written."""
+    from llmario_b200 import kernels
+    E = len(counts)
+    tiles = [-(-c // bn) for c in counts]
+    T = (sum(tiles) + 2) * bn                       # two tiles that are left out
+    x = torch.full((T, K), float("nan"), dtype=torch.bfloat16, device=DEV)
+    group, rows, expert = [], [], []
+    for e, c in enumerate(counts):
+        rows += range(len(group) * bn, len(group) * bn + c)
+        expert += [e] * c
+        group += [e] * tiles[e]
+    x[rows] = rnd(len(rows), K, dtype=torch.bfloat16, seed=1)
+    tg = torch.tensor(group + [-1, -1], dtype=torch.int32, device=DEV)
+    w = rnd(E, N, K, dtype=torch.bfloat16, seed=2, scale=K ** -0.5)
+    scale = torch.full((T,), float("nan"), device=DEV)
+    scale[rows] = rnd(len(rows), seed=3).abs()
+    ex = torch.tensor(expert, device=DEV)
+    xr = x[rows].double()
+    ref = torch.zeros(len(rows), N, dtype=torch.float64, device=DEV)
+    size = torch.zeros_like(ref)
+    for e in range(E):
+        ref[ex == e] = xr[ex == e] @ w[e].double().T
+        size[ex == e] = xr[ex == e].abs() @ w[e].abs().double().T
+    out = torch.full((T, N), 7.0, device=DEV)
+    kernels.gemm_grouped(x, w, out, tg, bn, gated=False, paired=True)
+    assert bool(((out[rows].double() - ref).abs() <= (K + 10) * 2 ** -23 * size).all())
+    assert bool((out[sum(tiles) * bn:] == 7.0).all())
+    r2 = torch.full((T, N), 7.0, dtype=torch.bfloat16, device=DEV)
+    kernels.gemm_grouped(x, w, r2, tg, bn, gated=False, activation="relu_squared", paired=True)
+    want = ref.clamp(min=0) ** 2
+    # 32-bit sums, squared, rounded to 8 bits of mantissa
+    assert bool(((r2[rows].double() - want).abs() <= 2 ** -8 * want + (K + 10) * 2 ** -21 * size * (size + 1)).all())
+    kernels.check_tc_status(torch.device(DEV))
+    if N % 32:
+        return
+    half = N // 2
+    blocks = ref.view(len(rows), N // 32, 2, 16)
+    gate, up = blocks[:, :, 0].reshape(-1, half), blocks[:, :, 1].reshape(-1, half)
+    act = torch.full((T, half), 7.0, dtype=torch.bfloat16, device=DEV)
+    one = torch.empty(T, half, dtype=torch.bfloat16, device=DEV)
+    for kw in (dict(), dict(activation="clamped_swish", limit=0.8, row_scale=scale)):
+        kernels.gemm_grouped(x, w, act, tg, bn, gated=True, interleaved=True, paired=True, **kw)
+        kernels.gemm_grouped(x, w, one, tg, bn, gated=True, interleaved=True, **kw)
+        if kw:
+            s = scale[rows].double()[:, None]
+            g, u = (gate * s).clamp(max=0.8), (up * s).clamp(-0.8, 0.8)
+            want = g * torch.sigmoid(1.702 * g) * (u + 1)
+        else:
+            want = gate * torch.sigmoid(gate) * up
+        # rounding of the result, and of 32-bit sums in front of functions with slopes below 2
+        bound = 2 ** -8 * want.abs() + 1e-5 * (1 + want.abs())
+        assert bool(((act[rows].double() - want).abs() <= bound).all())
+        assert torch.equal(act[rows], one[rows])       # the same sums in the same order
+        assert bool((act[sum(tiles) * bn:] == 7.0).all())
+    kernels.check_tc_status(torch.device(DEV))
