@@ -34,6 +34,9 @@ extern "C" {
 int llm_rms_norm(const float* x, const float* w, void* y, int out_dtype, const int* rows_index, int rows,
                  int width, float eps, cudaStream_t stream);
 int llm_silu_mul(const float* gate_up, void* out, int out_dtype, int rows, int ff, cudaStream_t stream);
+int llm_row_product_ok(int rows, int N, int K, int gated);
+int llm_row_product(const void* x, int ldx, const float* norm_w, float eps, const void* W, void* out, int ldc, int rows,
+                    int N, int K, int mode, int* status, cudaStream_t stream);
 int llm_gemm_simt(const void* A, int a_dtype, const void* W, int w_dtype, void* C, int c_dtype, int M, int N,
                   int K, int lda, int ldw, int ldc, int accumulate, cudaStream_t stream);
 int llm_gemm_tcgen05(const void* X, const void* W, void* C, int c_dtype, int T, int N, int K, int lda, int ldw,
@@ -178,9 +181,10 @@ int g_fuse_mode = 0;                        // 0: when few waves, 1: always, 2: 
 enum Kind : int {
   K_NORM, K_GEMM_TCGEN05, K_GEMM_SIMT, K_ROPE_TABLE, K_ROPE_STORE, K_DECODE_FUSED, K_DECODE_TMA, K_DECODE,
   K_FLASH, K_MERGE, K_TCGEN05, K_TCGEN05_X2, K_GENERIC, K_SILU_MUL, K_KV_GATHER, K_DECODE_PERSISTENT,
-  K_EXTRAS, K_LATENT, N_KINDS
+  K_EXTRAS, K_LATENT, K_ROW_PRODUCT, N_KINDS
 };
 long long g_counts[N_KINDS] = {};
+int g_row_product = 1;      // 0: every product by the kernels for more rows (for comparisons)
 
 int sm_count() {
   static int n = 0;
@@ -371,9 +375,19 @@ struct Run {
 
   int buffer(long long key, size_t bytes, void** out, bool zero = false) { return ar.get(key, bytes, zero, out); }
 
+  // whether a product of this step's rows with w goes to the kernel for one or two rows and small
+  // matrices (row_product.cu), which can make the norm of 32-bit rows itself
+  bool row_product_ok(const void* x, int ldx, const void* w, int w_dt, int ldw, int n, int k, bool gated) const {
+    return g_row_product && st.dtype == LLM_BF16 && w_dt == LLM_BF16 && ldw == k && ldx % 8 == 0 && aligned16(x) &&
+           aligned16(w) && llm_row_product_ok(st.rows, n, k, gated ? 1 : 0);
+  }
+
   // out (=|+=) a @ w^T with the fastest kernel that takes the operands (kernels.linear)
   int linear(const void* a, int a_dt, int lda, const void* w, int w_dt, int ldw, void* out, int out_dt, int ldc,
              int rows, int n, int k, bool accumulate, bool out_is_zero) {
+    if (a_dt == LLM_BF16 && out_dt == LLM_F32 && rows == st.rows && row_product_ok(a, lda, w, w_dt, ldw, n, k, false))
+      return check(llm_row_product(a, lda, nullptr, 0.f, w, out, ldc, rows, n, k, accumulate ? 1 : 0, st.status, stream),
+                   K_ROW_PRODUCT);
     if (tc_ok(a, a_dt, lda, w, w_dt, ldw, k)) {
       const int splits = out_dt == LLM_F32 ? llm_k_splits(rows, n, k) : 1;
       return check(llm_gemm_tcgen05(a, w, out, out_dt, rows, n, k, lda, ldw, ldc, accumulate ? 1 : 0, 0,
@@ -751,6 +765,7 @@ struct Run {
   }
 
   // the mixer: projections, per-head norm, rotation, cache write, attention, output projection
+  // (h null: the product of x's rows makes their norm itself)
   int mixer(const LlmLayerDesc& L, const LlmCallDesc& c, const void* h, float* x) {
     const int rows = st.rows, Hq = L.num_heads, Hkv = L.num_kv_heads, hd = L.head_dim;
     const int q_width = Hq * hd, kv_width = Hkv * hd, dt = st.dtype;
@@ -762,8 +777,12 @@ struct Run {
     int rc = buffer(kept_zero ? B_ZPROJ * 1000000LL + width : (long long)B_PROJ, (size_t)rows * width * 4, &proj,
                     kept_zero);
     if (rc) return rc;
-    rc = linear(h, dt, L.hidden, L.w_qkv, L.w_qkv_dtype, L.hidden, proj, LLM_F32, width, rows, width, L.hidden,
-                false, kept_zero);
+    if (h == nullptr)
+      rc = check(llm_row_product(x, L.hidden, L.mixer_norm_w, L.mixer_norm_eps, L.w_qkv, proj, width, rows, width,
+                                 L.hidden, 0, st.status, stream), K_ROW_PRODUCT);
+    else
+      rc = linear(h, dt, L.hidden, L.w_qkv, L.w_qkv_dtype, L.hidden, proj, LLM_F32, width, rows, width, L.hidden,
+                  false, kept_zero);
     if (rc) return rc;
     const float* cos_sin = nullptr;
     rc = rope_table(L, &cos_sin);
@@ -813,6 +832,12 @@ struct Run {
     void* act = nullptr;
     int rc = buffer(B_ACT, (size_t)rows * ff * esize(dt), &act);
     if (rc) return rc;
+    if (h == nullptr) {
+      rc = check(llm_row_product(x, L.hidden, L.ffn_norm_w, L.ffn_norm_eps, L.w_gate_up, act, ff, rows, ff, L.hidden, 2,
+                                 st.status, stream), K_ROW_PRODUCT);
+      if (rc) return rc;
+      return linear(act, dt, ff, L.w_down, L.w_down_dtype, ff, x, LLM_F32, L.hidden, rows, L.hidden, ff, true, false);
+    }
     const bool tc = tc_ok(h, dt, L.hidden, L.w_gate_up, L.w_gate_up_dtype, L.hidden, L.hidden);
     if (L.interleaved && !tc) return LLM_ERR_UNSUPPORTED;
     if (tc) {
@@ -835,17 +860,29 @@ struct Run {
     void* h = nullptr;
     int rc = buffer(B_H, (size_t)st.rows * L.hidden * esize(st.dtype), &h);
     if (rc) return rc;
-    rc = check(llm_rms_norm(st.x, L.mixer_norm_w, h, st.dtype, nullptr, st.rows, L.hidden, L.mixer_norm_eps, stream), K_NORM);
+    const int width = (L.num_heads + (c.writes_cache ? 2 * L.num_kv_heads : 0)) * L.head_dim;
+    const bool small_qkv = aligned16(L.mixer_norm_w) &&
+                           row_product_ok(st.x, L.hidden, L.w_qkv, L.w_qkv_dtype, L.hidden, width, L.hidden, false);
+    if (!small_qkv) {
+      rc = check(llm_rms_norm(st.x, L.mixer_norm_w, h, st.dtype, nullptr, st.rows, L.hidden, L.mixer_norm_eps, stream), K_NORM);
+      if (rc) return rc;
+    }
+    rc = mixer(L, c, small_qkv ? nullptr : h, st.x);
     if (rc) return rc;
-    rc = mixer(L, c, h, st.x);
-    if (rc) return rc;
-    rc = check(llm_rms_norm(st.x, L.ffn_norm_w, h, st.dtype, nullptr, st.rows, L.hidden, L.ffn_norm_eps, stream), K_NORM);
-    if (rc) return rc;
-    return feed_forward(L, h, st.x);
+    const bool small_ffn = L.interleaved && aligned16(L.ffn_norm_w) && L.intermediate % 16 == 0 &&
+                           row_product_ok(st.x, L.hidden, L.w_gate_up, L.w_gate_up_dtype, L.hidden, L.intermediate,
+                                          L.hidden, true);
+    if (!small_ffn) {
+      rc = check(llm_rms_norm(st.x, L.ffn_norm_w, h, st.dtype, nullptr, st.rows, L.hidden, L.ffn_norm_eps, stream), K_NORM);
+      if (rc) return rc;
+    }
+    return feed_forward(L, small_ffn ? nullptr : h, st.x);
   }
 };
 
 }  // namespace
+
+LLM_EXPORT void llm_set_row_product(int on) { g_row_product = on ? 1 : 0; }
 
 // ---- policies, exported so that the Python statement of the same rules can be held to them
 LLM_EXPORT int llm_token_tile(int rows) {

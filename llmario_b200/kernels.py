@@ -117,6 +117,8 @@ def _signatures():
         "llm_moe_combine": [P, P, P, P, P, I, P, I, I, I, I, I, P, I, P, I, I, P],
         "llm_gemm_tcgen05_grouped": [P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, F, P, P, P],
         "llm_gemm_tcgen05_grouped_pair": [P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, F, P, P, P],
+        "llm_row_product_ok": [I, I, I, I],
+        "llm_row_product": [P, I, P, F, P, P, I, I, I, I, I, P, P],
         "llm_gemm_tcgen05_clamped": [P, P, P, I, I, I, I, I, I, I, F, P, P],
         "llm_gemm_tcgen05_batched": [P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, P],
         "llm_moe_gate_up_rows": [P, P, P, P, I, I, I, I, I, I, I, F, P, I, P],
@@ -1009,6 +1011,30 @@ def k_splits(rows: int, out_features: int, in_features: int) -> int:
     return max(1, min(16, round(2 * sm_count() / tiles), in_features // 256))
 
 
+def row_product_ok(rows: int, out_features: int, in_features: int, gated: bool = False) -> bool:
+    """Whether :func:`row_product` takes these sizes: one or two rows, a matrix of a few MB."""
+    return rows <= 2 and bool(lib().llm_row_product_ok(rows, out_features, in_features, int(gated)))
+
+
+def row_product(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False,
+                gated: bool = False, norm_weight: Optional[torch.Tensor] = None,
+                eps: float = 0.0) -> None:
+    """out (=|+=) h @ w.T for one or two rows, ``out`` float32; with ``gated`` (``w`` as blocks of 16
+    gate rows and 16 up rows) ``out = silu(gate) * up`` in bfloat16.  ``x`` is h in bfloat16 or, with
+    ``norm_weight``, float32 rows whose RMS norm, rounded to bfloat16, is h."""
+    _cuda(x, w, out, norm_weight)
+    rows, k = x.shape
+    n = w.shape[0] // (2 if gated else 1)
+    assert w.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[1] == k
+    assert x.dtype == (torch.bfloat16 if norm_weight is None else torch.float32)
+    assert x.stride(1) == 1 and out.stride(1) == 1 and out.shape == (rows, n)
+    assert out.dtype == (torch.bfloat16 if gated else torch.float32) and not (gated and accumulate)
+    _check(lib().llm_row_product(_ptr(x), x.stride(0), _ptr(norm_weight), float(eps), _ptr(w),
+                                 _ptr(out), out.stride(0), rows, n, k,
+                                 2 if gated else int(accumulate), _ptr(tc_status(x.device)),
+                                 _stream()), "row_product")
+
+
 def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False,
            out_is_zero: bool = False) -> None:
     """out (=|+=) a @ w.T with the fastest hand-written kernel that takes these operands:
@@ -1016,7 +1042,10 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool
     CUDA-core kernels for everything else (32-bit operands, unaligned sizes).
     ``out_is_zero``: the caller guarantees that ``out`` holds zeros, so a split-K product need
     not clear it first."""
-    if _tc_ok(a, w, out):
+    if (a.shape[0] <= 2 and out.dtype == torch.float32 and _tc_ok(a, w) and w.is_contiguous()
+            and out.stride(1) == 1 and row_product_ok(a.shape[0], w.shape[0], a.shape[1])):
+        row_product(a, w, out, accumulate)
+    elif _tc_ok(a, w, out):
         rows, k = a.shape
         n = w.shape[0]
         splits = k_splits(rows, n, k) if out.dtype == torch.float32 else 1

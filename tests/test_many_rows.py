@@ -261,3 +261,43 @@ def test_grouped_products_on_cta_pairs(counts, N, K, bn):
         assert torch.equal(act[rows], one[rows])       # the same sums in the same order
         assert bool((act[sum(tiles) * bn:] == 7.0).all())
     kernels.check_tc_status(torch.device(DEV))
+
+
+@gpu
+@pytest.mark.parametrize("rows", (1, 2))
+@pytest.mark.parametrize("N,K", [(1024, 2048), (4096, 1024), (1024, 3072), (148, 1024), (7, 2048), (3056, 1024)])
+def test_row_product(rows, N, K):
+    """One or two rows through a small matrix: stored, added, gated, of 16-bit rows and of the norm of
+    32-bit rows; fewer outputs than SMs, slices that do not come out even, strided rows."""
+    from llmario_b200 import kernels
+    if not kernels.row_product_ok(rows, N, K):
+        assert K == 3072 and rows == 2
+        return
+    x = rnd(rows, K + 8, seed=1)[:, :K]
+    h = rnd(rows, K + 8, dtype=torch.bfloat16, seed=2)[:, :K]
+    g = 1 + 0.1 * rnd(K, seed=3)
+    w = rnd(N, K, dtype=torch.bfloat16, seed=4, scale=K ** -0.5)
+    xd = x.double()
+    normed = (xd * torch.rsqrt((xd * xd).mean(-1, keepdim=True) + 1e-6) * g.double())
+    out = torch.full((rows, N + 4), float("nan"), device=DEV)
+    for src, kw, exact in ((h, {}, h.double()), (x, dict(norm_weight=g, eps=1e-6), normed)):
+        ref = exact @ w.double().T
+        size = exact.abs() @ w.double().abs().T
+        # 32-bit sums; a normed row is rounded to 8 bits of mantissa first, each value by up to 2^-9
+        bound = (K + 10) * 2 ** -23 * size + (2 ** -9 * size if kw else 0)
+        kernels.row_product(src, w, out[:, :N], **kw)
+        assert bool(((out[:, :N].double() - ref).abs() <= bound).all())
+        first = out[:, :N].clone()
+        kernels.row_product(src, w, out[:, :N], accumulate=True, **kw)
+        assert torch.equal(out[:, :N], first + first)
+        assert bool(torch.isnan(out[:, N:]).all())
+        if N % 32 == 0 and kernels.row_product_ok(rows, N // 2, K, True):
+            act = torch.empty(rows, N // 2, dtype=torch.bfloat16, device=DEV)
+            kernels.row_product(src, w, act, gated=True, **kw)
+            b = ref.view(rows, N // 32, 2, 16)
+            gate, up = b[:, :, 0].reshape(rows, -1), b[:, :, 1].reshape(rows, -1)
+            want = gate * torch.sigmoid(gate) * up
+            s = size.view(rows, N // 32, 2, 16).amax(2).reshape(rows, -1) if kw else 0
+            slack = 2 ** -9 * s * (2 + gate.abs() + up.abs()) if kw else 0
+            assert bool(((act.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-5 * (1 + want.abs()) + slack).all())
+    kernels.check_tc_status(torch.device(DEV))
