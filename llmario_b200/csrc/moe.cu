@@ -477,13 +477,14 @@ LLM_EXPORT int llm_moe_gather(const void* h, const int* pos, void* xp, int dtype
                               const int* ids, int E, const float* wts, float* row_scale,
                               cudaStream_t stream) {
   if (n_pairs <= 0) return 0;
+  // (it stands in front of the grouped product on CTA pairs: see launched_many_blocks)
   if ((wts != nullptr) != (row_scale != nullptr)) return LLM_ERR_ARGUMENT;
   if (dtype == LLM_F32)
-    return launch_pdl(moe_gather_kernel<float>, n_pairs, 128, 0, stream, (const float*)h, pos, (float*)xp, width, top,
-                      ids, E, wts, row_scale);
+    return launched_many_blocks(launch_pdl(moe_gather_kernel<float>, n_pairs, 128, 0, stream, (const float*)h, pos,
+                                           (float*)xp, width, top, ids, E, wts, row_scale), n_pairs);
   if (dtype == LLM_BF16)
-    return launch_pdl(moe_gather_kernel<bf16>, n_pairs, 128, 0, stream, (const bf16*)h, pos, (bf16*)xp, width, top,
-                      ids, E, wts, row_scale);
+    return launched_many_blocks(launch_pdl(moe_gather_kernel<bf16>, n_pairs, 128, 0, stream, (const bf16*)h, pos,
+                                           (bf16*)xp, width, top, ids, E, wts, row_scale), n_pairs);
   return LLM_ERR_UNSUPPORTED;
 }
 
