@@ -22,8 +22,8 @@
 // taken (N = bn, 2 bn, ... 256), so that only the padding of an expert's last bn rows is multiplied for
 // nothing.  1,501 tokens with two of eight experts of 6,144 x 4,096, lone CTAs with tiles of 128 rows ->
 // pairs: up with its squared rectifier 241 -> 163 us (one kernel instead of two), gated 183 -> 164, down
-// 165 -> 165 (3,072 tokens: 299 -> 288).  (Dealing the pieces by length, the longest first, took 199 us: a matrix's pieces then are
-// not neighbours in time and its rows come from memory twice.)
+// 165 -> 165 (3,072 tokens: 299 -> 288).  (Dealing the pieces by length, the longest first, took 199 us:
+// a matrix's pieces then are not neighbours in time and its rows come from memory twice.)
 //
 // Epilogues: store, residual add, squared rectifier, gated silu(g) * u with gate and up rows
 // interleaved in blocks of 16.  The output must be reachable by TMA.  Every wait is bounded: a CTA that gives up sets
