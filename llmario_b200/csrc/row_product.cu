@@ -1,4 +1,4 @@
-// Products of one or two rows with a small weight matrix (a step of few requests through a small
+// Products of one to four rows with a small weight matrix (a step of few requests through a small
 // model):  out[r][n] (=|+=) sum_k h[r][k] * W[n][k],  bfloat16 W, 32-bit sums, in which h is given in
 // bfloat16 or is the RMS norm of 32-bit rows (made here: no kernel of its own), and a gated form
 // silu(gate) * up with gate and up rows interleaved in blocks of 16.
@@ -14,12 +14,16 @@
 // (28 layers of Qwen3-0.6B sizes) 935 -> 698 us.  No atomics: an output is one warp's sum.
 // Limits: K 1,024 or 2,048, or 3,072 for one row, so that the rows fit a warp's registers beside a
 // second CTA, and slices of at most 100 KB, so that the slices of two kernels of the chain fit an SM
-// and the next one's copies overlap this one's work.
+// and the next one's copies overlap this one's work.  What has more values of h (up to four rows of
+// up to 4,096) keeps them in shared memory, a warp per row making them, behind one barrier: a step of
+// three or four requests (14 layers) 507 -> 478 us.  With room for eight rows the dot products took
+// longer than the chain saved (six or eight requests: 511 -> 631 us), so those stay on tcgen05.
 #include "common.cuh"
 
 namespace {
 constexpr int RP_WARPS = 8, RP_ROWS = 4;       // warps; weight rows a warp multiplies at a time
-constexpr int RP_SLICE = 100 * 1024;
+constexpr int RP_SLICE = 100 * 1024, RP_SHARED = 112 * 1024;
+constexpr int RP_MAX = 4;                      // rows
 enum RowMode : int { ROW_STORE = 0, ROW_ADD = 1, ROW_GATED = 2 };
 
 __device__ __forceinline__ void bulk_load(void* smem, const void* gmem, uint32_t bytes, uint64_t* bar) {
@@ -184,6 +188,147 @@ __global__ void __launch_bounds__(RP_WARPS * 32, 2)
   }
 }
 
+// The same for more values of h: the rows lie in shared memory, up to RP_MAX of them (those that are
+// not there are summed from whatever lies there and not written).
+template <int MODE, bool NORM>
+__global__ void __launch_bounds__(RP_WARPS * 32, 2)
+    row_product_shared_kernel(const void* __restrict__ x, int ldx, const float* __restrict__ norm_w, float eps,
+                              const bf16* __restrict__ W, void* __restrict__ out, int ldc, int rows, int N, int K, int per,
+                              int* __restrict__ status) {
+  constexpr int R = RP_MAX;
+  extern __shared__ __align__(128) uint8_t rp_raw[];
+  bf16* h_s = reinterpret_cast<bf16*>(rp_raw);            // [R][K]
+  bf16* w_s = h_s + (size_t)R * K;
+  __shared__ __align__(8) uint64_t full;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int n0 = blockIdx.x * per, cnt = min(per, N - n0), chunks = K >> 8;
+  if (tid == 0) {
+    mbar_init(&full, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  pdl_trigger();
+  if (tid == 0 && cnt > 0) {
+    mbar_expect_tx(&full, (uint32_t)cnt * (MODE == ROW_GATED ? 2 : 1) * K * 2);
+    if (MODE != ROW_GATED) {
+      bulk_load(w_s, W + (size_t)n0 * K, (uint32_t)cnt * K * 2, &full);
+    } else {
+      for (int f = 0; f < cnt;) {
+        const int at = n0 + f, run = min(16 - (at & 15), cnt - f);
+        const bf16* gate = W + (size_t)((at >> 4) * 32 + (at & 15)) * K;
+        bulk_load(w_s + (size_t)f * K, gate, (uint32_t)run * K * 2, &full);
+        bulk_load(w_s + (size_t)(cnt + f) * K, gate + (size_t)16 * K, (uint32_t)run * K * 2, &full);
+        f += run;
+      }
+    }
+  }
+  pdl_wait();
+  if (cnt <= 0) return;
+  // a warp makes a row
+  if (warp < rows) {
+    uint4* dst = reinterpret_cast<uint4*>(h_s + (size_t)warp * K) + lane;
+    if (NORM) {
+      const float* xr = (const float*)x + (size_t)warp * ldx + lane * 8;
+      float ss = 0.f;
+#pragma unroll 4
+      for (int c = 0; c < chunks; ++c) {
+        const float4 a = *reinterpret_cast<const float4*>(xr + c * 256);
+        const float4 b = *reinterpret_cast<const float4*>(xr + c * 256 + 4);
+        ss = fmaf(a.x, a.x, ss), ss = fmaf(a.y, a.y, ss), ss = fmaf(a.z, a.z, ss), ss = fmaf(a.w, a.w, ss);
+        ss = fmaf(b.x, b.x, ss), ss = fmaf(b.y, b.y, ss), ss = fmaf(b.z, b.z, ss), ss = fmaf(b.w, b.w, ss);
+      }
+      const float scale = 1.0f / sqrtf(warp_sum(ss) / (float)K + eps);
+#pragma unroll 4
+      for (int c = 0; c < chunks; ++c) {
+        float v[8], w[8];
+        *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(xr + c * 256);
+        *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(xr + c * 256 + 4);
+        *reinterpret_cast<float4*>(w) = *reinterpret_cast<const float4*>(norm_w + c * 256 + lane * 8);
+        *reinterpret_cast<float4*>(w + 4) = *reinterpret_cast<const float4*>(norm_w + c * 256 + lane * 8 + 4);
+        uint32_t two[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const __nv_bfloat162 t = __floats2bfloat162_rn(v[2 * e] * scale * w[2 * e], v[2 * e + 1] * scale * w[2 * e + 1]);
+          two[e] = *reinterpret_cast<const uint32_t*>(&t);
+        }
+        dst[c * 32] = make_uint4(two[0], two[1], two[2], two[3]);
+      }
+    } else {
+      const uint4* src = reinterpret_cast<const uint4*>((const bf16*)x + (size_t)warp * ldx) + lane;
+#pragma unroll 4
+      for (int c = 0; c < chunks; ++c) dst[c * 32] = src[c * 32];
+    }
+  }
+  __syncthreads();
+  if (!mbar_wait(&full, 0)) {
+    if (lane == 0) atomicExch(status, 7);
+    return;
+  }
+  constexpr int OUTS = MODE == ROW_GATED ? RP_ROWS / 2 : RP_ROWS, VALUES = RP_ROWS * R;
+  const uint4* hr = reinterpret_cast<const uint4*>(h_s) + lane;
+  for (int i0 = warp * OUTS; i0 < cnt; i0 += RP_WARPS * OUTS) {
+    // value j * R + r, weight row j with row r, ends up in the lane of that number
+    const int my_v = lane & (VALUES - 1), my_j = my_v / R, my_r = my_v % R, my_o = i0 + my_j;
+    const bool mine = lane < OUTS * R && my_o < cnt && my_r < rows;
+    float old = 0.f;
+    if (MODE == ROW_ADD && mine) old = ((const float*)out)[(size_t)my_r * ldc + n0 + my_o];
+    const uint4* wr[RP_ROWS];
+#pragma unroll
+    for (int j = 0; j < RP_ROWS; ++j) {
+      const int o = min(i0 + (j % OUTS), cnt - 1) + (j / OUTS) * cnt;
+      wr[j] = reinterpret_cast<const uint4*>(w_s + (size_t)o * K) + lane;
+    }
+    float acc[VALUES];
+#pragma unroll
+    for (int i = 0; i < VALUES; ++i) acc[i] = 0.f;
+    for (int c = 0; c < chunks; ++c) {
+      float w[RP_ROWS][8];
+#pragma unroll
+      for (int j = 0; j < RP_ROWS; ++j) {
+        const uint4 v = wr[j][c * 32];
+        const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) w[j][2 * e] = __uint_as_float(u[e] << 16), w[j][2 * e + 1] = __uint_as_float(u[e] & 0xffff0000u);
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const uint4 v = hr[(size_t)r * (K / 8) + c * 32];
+        const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float lo = __uint_as_float(u[e] << 16), hi = __uint_as_float(u[e] & 0xffff0000u);
+#pragma unroll
+          for (int j = 0; j < RP_ROWS; ++j) {
+            acc[j * R + r] = fmaf(lo, w[j][2 * e], acc[j * R + r]);
+            acc[j * R + r] = fmaf(hi, w[j][2 * e + 1], acc[j * R + r]);
+          }
+        }
+      }
+    }
+    static_assert(VALUES == 16, "the two halves of a warp are summed first");
+#pragma unroll
+    for (int i = 0; i < VALUES; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 16);
+#pragma unroll
+    for (int half = VALUES / 2; half > 0; half >>= 1) {
+      const bool hi = (lane & half) != 0;
+#pragma unroll
+      for (int i = 0; i < half; ++i) {
+        const float send = hi ? acc[i] : acc[i + half], keep = hi ? acc[i + half] : acc[i];
+        acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+      }
+    }
+    float val = acc[0];
+    if (MODE == ROW_GATED) {
+      const float up = __shfl_down_sync(0xffffffffu, val, OUTS * R);
+      val = __fdividef(val, 1.0f + __expf(-val)) * up;
+    }
+    if (mine) {
+      if (MODE == ROW_GATED) ((bf16*)out)[(size_t)my_r * ldc + n0 + my_o] = from_f32<bf16>(val);
+      else ((float*)out)[(size_t)my_r * ldc + n0 + my_o] = MODE == ROW_ADD ? old + val : val;
+    }
+  }
+}
+
 int rp_sm_count() {
   static int n = 0;
   if (!n) {
@@ -217,15 +362,32 @@ int rp_mode(const void* x, int ldx, const float* norm_w, float eps, const void* 
   RP(ROW_GATED);
 #undef RP
 }
+int rp_shared(const void* x, int ldx, const float* norm_w, float eps, const void* W, void* out, int ldc, int rows, int N,
+              int K, int per, int mode, int* status, cudaStream_t stream) {
+  const int smem = (RP_MAX * K + per * (mode == ROW_GATED ? 2 : 1) * K) * 2;
+  auto go = [&](auto kernel) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RP_SHARED);
+    if (e != cudaSuccess) return (int)e;
+    return launch_pdl(kernel, (N + per - 1) / per, RP_WARPS * 32, smem, stream, x, ldx, norm_w, eps, (const bf16*)W, out,
+                      ldc, rows, N, K, per, status);
+  };
+  if (mode == ROW_STORE) return norm_w ? go(row_product_shared_kernel<ROW_STORE, true>) : go(row_product_shared_kernel<ROW_STORE, false>);
+  if (mode == ROW_ADD) return norm_w ? go(row_product_shared_kernel<ROW_ADD, true>) : go(row_product_shared_kernel<ROW_ADD, false>);
+  return norm_w ? go(row_product_shared_kernel<ROW_GATED, true>) : go(row_product_shared_kernel<ROW_GATED, false>);
+}
+
+// whether the rows fit a warp's registers
+bool rp_in_registers(int rows, int K) { return rows <= 2 && (K == 1024 || K == 2048 || (K == 3072 && rows == 1)); }
 }  // namespace
 
 // Whether llm_row_product takes these sizes: rows x K values of h in registers, N (gated: features)
 // outputs whose weights fit the SMs' slices.
 LLM_EXPORT int llm_row_product_ok(int rows, int N, int K, int gated) {
-  if (rows < 1 || rows > 2 || N < 1) return 0;
-  if (K != 1024 && K != 2048 && !(K == 3072 && rows == 1)) return 0;
+  if (rows < 1 || rows > RP_MAX || N < 1 || K < 256 || K > 4096 || K % 256) return 0;
   const int per = (N + rp_sm_count() - 1) / rp_sm_count();
-  return (long long)per * (gated ? 2 : 1) * K * 2 <= RP_SLICE;
+  const long long slice = (long long)per * (gated ? 2 : 1) * K * 2;
+  if (rp_in_registers(rows, K)) return slice <= RP_SLICE;
+  return slice <= RP_SLICE && slice + RP_MAX * K * 2 <= RP_SHARED;
 }
 
 // mode 0: out f32 = h W^T; 1: out f32 += h W^T; 2: out bf16 = silu(gate) * up, W interleaved, N features
@@ -238,6 +400,8 @@ LLM_EXPORT int llm_row_product(const void* x, int ldx, const float* norm_w, floa
   if (!llm_row_product_ok(rows, N, K, mode == ROW_GATED) || (mode == ROW_GATED && N % 16)) return LLM_ERR_UNSUPPORTED;
   if ((((uintptr_t)x | (uintptr_t)W | (uintptr_t)norm_w) & 15) || ldx % (norm_w ? 4 : 8)) return LLM_ERR_UNSUPPORTED;
   const int per = (N + rp_sm_count() - 1) / rp_sm_count();
+  if (!rp_in_registers(rows, K))
+    return rp_shared(x, ldx, norm_w, eps, W, out, ldc, rows, N, K, per, mode, status, stream);
 #define RP_GO(KC, R) return rp_mode<KC, R>(x, ldx, norm_w, eps, W, out, ldc, N, per, mode, status, stream)
   switch (K / 256 * 8 + rows) {
     case 4 * 8 + 1: RP_GO(4, 1);

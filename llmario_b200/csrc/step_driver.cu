@@ -184,7 +184,7 @@ enum Kind : int {
   K_EXTRAS, K_LATENT, K_ROW_PRODUCT, N_KINDS
 };
 long long g_counts[N_KINDS] = {};
-int g_row_product = 1;      // 0: every product by the kernels for more rows (for comparisons)
+int g_row_product = 4;      // steps of up to so many rows; 0: every product by the kernels for more (for comparisons)
 
 int sm_count() {
   static int n = 0;
@@ -375,10 +375,10 @@ struct Run {
 
   int buffer(long long key, size_t bytes, void** out, bool zero = false) { return ar.get(key, bytes, zero, out); }
 
-  // whether a product of this step's rows with w goes to the kernel for one or two rows and small
+  // whether a product of this step's rows with w goes to the kernel for few rows and small
   // matrices (row_product.cu), which can make the norm of 32-bit rows itself
   bool row_product_ok(const void* x, int ldx, const void* w, int w_dt, int ldw, int n, int k, bool gated) const {
-    return g_row_product && st.dtype == LLM_BF16 && w_dt == LLM_BF16 && ldw == k && ldx % 8 == 0 && aligned16(x) &&
+    return st.rows <= g_row_product && st.dtype == LLM_BF16 && w_dt == LLM_BF16 && ldw == k && ldx % 8 == 0 && aligned16(x) &&
            aligned16(w) && llm_row_product_ok(st.rows, n, k, gated ? 1 : 0);
   }
 
@@ -882,7 +882,7 @@ struct Run {
 
 }  // namespace
 
-LLM_EXPORT void llm_set_row_product(int on) { g_row_product = on ? 1 : 0; }
+LLM_EXPORT void llm_set_row_product(int rows) { g_row_product = rows; }
 
 // ---- policies, exported so that the Python statement of the same rules can be held to them
 LLM_EXPORT int llm_token_tile(int rows) {

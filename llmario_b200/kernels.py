@@ -1012,14 +1012,14 @@ def k_splits(rows: int, out_features: int, in_features: int) -> int:
 
 
 def row_product_ok(rows: int, out_features: int, in_features: int, gated: bool = False) -> bool:
-    """Whether :func:`row_product` takes these sizes: one or two rows, a matrix of a few MB."""
-    return rows <= 2 and bool(lib().llm_row_product_ok(rows, out_features, in_features, int(gated)))
+    """Whether :func:`row_product` takes these sizes: one to four rows, a matrix of a few MB."""
+    return rows <= 4 and bool(lib().llm_row_product_ok(rows, out_features, in_features, int(gated)))
 
 
 def row_product(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool = False,
                 gated: bool = False, norm_weight: Optional[torch.Tensor] = None,
                 eps: float = 0.0) -> None:
-    """out (=|+=) h @ w.T for one or two rows, ``out`` float32; with ``gated`` (``w`` as blocks of 16
+    """out (=|+=) h @ w.T for one to four rows, ``out`` float32; with ``gated`` (``w`` as blocks of 16
     gate rows and 16 up rows) ``out = silu(gate) * up`` in bfloat16.  ``x`` is h in bfloat16 or, with
     ``norm_weight``, float32 rows whose RMS norm, rounded to bfloat16, is h."""
     _cuda(x, w, out, norm_weight)
@@ -1042,7 +1042,7 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool
     CUDA-core kernels for everything else (32-bit operands, unaligned sizes).
     ``out_is_zero``: the caller guarantees that ``out`` holds zeros, so a split-K product need
     not clear it first."""
-    if (a.shape[0] <= 2 and out.dtype == torch.float32 and _tc_ok(a, w) and w.is_contiguous()
+    if (a.shape[0] <= 4 and out.dtype == torch.float32 and _tc_ok(a, w) and w.is_contiguous()
             and out.stride(1) == 1 and row_product_ok(a.shape[0], w.shape[0], a.shape[1])):
         row_product(a, w, out, accumulate)
     elif _tc_ok(a, w, out):

@@ -264,15 +264,15 @@ def test_grouped_products_on_cta_pairs(counts, N, K, bn):
 
 
 @gpu
-@pytest.mark.parametrize("rows", (1, 2))
-@pytest.mark.parametrize("N,K", [(1024, 2048), (4096, 1024), (1024, 3072), (148, 1024), (7, 2048), (3056, 1024)])
+@pytest.mark.parametrize("rows", (1, 2, 3, 4))
+@pytest.mark.parametrize("N,K", [(1024, 2048), (4096, 1024), (1024, 3072), (148, 1024), (7, 2048), (3056, 1024), (640, 256),
+                                 (96, 4096)])
 def test_row_product(rows, N, K):
-    """One or two rows through a small matrix: stored, added, gated, of 16-bit rows and of the norm of
-    32-bit rows; fewer outputs than SMs, slices that do not come out even, strided rows."""
+    """One to four rows through a small matrix (held in registers or in shared memory): stored, added,
+    gated, of 16-bit rows and of the norm of 32-bit rows; fewer outputs than SMs, slices that do not
+    come out even, strided rows."""
     from llmario_b200 import kernels
-    if not kernels.row_product_ok(rows, N, K):
-        assert K == 3072 and rows == 2
-        return
+    assert kernels.row_product_ok(rows, N, K)
     x = rnd(rows, K + 8, seed=1)[:, :K]
     h = rnd(rows, K + 8, dtype=torch.bfloat16, seed=2)[:, :K]
     g = 1 + 0.1 * rnd(K, seed=3)
