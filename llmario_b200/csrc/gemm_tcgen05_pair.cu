@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
     works = m_tiles * n_tiles;
   }
   // the tile and the range of K of a work item: items of whole tiles before those of the last tokens
-  const int n_whole = GROUPED ? 0 : m_tiles * (T / BN);
+  const int n_whole = GROUPED ? 0 : FORM == WHOLE_TILES ? m_tiles * n_tiles : m_tiles * (T / BN);
   auto item = [&](int work, int& tile, int& ks) {
     if (GROUPED) {
       tile = work, ks = 0;
@@ -419,9 +419,13 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
 // tiles than pairs some never work.  A work item costs its 64-wide blocks of K plus about six
 // blocks' worth of start and epilogue (fitted to measured times of seven shapes); K is cut into
 // the number of ranges, each of at least eight blocks, for which the rounds cost least.
-// The last tokens of a T that is not a multiple of 256 make shorter items, dealt last.
+// The last tokens of a T that is not a multiple of 256 make shorter items, dealt last, where they are
+// at most half a tile: with more of them the padding saved is less than what the variant with a width
+// read at run time loses.
+bool short_tail(int T) { return T % BN != 0 && T % BN <= BN / 2; }
 double rounds_cost(int m_tiles, int T, int nkb, int pairs, int s) {
-  const int whole = m_tiles * (T / BN) * s, rest = T % BN ? m_tiles * s : 0;
+  const bool tail = short_tail(T);
+  const int whole = m_tiles * (tail ? T / BN : (T + BN - 1) / BN) * s, rest = tail ? m_tiles * s : 0;
   const int first = (whole + pairs - 1) / pairs, all = (whole + rest + pairs - 1) / pairs;
   return first * ((double)nkb / s + 6.0) + (all - first) * ((double)nkb / s * (0.25 + 0.75 * (T % BN) / BN) + 5.0);
 }
@@ -497,7 +501,7 @@ int launch_form(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap&
 template <int STAGES, int EPI, typename TC>
 int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mxs, const CUtensorMap& mc, int T, int N,
            int K, int half, int sm_count, int* status, cudaStream_t stream, float act_limit = 0.f) {
-  if (T % BN)
+  if (short_tail(T))
     return launch_form<STAGES, EPI, TC, LAST_TOKENS>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream, act_limit);
   return launch_form<STAGES, EPI, TC, WHOLE_TILES>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream, act_limit);
 }
