@@ -135,6 +135,7 @@ struct Grouping {
   const int* tile_group;
   int bn, n_small, group_rows;
   const float* row_scale;
+  int in_order;      // LAST_TOKENS: a matrix tile's last tokens follow its whole tiles (see launch)
 };
 
 // What a tile holds: 256 tokens always; 256 or, at the end of T, fewer; or the grouped form's pieces.
@@ -217,6 +218,11 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
       tile = work, ks = 0;
     } else if (FORM == WHOLE_TILES) {
       tile = work % n_whole, ks = work / n_whole;
+    } else if (grouping.in_order) {
+      // (dealt one place further in every round, so that the short items do not all meet the same pairs)
+      const int all = m_tiles * n_tiles, round = work / n_pairs, base = round * n_pairs;
+      const int at = base + (work - base + round) % min(n_pairs, works - base);
+      ks = at / all, tile = at % all;
     } else if (work < n_whole * ksplits) {
       tile = work % n_whole, ks = work / n_whole;
     } else {
@@ -237,7 +243,10 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
       // an MMA as wide as they are (in steps of 32)
       const int whole = T / BN;
       w0 = 0;
-      if (tile < n_whole) m = tile / whole, t0 = (tile % whole) * BN, n = BN;
+      if (grouping.in_order) {
+        m = tile / n_tiles, t0 = (tile % n_tiles) * BN;
+        n = T - t0 >= BN ? BN : (T - t0 + 31) & ~31;
+      } else if (tile < n_whole) m = tile / whole, t0 = (tile % whole) * BN, n = BN;
       else m = tile - n_whole, t0 = whole * BN, n = (T - t0 + 31) & ~31;
     }
   };
@@ -419,10 +428,12 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
 // tiles than pairs some never work.  A work item costs its 64-wide blocks of K plus about six
 // blocks' worth of start and epilogue (fitted to measured times of seven shapes); K is cut into
 // the number of ranges, each of at least eight blocks, for which the rounds cost least.
-// The last tokens of a T that is not a multiple of 256 make shorter items, dealt last, where they are
-// at most half a tile: with more of them the padding saved is less than what the variant with a width
-// read at run time loses.
-bool short_tail(int T) { return T % BN != 0 && T % BN <= BN / 2; }
+// The last tokens of a T that is not a multiple of 256 make shorter items where they are at most half a
+// tile and there are fewer than four whole ones: beyond that the padding saved is less than what the
+// variant with a width read at run time loses.  Four layers of Qwen3-8B widths, padded -> narrow, 520 /
+// 600 / 800 tokens: 1,231 / 1,252 / 1,625 -> 1,183 / 1,187 / 1,543 us; 1,100 / 2,100: 1,849 / 3,022 -> 1,858 /
+// 3,044; 1,500 / 3,000 (220 and 184 left over): 2,161 / 4,133 -> 2,230 / 4,238.
+bool short_tail(int T) { return T < 4 * BN && T % BN != 0 && T % BN <= BN / 2; }
 double rounds_cost(int m_tiles, int T, int nkb, int pairs, int s) {
   const bool tail = short_tail(T);
   const int whole = m_tiles * (tail ? T / BN : (T + BN - 1) / BN) * s, rest = tail ? m_tiles * s : 0;
@@ -501,8 +512,14 @@ int launch_form(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap&
 template <int STAGES, int EPI, typename TC>
 int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mxs, const CUtensorMap& mc, int T, int N,
            int K, int half, int sm_count, int* status, cudaStream_t stream, float act_limit = 0.f) {
-  if (short_tail(T))
-    return launch_form<STAGES, EPI, TC, LAST_TOKENS>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream, act_limit);
+  if (short_tail(T)) {
+    // Dealt last, the short items even out the pairs, but they meet every weight a second time: fine
+    // while the weights stay in the L2 (some 48 MB), else they follow their tiles (600 tokens 1,199 ->
+    // 1,187 us, 1,100 tokens 1,869 -> 1,858).
+    Grouping g = Grouping();
+    g.in_order = (long long)N * K * 2 > 48LL << 20;
+    return launch_form<STAGES, EPI, TC, LAST_TOKENS>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream, act_limit, g);
+  }
   return launch_form<STAGES, EPI, TC, WHOLE_TILES>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream, act_limit);
 }
 }  // namespace

@@ -128,7 +128,7 @@ def test_recurrence_in_runs(kind, H, G, K, V, lengths):
 
 @gpu
 @pytest.mark.parametrize("T,N,K", [(777, 4096, 1024), (1024, 520, 72), (543, 6144, 200), (2048, 1024, 3072),
-                                   (513, 264, 512), (1500, 136, 4096), (600, 4096, 2056), (2049, 520, 1024)])
+                                   (513, 264, 512), (586, 8200, 3080), (1500, 136, 4096), (600, 4096, 2056), (2049, 520, 1024)])
 def test_linear_many_rows_few_tiles(T, N, K):
     """Products with fewer tiles than CTAs, stored whole or added in ranges of K."""
     from llmario_b200 import kernels
