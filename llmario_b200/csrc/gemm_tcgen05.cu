@@ -32,7 +32,7 @@
 int llm_zero_f32(float* p, int rows, int cols, int ld, cudaStream_t stream);   // elementwise.cu
 int llm_pair_store_way(int T, int N, int K, int splits);                       // gemm_tcgen05_pair.cu
 int llm_gemm_tcgen05_pair(const void* X, const void* W, void* C, int c_dtype, int T, int N, int K, int lda,
-                          int ldw, int ldc, int mode, int half, float limit, int* status, cudaStream_t stream);
+                          int ldw, int ldc, int mode, int half, float limit, int ranges, int* status, cudaStream_t stream);
 int llm_gemm_tcgen05_persistent(const void* X, const void* W, void* C, int c_dtype, int T, int N, int K,
                                 int lda, int ldw, int ldc, int mode, int half, int* status,
                                 cudaStream_t stream);                        // gemm_tcgen05_persistent.cu
@@ -460,25 +460,30 @@ static int gemm_any(const void* X, const void* W, void* C, int c_dtype, int T, i
   if (K <= 0 || K % 8 || lda % 8 || ldw % 8) return LLM_ERR_UNSUPPORTED;
   if (((uintptr_t)X | (uintptr_t)W) & 15) return LLM_ERR_UNSUPPORTED;
   if (splits < 1) return LLM_ERR_ARGUMENT;
+  const int kblocks = (K + TILE_K - 1) / TILE_K;
+  int lone_splits = min(splits, kblocks);
+  // no split may be empty
+  while (lone_splits > 1 && (lone_splits - 1) * ((kblocks + lone_splits - 1) / lone_splits) >= kblocks) --lone_splits;
   if (bn == 256) {
     // many rows: the persistent kernels (tiles of 256 tokens, epilogue overlapped with the next
     // tile), on CTA pairs where that form exists; if the output cannot be written by TMA, the
     // one-tile kernel with 128 tokens
     // (the pair kernel cuts K itself where its adding epilogue allows, so it also takes the
     // products for which the caller asked for a split)
-    const int way = mode == 0 && splits > 1 && c_dtype == LLM_F32 ? llm_pair_store_way(T, N, K, splits) : 2;
+    const int way = mode == 0 && lone_splits > 1 && c_dtype == LLM_F32 ? llm_pair_store_way(T, N, K, lone_splits) : 2;
     if (way < 2) {
       if (way == 1 && !out_is_zero) {
         const int z = llm_zero_f32((float*)C, T, N, ldc, stream);
         if (z != 0) return z;
         g_llm_after_rotation = 1;      // (a kernel of many blocks: see launched_many_blocks)
       }
-      int r = llm_gemm_tcgen05_pair(X, W, C, c_dtype, T, N, K, lda, ldw, ldc, way, half, limit, status, stream);
+      int r = llm_gemm_tcgen05_pair(X, W, C, c_dtype, T, N, K, lda, ldw, ldc, way, half, limit, lone_splits == 2 ? 2 : 0, status,
+                                    stream);
       if (r != LLM_ERR_UNSUPPORTED) return r;
       if (way == 1) out_is_zero = 1;
     }
     if (splits == 1 || mode == 1) {
-      int r = llm_gemm_tcgen05_pair(X, W, C, c_dtype, T, N, K, lda, ldw, ldc, mode, half, limit, status, stream);
+      int r = llm_gemm_tcgen05_pair(X, W, C, c_dtype, T, N, K, lda, ldw, ldc, mode, half, limit, 0, status, stream);
       if (r != LLM_ERR_UNSUPPORTED) return r;
     }
     if (splits == 1 && mode != 4) {
@@ -487,10 +492,7 @@ static int gemm_any(const void* X, const void* W, void* C, int c_dtype, int T, i
     }
     bn = 128;
   }
-  const int kblocks = (K + TILE_K - 1) / TILE_K;
-  if (splits > kblocks) splits = kblocks;
-  // no split may be empty
-  while (splits > 1 && (splits - 1) * ((kblocks + splits - 1) / splits) >= kblocks) --splits;
+  splits = lone_splits;
   CUtensorMap mw, mx;
   if (!llm_tensor_map(W, N, K, ldw, mode == 2 ? 16 : TILE_M, TILE_K, 0, &mw)) return LLM_ERR_UNSUPPORTED;
   if (!llm_tensor_map(X, T, K, lda, bn, TILE_K, 0, &mx)) return LLM_ERR_UNSUPPORTED;

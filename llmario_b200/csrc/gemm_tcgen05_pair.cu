@@ -136,6 +136,7 @@ struct Grouping {
   int bn, n_small, group_rows;
   const float* row_scale;
   int in_order;      // LAST_TOKENS: a matrix tile's last tokens follow its whole tiles (see launch)
+  int k_up;          // the ranges of K: range ks begins at its share of the blocks of K, rounded down (0) or up (1)
 };
 
 // What a tile holds: 256 tokens always; 256 or, at the end of T, fewer; or the grouped form's pieces.
@@ -151,6 +152,10 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
     int m_tiles, int n_tiles, int ksplits, float act_limit, int* __restrict__ status, const Grouping grouping) {
   constexpr bool GATED = gated_epilogue(EPI), GROUPED = FORM == GROUPED_TILES;
   constexpr int FEAT = GATED ? 64 : TILE_M;     // output features of this CTA per tile
+  // EPI_TWO_SUMS: the accumulators hold the sums over the first and the second half of K of one tile,
+  // which are added where they are read: the bits of a product whose halves were added in memory,
+  // without the additions (a tile's epilogue then has no next tile beside it)
+  constexpr int SUMS = EPI == EPI_TWO_SUMS ? 2 : 1;
   extern __shared__ uint8_t raw[];
   auto& sm = *reinterpret_cast<PairStorage<STAGES, FEAT, TC, GROUPED>*>(
       (reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
@@ -230,6 +235,9 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
       tile = n_whole + rest % m_tiles, ks = rest / m_tiles;
     }
   };
+  auto range_start = [&](int ks) {
+    return (int)(((long long)ks * nkb + (grouping.k_up ? ksplits - 1 : 0)) / ksplits);
+  };
   // a tile's place among the tiles of weight rows, its first row of X, its rows, and the row of W
   // where its matrix starts
   auto place = [&](int tile, int& m, int& t0, int& n, int& w0) {
@@ -276,7 +284,7 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
       int tile, ks, m, t0, n, w0;
       item(work, tile, ks);
       place(tile, m, t0, n, w0);
-      const int kb0 = (int)((long long)ks * nkb / ksplits), kb1 = (int)((long long)(ks + 1) * nkb / ksplits);
+      const int kb0 = range_start(ks), kb1 = range_start(ks + 1);
       const int f0 = m * (2 * FEAT) + (int)rank * FEAT;          // first output feature
       const int row0 = w0 + (GATED ? 2 * f0 : f0);               // first weight row
       t0 += (int)rank * (n >> 1);                                // (this CTA's half of the tokens)
@@ -311,26 +319,30 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
       item(work, tile, ks);
       place(tile, m, t0, n, w0);
       const uint32_t idesc = idesc_0 | ((uint32_t)(n >> 3) << 17);
-      const int kb0 = (int)((long long)ks * nkb / ksplits), kb1 = (int)((long long)(ks + 1) * nkb / ksplits);
-      const int buf = local & 1;
-      ok = mbar_wait_pair(&sm.acc_empty[buf], (uint32_t)((local >> 1) & 1) ^ 1);
-      if (!ok) { atomicExch(status, 2); sm.dead = 1; break; }
-      tc_fence_after();
-      const uint32_t acc = tmem + (uint32_t)buf * BN;
-      for (int kb = kb0; kb < kb1; ++kb, ++it) {
-        const int s = (int)(it % STAGES);
-        ok = mbar_wait_pair(&sm.full[s], (uint32_t)((it / STAGES) & 1));
+#pragma unroll 1
+      for (int sum = 0; sum < SUMS && ok; ++sum) {
+        const int kb0 = SUMS == 2 ? sum * ((nkb + 1) / 2) : range_start(ks);
+        const int kb1 = SUMS == 2 ? (sum ? nkb : (nkb + 1) / 2) : range_start(ks + 1);
+        const int buf = SUMS == 2 ? sum : local & 1, use = SUMS == 2 ? local : local >> 1;
+        ok = mbar_wait_pair(&sm.acc_empty[buf], (uint32_t)(use & 1) ^ 1);
         if (!ok) { atomicExch(status, 2); sm.dead = 1; break; }
         tc_fence_after();
-        const uint64_t da = smem_desc(smem_u32(sm.a[s]));
-        const uint64_t db = smem_desc(smem_u32(sm.b[s]));
+        const uint32_t acc = tmem + (uint32_t)buf * BN;
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+          const int s = (int)(it % STAGES);
+          ok = mbar_wait_pair(&sm.full[s], (uint32_t)((it / STAGES) & 1));
+          if (!ok) { atomicExch(status, 2); sm.dead = 1; break; }
+          tc_fence_after();
+          const uint64_t da = smem_desc(smem_u32(sm.a[s]));
+          const uint64_t db = smem_desc(smem_u32(sm.b[s]));
 #pragma unroll
-        for (int k = 0; k < TILE_K / UMMA_K; ++k)
-          pair_mma(acc, da + (uint64_t)(k * UMMA_K * 2 >> 4), db + (uint64_t)(k * UMMA_K * 2 >> 4), idesc,
-                   (kb > kb0 || k > 0) ? 1u : 0u);
-        pair_commit(&sm.empty[s]);
+          for (int k = 0; k < TILE_K / UMMA_K; ++k)
+            pair_mma(acc, da + (uint64_t)(k * UMMA_K * 2 >> 4), db + (uint64_t)(k * UMMA_K * 2 >> 4), idesc,
+                     (kb > kb0 || k > 0) ? 1u : 0u);
+          pair_commit(&sm.empty[s]);
+        }
+        if (ok) pair_commit(&sm.acc_full[buf]);
       }
-      if (ok) pair_commit(&sm.acc_full[buf]);
     }
   } else if (warp >= 2) {
     // ------------------------------------------------------------------ epilogue (both CTAs)
@@ -345,8 +357,9 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
       item(work, tile, ks);
       place(tile, m, t0, n_cols, w0);
       const int n0 = m * (2 * FEAT) + (int)rank * FEAT;
-      const int buf = local & 1;
-      bool ok = mbar_wait_pair(&sm.acc_full[buf], (uint32_t)((local >> 1) & 1));
+      const int buf = SUMS == 2 ? 0 : local & 1, use = SUMS == 2 ? local : local >> 1;
+      bool ok = mbar_wait_pair(&sm.acc_full[buf], (uint32_t)(use & 1));
+      if (SUMS == 2 && ok) ok = mbar_wait_pair(&sm.acc_full[1], (uint32_t)(use & 1));
       if (!ok) { if (lane == 0) atomicExch(status, 3); sm.dead = 1; }
       // the four warps decide together whether to go on
       asm volatile("bar.sync 1, 128;" ::: "memory");
@@ -363,7 +376,15 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
         for (int h = 0; h < CH / 16; ++h) {
           uint32_t v[16];
           tmem_ld16(acc + (uint32_t)(c + h * 16), v);
-          tmem_ld_wait();
+          if (SUMS == 2) {
+            uint32_t second[16];
+            tmem_ld16(acc + (uint32_t)(BN + c + h * 16), second);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(second[j]));
+          } else {
+            tmem_ld_wait();
+          }
           if (GATED) {
             const int f = q * 16 + (lane & 15);
             const int col0 = h * 16 + (lane < 16 ? 0 : 8);
@@ -392,8 +413,10 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
           tc_fence_before();
           __syncwarp();
           if (lane == 0) {
-            if (leader) mbar_arrive_local(&sm.acc_empty[buf]);
-            else mbar_arrive_in(&sm.acc_empty[buf], 0);
+            for (int b = buf; b < buf + SUMS; ++b) {
+              if (leader) mbar_arrive_local(&sm.acc_empty[b]);
+              else mbar_arrive_in(&sm.acc_empty[b], 0);
+            }
           }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -423,38 +446,49 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
   }
 }
 
-// The adding epilogue lets K be cut.  With few tiles to a pair the last round of tiles leaves
-// most pairs idle (160 tiles on 74 pairs: three rounds for the work of 2.2), and with fewer
-// tiles than pairs some never work.  A work item costs its 64-wide blocks of K plus about six
-// blocks' worth of start and epilogue (fitted to measured times of seven shapes); K is cut into
-// the number of ranges, each of at least eight blocks, for which the rounds cost least.
 // The last tokens of a T that is not a multiple of 256 make shorter items where they are at most half a
 // tile and there are fewer than four whole ones: beyond that the padding saved is less than what the
 // variant with a width read at run time loses.  Four layers of Qwen3-8B widths, padded -> narrow, 520 /
 // 600 / 800 tokens: 1,231 / 1,252 / 1,625 -> 1,183 / 1,187 / 1,543 us; 1,100 / 2,100: 1,849 / 3,022 -> 1,858 /
 // 3,044; 1,500 / 3,000 (220 and 184 left over): 2,161 / 4,133 -> 2,230 / 4,238.
 bool short_tail(int T) { return T < 4 * BN && T % BN != 0 && T % BN <= BN / 2; }
-double rounds_cost(int m_tiles, int T, int nkb, int pairs, int s) {
-  const bool tail = short_tail(T);
+// Dealt last, the short items even out the pairs, but they meet every weight a second time: fine
+// while the weights stay in the L2 (some 48 MB), else they follow their tiles (600 tokens 1,199 ->
+// 1,187 us, 1,100 tokens 1,869 -> 1,858).
+bool tail_in_order(int N, int K) { return (long long)N * K * 2 > 48LL << 20; }
+
+// What a product in s ranges of K takes, in blocks of K of a whole tile: a work item costs its 64-wide
+// blocks of K plus about six blocks' worth of start and epilogue (fitted to measured times of seven
+// shapes), an item of last tokens less where they are dealt last.
+double rounds_cost(int N, int K, int T, int pairs, int s) {
+  const bool tail = short_tail(T) && !tail_in_order(N, K);
+  const int m_tiles = (N + 2 * TILE_M - 1) / (2 * TILE_M), nkb = (K + TILE_K - 1) / TILE_K;
   const int whole = m_tiles * (tail ? T / BN : (T + BN - 1) / BN) * s, rest = tail ? m_tiles * s : 0;
   const int first = (whole + pairs - 1) / pairs, all = (whole + rest + pairs - 1) / pairs;
   return first * ((double)nkb / s + 6.0) + (all - first) * ((double)nkb / s * (0.25 + 0.75 * (T % BN) / BN) + 5.0);
 }
-int cheapest_cut(int m_tiles, int T, int nkb, int pairs, double* cost_of_it) {
+
+// The adding epilogue lets K be cut.  With few tiles to a pair the last round of tiles leaves
+// most pairs idle (160 tiles on 74 pairs: three rounds for the work of 2.2), and with fewer
+// tiles than pairs some never work.  K is cut into the number of ranges, each of at least eight
+// blocks, for which the rounds of whole tiles cost least.  (Narrow last tiles do not enter: how often a
+// sum is cut decides its rounding, and one range alone gives the same bits every time.)
+int cheapest_cut(int m_tiles, int T, int nkb, int pairs) {
+  const int tiles = m_tiles * ((T + BN - 1) / BN);
   int ksplits = 1;
   double best = 0;
-  for (int s = 1; s <= 8 && (s == 1 || nkb / s >= 8); ++s) {
-    const double cost = rounds_cost(m_tiles, T, nkb, pairs, s);
+  for (int s = 1; s <= 8 && nkb / s >= 8; ++s) {
+    const int rounds = (tiles * s + pairs - 1) / pairs;
+    const double cost = rounds * ((double)nkb / s + 6.0);
     if (s == 1 || cost < best * 0.99) best = cost, ksplits = s;
   }
-  *cost_of_it = best;
   return ksplits;
 }
 
 template <int STAGES, int EPI, typename TC, int FORM>
 int launch_form(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mxs, const CUtensorMap& mc, int T, int N,
            int K, int half, int sm_count, int* status, cudaStream_t stream, float act_limit = 0.f,
-           const Grouping& grouping = Grouping()) {
+           const Grouping& grouping = Grouping(), int ranges = 0) {
   constexpr bool GATED = gated_epilogue(EPI), GROUPED = FORM == GROUPED_TILES;
   constexpr int FEAT = GATED ? 64 : TILE_M;
   auto kernel = gemm_pair_kernel<STAGES, EPI, TC, FORM>;
@@ -495,8 +529,7 @@ int launch_form(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap&
   int ksplits = 1;
   if (EPI == EPI_ACCUM) {
     const int nkb = (K + TILE_K - 1) / TILE_K;
-    double cost;
-    ksplits = cheapest_cut(m_tiles, T, nkb, resident_pairs, &cost);
+    ksplits = ranges > 0 ? ranges : cheapest_cut(m_tiles, T, nkb, resident_pairs);
     if (g_llm_pair_ksplits > 0 && nkb / g_llm_pair_ksplits >= 1) ksplits = g_llm_pair_ksplits;
   }
   const int works = m_tiles * n_tiles * ksplits;
@@ -511,35 +544,40 @@ int launch_form(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap&
 
 template <int STAGES, int EPI, typename TC>
 int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mxs, const CUtensorMap& mc, int T, int N,
-           int K, int half, int sm_count, int* status, cudaStream_t stream, float act_limit = 0.f) {
+           int K, int half, int sm_count, int* status, cudaStream_t stream, float act_limit = 0.f, int ranges = 0) {
+  Grouping g = Grouping();
+  g.k_up = ranges > 0;
   if (short_tail(T)) {
-    // Dealt last, the short items even out the pairs, but they meet every weight a second time: fine
-    // while the weights stay in the L2 (some 48 MB), else they follow their tiles (600 tokens 1,199 ->
-    // 1,187 us, 1,100 tokens 1,869 -> 1,858).
-    Grouping g = Grouping();
-    g.in_order = (long long)N * K * 2 > 48LL << 20;
-    return launch_form<STAGES, EPI, TC, LAST_TOKENS>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream, act_limit, g);
+    g.in_order = tail_in_order(N, K);
+    return launch_form<STAGES, EPI, TC, LAST_TOKENS>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream, act_limit, g,
+                                                     ranges);
   }
-  return launch_form<STAGES, EPI, TC, WHOLE_TILES>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream, act_limit);
+  return launch_form<STAGES, EPI, TC, WHOLE_TILES>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream, act_limit, g,
+                                                   ranges);
 }
 }  // namespace
 
 // How a 32-bit product of many rows with few tiles, for which the caller asked for a split of K, is
-// made soonest: 0 whole sums on pairs, 1 the output cleared and ranges of K added into it on pairs,
-// 2 the same on lone CTAs with tiles of 128 x 128 in `splits` ranges.  In units of one 64-wide block
-// of K of a pair's tile (0.39 us): clearing is a launch and a pass over the output (2.5 us, then
-// 3 TB/s with the additions' own traffic); a lone CTA's block is 1.4 units with two CTAs to an SM.
-// Measured, lone CTAs against the choice made here, with weights from memory: 777 x 4,096 x 1,024
-// (rows x N x K) 29.7 -> 18.4 us, 2,048 x 1,024 x 3,072 39.6 -> 27.4 (ranges of K), 1,501 x 4,096 x 4,096
-// 70.5 -> 56.3, 512 x 6,144 x 4,096 46.1 -> 37.7; 513 x 1,024 x 1,024 stays on lone CTAs (15.4 against
-// 18.4 on pairs).
+// made soonest: 0 without additions in memory on pairs, 1 the output cleared and ranges of K added into
+// it on pairs, 2 the same on lone CTAs with tiles of 128 x 128 in `splits` ranges.  In units of one
+// 64-wide block of K of a pair's tile (0.39 us): clearing is a launch and a pass over the output (2.5
+// us, then 3 TB/s with the additions' own traffic); a lone CTA's block is 1.4 units with two CTAs to an SM.
+// Two sums that are added into zeros commute, so a product that is asked for in two ranges gives the
+// same bits every time, and keeps them in all three ways (two sums in the first, the same two ranges in
+// the second).  Three or more have no order in memory, so how many there are is free.
+// Measured, lone CTAs against the choice made here, with weights from memory: 2,048 x 1,024 x 3,072
+// (rows x N x K) 39.6 -> 27.4 us (ranges of K), 777 x 4,096 x 1,024 29.7 -> 20.5 (two sums; one sum 19.5,
+// two ranges added in memory 26.6), 1,501 x 4,096 x 4,096 70.5 -> 57.3 (two ranges; one sum 56.3, two sums
+// 61.5); 513 x 1,024 x 1,024 stays on lone CTAs (15.4 against 18.4 on pairs).
 int llm_pair_store_way(int T, int N, int K, int splits) {
   const int pairs = 74, nkb = (K + TILE_K - 1) / TILE_K;
   const int m_tiles = (N + 2 * TILE_M - 1) / (2 * TILE_M);
   const double clear = (2.5 + (double)T * N * 4 / 3e6) / 0.39;
-  const double whole = rounds_cost(m_tiles, T, nkb, pairs, 1);
-  double cut;
-  if (cheapest_cut(m_tiles, T, nkb, pairs, &cut) == 1) cut = 1e30;
+  // (two sums leave no accumulator for the next tile: every round but the last waits for its epilogue)
+  const int rounds = (m_tiles * ((T + BN - 1) / BN) + pairs - 1) / pairs;
+  const double whole = rounds_cost(N, K, T, pairs, 1) + (splits == 2 ? 6.0 * (rounds - 1) : 0.0);
+  const int s = splits == 2 ? 2 : cheapest_cut(m_tiles, T, nkb, pairs);
+  const double cut = s == 1 ? 1e30 : rounds_cost(N, K, T, pairs, s);
   const long long lone = (long long)((N + TILE_M - 1) / TILE_M) * ((T + 127) / 128) * splits;
   const double alone = (double)((lone + 4 * pairs - 1) / (4 * pairs)) * (1.4 * nkb / splits + 6.0) + clear;
   if (alone < whole && alone < cut + clear) return 2;
@@ -547,7 +585,8 @@ int llm_pair_store_way(int T, int N, int K, int splits) {
 }
 
 // The pair kernel for bfloat16 X [T][K], W [N][K]; modes 0, 1, 3 and 4 of llm_gemm_tcgen05 (no K
-// split; the gated form only with interleaved rows).  Returns LLM_ERR_UNSUPPORTED when the output
+// split but in mode 1, in `ranges` ranges or, for 0, as many as are soonest, and in mode 0 with 32-bit C
+// as two sums for ranges = 2; the gated form only with interleaved rows).  Returns LLM_ERR_UNSUPPORTED when the output
 // cannot be written by TMA or the mode is not one of these: the caller then uses the one-CTA kernel.
 int g_llm_pair = 1;   // 0: the dispatcher keeps to the one-CTA kernels (for comparisons)
 int g_llm_pair_ksplits = 0;   // > 0: this many ranges of K in the adding epilogue (for measurements)
@@ -566,7 +605,7 @@ static int pair_sm_count() {
 }
 
 int llm_gemm_tcgen05_pair(const void* X, const void* W, void* C, int c_dtype, int T, int N, int K, int lda,
-                          int ldw, int ldc, int mode, int half, float limit, int* status, cudaStream_t stream) {
+                          int ldw, int ldc, int mode, int half, float limit, int ranges, int* status, cudaStream_t stream) {
   if (!g_llm_pair) return LLM_ERR_UNSUPPORTED;
   const int sm_count = pair_sm_count();
   if (mode != 0 && mode != 1 && mode != 3 && mode != 4) return LLM_ERR_UNSUPPORTED;
@@ -580,10 +619,12 @@ int llm_gemm_tcgen05_pair(const void* X, const void* W, void* C, int c_dtype, in
   if (!llm_tensor_map(C, T, out_cols, ldc, CH, mode >= 3 ? 64 : TILE_M, c_dtype == LLM_F32 ? 2 : 1, &mc))
     return LLM_ERR_UNSUPPORTED;
   if (mode == 0) {
+    if (c_dtype == LLM_F32 && ranges == 2)
+      return launch<5, EPI_TWO_SUMS, float>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream);
     if (c_dtype == LLM_F32) return launch<5, EPI_STORE, float>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream);
     if (c_dtype == LLM_BF16) return launch<6, EPI_STORE, bf16>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream);
   } else if (mode == 1) {
-    if (c_dtype == LLM_F32) return launch<5, EPI_ACCUM, float>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream);
+    if (c_dtype == LLM_F32) return launch<5, EPI_ACCUM, float>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream, 0.f, ranges);
   } else {
     if (N != 2 * half || half % 16) return LLM_ERR_ARGUMENT;
     if (mode == 4)
@@ -611,7 +652,7 @@ LLM_EXPORT int llm_gemm_tcgen05_grouped_pair(const void* X, const void* W, void*
   if ((long long)groups * N > 0x7fffffffLL || (mode == 0) != (c_dtype == LLM_F32)) return LLM_ERR_UNSUPPORTED;
   const int esize = c_dtype == LLM_F32 ? 4 : 2;
   if (((uintptr_t)C & 15) || ((size_t)ldc * esize) % 16) return LLM_ERR_UNSUPPORTED;
-  Grouping g;
+  Grouping g = Grouping();
   g.tile_group = tile_group, g.bn = bn, g.n_small = (T + bn - 1) / bn, g.group_rows = N, g.row_scale = row_scale;
   if (g.n_small > MAX_SMALL) return LLM_ERR_UNSUPPORTED;
   CUtensorMap mw, mx, mxs, mc;

@@ -10,7 +10,7 @@ constexpr int UMMA_K = 16;
 
 
 // (the gated ones: silu(g) u, and the clamped form of clamped_swish_mul below)
-enum Epilogue : int { EPI_STORE = 0, EPI_ACCUM = 1, EPI_GATED = 2, EPI_CLAMPED = 3, EPI_RELU2 = 4 };
+enum Epilogue : int { EPI_STORE = 0, EPI_ACCUM = 1, EPI_GATED = 2, EPI_CLAMPED = 3, EPI_RELU2 = 4, EPI_TWO_SUMS = 5 };
 constexpr bool gated_epilogue(int epi) { return epi == EPI_GATED || epi == EPI_CLAMPED; }
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {

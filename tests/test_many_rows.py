@@ -301,3 +301,44 @@ def test_row_product(rows, N, K):
             slack = 2 ** -9 * s * (2 + gate.abs() + up.abs()) if kw else 0
             assert bool(((act.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-5 * (1 + want.abs()) + slack).all())
     kernels.check_tc_status(torch.device(DEV))
+
+
+@gpu
+@pytest.mark.parametrize("T,N,K", [(1501, 4096, 4096), (700, 6144, 1096), (520, 6144, 4096), (2048, 2304, 2056), (900, 4096, 584),
+                                   (1024, 4608, 520)])
+def test_linear_in_two_ranges_keeps_its_sum(T, N, K):
+    """A product that is asked for in two ranges of K is their sum, whichever kernel makes it (odd
+    numbers of blocks of K, ragged N, last tokens)."""
+    from llmario_b200 import kernels
+    assert kernels.k_splits(T, N, K) == 2
+    a, w = rnd(T, K, dtype=torch.bfloat16, seed=1), rnd(N, K, dtype=torch.bfloat16, seed=2)
+    got, lone = torch.empty(T, N, device=DEV), torch.empty(T, N, device=DEV)
+    kernels.linear(a, w, got)
+    kernels.use_cta_pairs(False)
+    try:
+        kernels.linear(a, w, lone)
+    finally:
+        kernels.use_cta_pairs(True)
+    assert torch.equal(got, lone)
+    got.zero_()
+    kernels.linear(a, w, got, out_is_zero=True)
+    assert torch.equal(got, lone)
+    kernels.check_tc_status(torch.device(DEV))
+
+
+@gpu
+@pytest.mark.parametrize("T,N,K", [(513, 4096, 1024), (545, 6144, 3072), (600, 5120, 4096)])
+def test_added_products_stay_whole_with_few_last_tokens(T, N, K):
+    """Where whole tiles are summed over K at once, so are tiles beside a narrow one."""
+    from llmario_b200 import kernels
+    a, w = rnd(T, K, dtype=torch.bfloat16, seed=1), rnd(N, K, dtype=torch.bfloat16, seed=2)
+    got = rnd(T, N, seed=3)
+    whole = got.clone()
+    kernels.linear(a, w, got, accumulate=True)
+    kernels.force_pair_k_ranges(1)
+    try:
+        kernels.linear(a, w, whole, accumulate=True)
+    finally:
+        kernels.force_pair_k_ranges(0)
+    assert torch.equal(got, whole)
+    kernels.check_tc_status(torch.device(DEV))
