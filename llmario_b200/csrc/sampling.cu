@@ -438,6 +438,7 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(
     }
     __syncthreads();
     const int cut = s.control.cut;
+    __syncthreads();                     // (all have read it: the thread that owns the cut writes the word)
     if (cut / PER == (int)threadIdx.x) {
       // `before` stands at the cut for this thread: it left its loop there
       const bool list = before <= CAP && isfinite(inv_t) && floor_logit <= M;
