@@ -128,10 +128,10 @@ def test_device_sampler_matches_plain_chain():
 
 
 def _chain64(l, t, k, p, mp):
-    """(ids, cumulative weights) that the draw walks, in float64, and how near a filter's edge was."""
+    """(ids, cumulative weights) that the draw walks, in float64."""
     ids = np.arange(len(l))
     l = l.astype(np.float64)
-    near, is_sorted = 1.0, False
+    is_sorted = False
     rank = lambda: np.lexsort((ids, -l))  # noqa: E731
     if 0 < k < len(l):
         ids, is_sorted = rank()[:k], True
@@ -139,14 +139,11 @@ def _chain64(l, t, k, p, mp):
         ids, is_sorted = (ids if is_sorted else rank()), True
         w = np.exp(l[ids] - l.max())
         cum = np.cumsum(w) / w.sum()
-        near = np.abs(cum - p).min()
         ids = ids[:np.searchsorted(cum, p) + 1]
     if mp > 0:
-        floor = l.max() + np.log(mp)
-        near = min(near, np.abs(l[ids] - floor).min())
-        ids = ids[l[ids] >= floor]
+        ids = ids[l[ids] >= l.max() + np.log(mp)]
     w = np.exp((l[ids] - l.max()) / t)
-    return ids, np.cumsum(w), near
+    return ids, np.cumsum(w)
 
 
 @pytest.mark.parametrize("vocab,stride", [(1, 1), (7, 7), (333, 333), (2049, 2052), (8191, 8191),
@@ -156,8 +153,7 @@ def test_sample_kernel_over_sizes_and_shapes_of_distributions(vocab, stride):
     """One block below 8,192 logits, a cluster of eight from there; rows whose survivors fit the
     sorted list and rows whose do not (flat, tied, no filter); rows that are not aligned to 16 bytes;
     masked tokens (-inf).  Against the chain in float64: the drawn token's stretch of the cumulative
-    weights holds the uniform.  The kernel's 32-bit weights sum to within vocab * 2**-24 of Z in the
-    worst order, and each is within 2**-22 of the true one: 1e-3 * Z is above both."""
+    weights holds the uniform, to 1e-3 of their sum."""
     from llmario_b200 import kernels
     g = torch.Generator().manual_seed(vocab)
     options = [(1.0, 0, 1.0, 0.0), (0.7, 40, 0.9, 0.0), (1.0, 40, 0.95, 0.05), (0.8, 0, 1.0, 0.1),
@@ -185,18 +181,27 @@ def test_sample_kernel_over_sizes_and_shapes_of_distributions(vocab, stride):
     out = torch.full((n,), -7, dtype=torch.int32, device=DEV)
     kernels.sample(wide.to(DEV)[:, :vocab], col(0, torch.float32), col(1, torch.int32),
                    col(2, torch.float32), col(3, torch.float32), u.to(DEV), out)
+    checked = 0
     for (name, (t, k, p, mp), l), ui, got in zip(rows, u.tolist(), out.tolist()):
         l = l.numpy()
         if t == 0.0:
             assert got == int(np.argmax(l)), (name, t, k, p, mp)
             continue
-        ids, cum, near = _chain64(l, t, k, p, mp)
-        if near < 1e-5:
-            continue          # a filter's edge lies within the rounding of 32-bit sums
-        at = np.flatnonzero(ids == got)
+        # A filter's edge may lie anywhere within the rounding of 32-bit sums (1e-4 of the mass: the
+        # thousands of roundings of a sum do not conspire) and of the floor's logarithm: the token
+        # belongs to the widest set, and its stretch of the weights, from what the narrowest set has
+        # before it to what the widest has up to it, holds the uniform.
+        few, few_cum = _chain64(l, t, k, p - 1e-4 if p < 1 else p, mp * (1 + 1e-5))
+        all_, all_cum = _chain64(l, t, k, p + 1e-4 if p < 1 - 1e-4 else p, mp * (1 - 1e-5))
+        at = np.flatnonzero(all_ == got)
         assert len(at) == 1, (name, t, k, p, mp, got)
-        lo, hi = (cum[at[0] - 1] if at[0] else 0.0), cum[at[0]]
-        assert lo - 1e-3 * cum[-1] <= ui * cum[-1] <= hi + 1e-3 * cum[-1], (name, t, k, p, mp)
+        w = float(all_cum[at[0]] - (all_cum[at[0] - 1] if at[0] else 0.0))
+        where = np.flatnonzero(few == got)
+        lo = float(few_cum[where[0]]) - w if len(where) else float(few_cum[-1])
+        slack = 1e-3 * all_cum[-1]
+        assert lo - slack <= ui * all_cum[-1] and ui * few_cum[-1] <= all_cum[at[0]] + slack, (name, t, k, p, mp)
+        checked += 1
+    assert checked == sum(r[1][0] > 0 for r in rows)
 
 
 def test_device_sampler_penalties_and_streams():
