@@ -8,14 +8,16 @@
 // inverted id): by count for top-k, by accumulated probability mass for top-p and for the draw.
 // Nothing is sorted there and no size is limited.
 //
-// That selection reads a row some twenty times from one block.  Almost every row needs far less:
+// That selection reads a row some twenty times.  Almost every row needs far less:
 // the filters leave a few tokens.  So the blocks of a row first count its logits in bins of 1/64
 // below its maximum (one reading for the maximum, one for the bins), which bounds the tokens that
 // can survive, gather those (a third reading) into the first block's shared memory, sort them there
 // and finish the chain on the sorted list.  A row whose bound is above CAP tokens (no filter, or a
-// flat distribution) goes the general way.  What bounds it: the three readings, from L2 behind the
-// head's product.  64 rows of 151,936 logits with the four mixes of options of a server: 1,248 us
-// with one block per row, 45 us so (one row: 25 us).
+// flat distribution) goes the general way, every block with its slice of the row.  (In the first
+// block alone, 64 rows took 12 to 30 % longer than a grid of one block per row, whose blocks do not
+// share SMs.)  What bounds the short way: the three readings, from L2 behind the head's product.  64
+// rows of 151,936 logits with the four mixes of options of a server: 1,248 us with one block per row,
+// 45 us so (one row: 25 us).
 #include "common.cuh"
 
 #include <cooperative_groups.h>
@@ -41,36 +43,33 @@ __device__ __forceinline__ uint64_t id_key(float, int id) { return (uint32_t)(~(
 
 struct Shared {
   float red[33];
-  float hist_f[256];
-  int hist_i[256];
-  unsigned long long best;
+  float hist_f[256], all_f[256];     // of this block's slice; in the first block also of the row
+  int hist_i[256], all_i[256];
   unsigned long long prefix;
   float carry_f;
   int carry_i;
-  int bin;
 };
 
-// Largest order key of the row (the arg max, lowest id among equals).
-__device__ uint64_t block_best(const float* row, int V, Shared& s) {
-  uint64_t b = 0;
-  for (int i = threadIdx.x; i < V; i += THREADS) {
-    const uint64_t k = order_key(row[i], i);
-    b = k > b ? k : b;
-  }
-  if (threadIdx.x == 0) s.best = 0;
+// All threads of a row's blocks.  (The block's barrier first: threads leave the loops over the
+// logits one by one, and the cluster's barrier counts whole warps.)
+__device__ __forceinline__ void row_sync(const cg::cluster_group& cluster) {
   __syncthreads();
-  atomicMax(&s.best, (unsigned long long)b);
-  __syncthreads();
-  return s.best;
+  cluster.sync();
 }
 
-// Radix selection, most significant byte first.  Elements take part when their order key is
-// >= low.  BY_MASS = false: the `target`-th largest key (target counts from 1).  BY_MASS = true:
-// walking keys downwards, the first key at which the accumulated mass w = exp((l - M) * inv_t)
-// reaches the target (`>=` when inclusive, `>` otherwise); if it never does, the smallest key
-// with non-zero mass.  ID_ORDER walks by ascending token id instead of by logit.
+// A row as its blocks see it: this one has the ids [begin, end).
+struct Row {
+  const float* logits;
+  int begin, end, blocks, rank;
+};
+
+// Radix selection, most significant byte first, by all blocks of a row.  Elements take part when
+// their order key is >= low.  BY_MASS = false: the `target`-th largest key (target counts from 1).
+// BY_MASS = true: walking keys downwards, the first key at which the accumulated mass
+// w = exp((l - M) * inv_t) reaches the target (`>=` when inclusive, `>` otherwise); if it never does,
+// the smallest key with non-zero mass.  ID_ORDER walks by ascending token id instead of by logit.
 template <bool BY_MASS, bool ID_ORDER>
-__device__ uint64_t radix_select(const float* row, int V, uint64_t low, float M, float inv_t,
+__device__ uint64_t radix_select(const cg::cluster_group& cluster, const Row& row, uint64_t low, float M, float inv_t,
                                  float target_f, int target_i, bool inclusive, Shared& s) {
   const int top_byte = ID_ORDER ? 3 : 7;
   if (threadIdx.x == 0) { s.prefix = 0; s.carry_f = 0.f; s.carry_i = 0; }
@@ -80,8 +79,8 @@ __device__ uint64_t radix_select(const float* row, int V, uint64_t low, float M,
     __syncthreads();
     const uint64_t prefix = s.prefix;
     const int shift = 8 * b;
-    for (int i = threadIdx.x; i < V; i += THREADS) {
-      const float l = row[i];
+    for (int i = row.begin + threadIdx.x; i < row.end; i += THREADS) {
+      const float l = row.logits[i];
       if (order_key(l, i) < low) continue;
       const uint64_t k = ID_ORDER ? id_key(l, i) : order_key(l, i);
       if (b < top_byte && (k >> (shift + 8)) != (prefix >> (shift + 8))) continue;
@@ -93,51 +92,68 @@ __device__ uint64_t radix_select(const float* row, int V, uint64_t low, float M,
         atomicAdd(&s.hist_i[bin], 1);
       }
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int chosen = -1, last_nonempty = -1;
-      if (BY_MASS) {
-        float cum = s.carry_f;
-        for (int bin = 255; bin >= 0; --bin) {
-          if (s.hist_i[bin] == 0) continue;
-          last_nonempty = bin;
-          const float next = cum + s.hist_f[bin];
-          // at the last byte a bin is one element: apply the crossing rule exactly there;
-          // before it, descend into the first bin whose end reaches the target
-          const bool hit = inclusive ? (next >= target_f) : (next > target_f);
-          if (hit) { chosen = bin; break; }
-          cum = next;
+    row_sync(cluster);
+    if (row.rank == 0) {
+      for (int i = threadIdx.x; i < 256; i += THREADS) {
+        float f = 0.f;
+        int n = 0;
+        for (int p = 0; p < row.blocks; ++p) {
+          const Shared* peer = cluster.map_shared_rank(&s, p);
+          if (BY_MASS) f += peer->hist_f[i];
+          n += peer->hist_i[i];
         }
-        // never reached (rounding): stay on the smallest keys that carry mass; the carry is
-        // left as it was, so the finer levels do not reach the target either
-        if (chosen < 0) chosen = last_nonempty < 0 ? 0 : last_nonempty;
-        else s.carry_f = cum;
-      } else {
-        int cum = s.carry_i;
-        for (int bin = 255; bin >= 0; --bin) {
-          if (s.hist_i[bin] == 0) continue;
-          last_nonempty = bin;
-          if (cum + s.hist_i[bin] >= target_i) { chosen = bin; break; }
-          cum += s.hist_i[bin];
-        }
-        if (chosen < 0) chosen = last_nonempty < 0 ? 0 : last_nonempty;
-        else s.carry_i = cum;
+        s.all_f[i] = f, s.all_i[i] = n;
       }
-      s.prefix = prefix | ((uint64_t)chosen << shift);
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        int chosen = -1, last_nonempty = -1;
+        if (BY_MASS) {
+          float cum = s.carry_f;
+          for (int bin = 255; bin >= 0; --bin) {
+            if (s.all_i[bin] == 0) continue;
+            last_nonempty = bin;
+            const float next = cum + s.all_f[bin];
+            // at the last byte a bin is one element: apply the crossing rule exactly there;
+            // before it, descend into the first bin whose end reaches the target
+            const bool hit = inclusive ? (next >= target_f) : (next > target_f);
+            if (hit) { chosen = bin; break; }
+            cum = next;
+          }
+          // never reached (rounding): stay on the smallest keys that carry mass; the carry is
+          // left as it was, so the finer levels do not reach the target either
+          if (chosen < 0) chosen = last_nonempty < 0 ? 0 : last_nonempty;
+          else s.carry_f = cum;
+        } else {
+          int cum = s.carry_i;
+          for (int bin = 255; bin >= 0; --bin) {
+            if (s.all_i[bin] == 0) continue;
+            last_nonempty = bin;
+            if (cum + s.all_i[bin] >= target_i) { chosen = bin; break; }
+            cum += s.all_i[bin];
+          }
+          if (chosen < 0) chosen = last_nonempty < 0 ? 0 : last_nonempty;
+          else s.carry_i = cum;
+        }
+        const uint64_t next = prefix | ((uint64_t)chosen << shift);
+        for (int p = 0; p < row.blocks; ++p) cluster.map_shared_rank(&s, p)->prefix = next;
+      }
     }
-    __syncthreads();
+    row_sync(cluster);
   }
-  return s.prefix;
+  const uint64_t found = s.prefix;
+  __syncthreads();
+  return found;
 }
 
-__device__ float block_mass(const float* row, int V, uint64_t low, float M, float inv_t, Shared& s) {
+// The mass of the elements with order keys >= low, in every block of the row.
+__device__ float row_mass(const cg::cluster_group& cluster, const Row& row, uint64_t low, float M, float inv_t,
+                          Shared& s) {
   float z = 0.f;
-  for (int i = threadIdx.x; i < V; i += THREADS) {
-    const float l = row[i];
+  for (int i = row.begin + threadIdx.x; i < row.end; i += THREADS) {
+    const float l = row.logits[i];
     if (order_key(l, i) >= low) z += expf((l - M) * inv_t);
   }
   z = warp_sum(z);
-  __syncthreads();
   if ((threadIdx.x & 31) == 0) s.red[threadIdx.x >> 5] = z;
   __syncthreads();
   if (threadIdx.x < 32) {
@@ -145,22 +161,25 @@ __device__ float block_mass(const float* row, int V, uint64_t low, float M, floa
     t = warp_sum(t);
     if (threadIdx.x == 0) s.red[32] = t;
   }
-  __syncthreads();
-  return s.red[32];
+  row_sync(cluster);
+  float all = 0.f;
+  for (int p = 0; p < row.blocks; ++p) all += cluster.map_shared_rank(&s, p)->red[32];
+  row_sync(cluster);
+  return all;
 }
 
-// The whole chain by radix selection, for one block: any number of survivors.
-__device__ void sample_general(const float* row, int V, float M, float temp, int k, float p, float mp,
-                               double u, int* out, Shared& s) {
+// The whole chain by radix selection, for all blocks of a row: any number of survivors.
+__device__ void sample_general(const cg::cluster_group& cluster, const Row& row, int V, float M, float temp, int k, float p,
+                               float mp, double u, int* out, Shared& s) {
   uint64_t low = 0;
   bool sorted = false;
   if (k > 0 && k < V) {
-    low = radix_select<false, false>(row, V, 0, M, 1.f, 0.f, k, true, s);
+    low = radix_select<false, false>(cluster, row, 0, M, 1.f, 0.f, k, true, s);
     sorted = true;
   }
   if (p < 1.0f && !(k == 1)) {
-    const float Z = block_mass(row, V, low, M, 1.f, s);
-    const uint64_t t = radix_select<true, false>(row, V, low, M, 1.f, p * Z, 0, true, s);
+    const float Z = row_mass(cluster, row, low, M, 1.f, s);
+    const uint64_t t = radix_select<true, false>(cluster, row, low, M, 1.f, p * Z, 0, true, s);
     low = t > low ? t : low;
     sorted = true;
   }
@@ -170,11 +189,11 @@ __device__ void sample_general(const float* row, int V, float M, float temp, int
     low = t > low ? t : low;
   }
   const float inv_t = 1.0f / temp;
-  const float Z = block_mass(row, V, low, M, inv_t, s);
+  const float Z = row_mass(cluster, row, low, M, inv_t, s);
   const float target = (float)(u * (double)Z);
-  const uint64_t pick = sorted ? radix_select<true, false>(row, V, low, M, inv_t, target, 0, false, s)
-                               : radix_select<true, true>(row, V, low, M, inv_t, target, 0, false, s);
-  if (threadIdx.x == 0) *out = (int)(~(uint32_t)(pick & 0xffffffffu));
+  const uint64_t pick = sorted ? radix_select<true, false>(cluster, row, low, M, inv_t, target, 0, false, s)
+                               : radix_select<true, true>(cluster, row, low, M, inv_t, target, 0, false, s);
+  if (row.rank == 0 && threadIdx.x == 0) *out = (int)(~(uint32_t)(pick & 0xffffffffu));
 }
 
 // f(logit, id) for the ids [begin, end) of a row, in batches of four 16-byte loads per thread where
@@ -219,7 +238,6 @@ struct ListShared {
   unsigned long long best[MAX_BLOCKS], warp_best[THREADS / 32];
   double part[THREADS / 32];
   int part_i[THREADS / 32];
-  double total;
   int crossing;
   union {
     struct { alignas(16) int count[BINS]; alignas(16) float mass[BINS]; } bins;
@@ -315,13 +333,6 @@ __device__ __forceinline__ float logit_of_key(uint32_t k) {
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
-// All threads of a row's blocks.  (The block's barrier first: threads leave the loops over the
-// logits one by one, and the cluster's barrier counts whole warps.)
-__device__ __forceinline__ void row_sync(const cg::cluster_group& cluster) {
-  __syncthreads();
-  cluster.sync();
-}
-
 // One cluster of blocks per row (grid: blocks of a row, rows).
 __global__ void __launch_bounds__(THREADS) sample_kernel(
     const float* __restrict__ logits, long long ld, int V, const float* __restrict__ temperature,
@@ -353,8 +364,7 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(
   }
   if ((threadIdx.x & 31) == 0) s.warp_best[threadIdx.x >> 5] = b;
   row_sync(cluster);                     // every block of the row has started
-  // each block hands its best to all of them (plain stores: 64-bit maxima on another block's
-  // shared memory lost updates)
+  // each block hands its best to all of them
   if (threadIdx.x < blocks) {
     for (int w = 0; w < THREADS / 32; ++w) b = s.warp_best[w] > b ? s.warp_best[w] : b;
     cluster.map_shared_rank(&s, threadIdx.x)->best[rank] = b;
@@ -452,7 +462,7 @@ __global__ void __launch_bounds__(THREADS) sample_kernel(
   row_sync(cluster);                        // the first block is done with the bins as well
   const int cut = s.control.cut, n = s.control.n;
   if (cut < 0) {
-    if (rank == 0) sample_general(row, V, M, temp, k, p, mp, uniform[r], out + r, s.general);
+    sample_general(cluster, Row{row, begin, end, blocks, rank}, V, M, temp, k, p, mp, uniform[r], out + r, s.general);
     return;
   }
 
