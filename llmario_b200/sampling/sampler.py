@@ -183,9 +183,16 @@ class DeviceSampler:
                                                  p.presence_penalty)
                     k[r] = p.top_k
                 self._host_key[i] = key
-            # (greedy rows do not advance their streams)
-            next_uniforms([None if s.params.greedy else s.rng for s in samplers],
-                          self._host[i].data_ptr() + 8 * c * 4)
+            # (greedy rows do not advance their streams; samplers with a next_uniform of their own
+            # are asked)
+            streams = [None if s.params.greedy else s.rng for s in samplers]
+            own = [r for r, s in enumerate(samplers)
+                   if type(s) is not RequestSampler or "next_uniform" in s.__dict__]
+            for r in own:
+                streams[r] = None
+            next_uniforms(streams, self._host[i].data_ptr() + 8 * c * 4)
+            for r in own:
+                h[8 * c:10 * c].view(np.float64)[r] = samplers[r].next_uniform()
             self._dev.copy_(self._host[i], non_blocking=True)
             self.h2d_bytes += self._host[i].numel() * 4
             self._host_event[i] = torch.cuda.Event()

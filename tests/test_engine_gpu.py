@@ -232,6 +232,24 @@ def test_device_sampler_penalties_and_streams():
     assert abs(freqs[0] - 0.5) < 0.09 and abs(freqs[1] - 0.3) < 0.09 and abs(freqs[2] - 0.2) < 0.08
 
 
+def test_samplers_with_their_own_uniforms_are_asked():
+    from llmario_b200.sampling import DeviceSampler, RequestSampler, SamplingParams
+
+    class Fixed(RequestSampler):
+        def next_uniform(self):
+            return 0.9
+
+    V = 4
+    params = SamplingParams(temperature=1.0, top_k=0, top_p=1.0, min_p=0.0, seed=1)
+    patched = RequestSampler(params, V)
+    patched.next_uniform = lambda: 0.6
+    foreign = RequestSampler(params, V)
+    foreign.rng = type("Rng", (), {"next_f64": lambda self: 0.3})()
+    rows = [Fixed(params, V), patched, foreign, RequestSampler(SamplingParams(temperature=0), V)]
+    logits = torch.log(torch.tensor([[0.25, 0.25, 0.25, 0.25]])).repeat(4, 1)
+    assert DeviceSampler(DEV).sample(logits.to(DEV), rows) == [3, 2, 1, 0]
+
+
 def test_penalties_count_a_token_in_flight():
     """A step queued ahead draws with penalties while the token that just entered the window is
     still on the device: the sampler gets the counts without that token and the row of the draw

@@ -200,6 +200,44 @@ def test_uniforms_of_many_streams():
     assert mine[3].next_u64() == alone[3].next_u64()
 
 
+def test_a_stream_is_saved_restored_and_copied():
+    """A request's sampling state goes through pickle in the middle of its stream, as its four numbers
+    do through JSON; the numbers may be set, or changed in place; what earlier versions saved is read."""
+    import copy
+    import ctypes
+    import json
+    import pickle
+    from llmario_b200.sampling import RequestSampler, SamplingParams
+    from llmario_b200.sampling.rng import Xoshiro256StarStar, next_uniforms
+    a = RequestSampler(SamplingParams(seed=3), 100)
+    a.next_uniform()
+    b = pickle.loads(pickle.dumps(a))
+    c, text = copy.deepcopy(a), json.dumps(a.rng.s)
+    d = Xoshiro256StarStar(99)
+    d.s = json.loads(text)
+    old = Xoshiro256StarStar.__new__(Xoshiro256StarStar)
+    old.__setstate__({"s": json.loads(text)})
+    e = Xoshiro256StarStar(0)
+    e.s[:] = json.loads(text)
+    assert isinstance(a.rng.s, list) and d.s == a.rng.s == e.s
+
+    class Twice(Xoshiro256StarStar):
+        def next_f64(self):
+            return super().next_f64() / 2
+
+    half, plain = Twice(3), Xoshiro256StarStar(3)
+    half.next_u64(), plain.next_u64()
+    out = (ctypes.c_double * 7)()
+    for _ in range(3):
+        next_uniforms([a.rng, b.rng, c.rng, d, old, e, half], ctypes.addressof(out))
+        want = plain.next_f64()
+        assert list(out) == [want] * 6 + [want / 2]
+    assert a.rng.s == d.s == plain.s and a.rng.next_u64() == plain.next_u64()
+    shared = copy.copy(plain)                    # a shallow copy is the same stream
+    first = plain.next_u64()
+    assert shared.next_u64() != first and shared.s is plain.s
+
+
 @gpu
 @pytest.mark.parametrize("bn", (32, 64, 128))
 @pytest.mark.parametrize("counts,N,K", [([300, 0, 1, 129, 256, 64], 512, 256), ([700, 33, 32], 272, 72),
