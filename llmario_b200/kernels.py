@@ -1043,6 +1043,7 @@ def linear(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: bool
     ``out_is_zero``: the caller guarantees that ``out`` holds zeros, so a split-K product need
     not clear it first."""
     if (a.shape[0] <= 4 and out.dtype == torch.float32 and _tc_ok(a, w) and w.is_contiguous()
+            and w.shape[1] == a.shape[1] and out.shape == (a.shape[0], w.shape[0])
             and out.stride(1) == 1 and row_product_ok(a.shape[0], w.shape[0], a.shape[1])):
         row_product(a, w, out, accumulate)
     elif _tc_ok(a, w, out):

@@ -380,3 +380,20 @@ def test_added_products_stay_whole_with_few_last_tokens(T, N, K):
         kernels.force_pair_k_ranges(0)
     assert torch.equal(got, whole)
     kernels.check_tc_status(torch.device(DEV))
+
+
+@gpu
+@pytest.mark.parametrize("rows", (1, 3))
+def test_linear_takes_wider_operands_at_few_rows(rows):
+    """A matrix with more columns than the rows have, and an output with more rows and columns than
+    the product: the leading part is what is used, whatever the number of rows."""
+    from llmario_b200 import kernels
+    a = rnd(rows, 1024, dtype=torch.bfloat16, seed=1)
+    w = rnd(96, 1280, dtype=torch.bfloat16, seed=2)
+    out = torch.zeros(rows + 2, 128, device=DEV)
+    kernels.linear(a, w, out)
+    ref = a.double() @ w[:, :1024].double().T
+    bound = (1024 + 10) * 2 ** -23 * (a.abs().double() @ w[:, :1024].abs().double().T)
+    assert bool(((out[:rows, :96].double() - ref).abs() <= bound).all())
+    assert not out[rows:].any() and not out[:, 96:].any()
+    kernels.check_tc_status(torch.device(DEV))
