@@ -11,9 +11,11 @@
 // Everything here is 32-bit: the inputs are the 32-bit results of the projections, the state
 // lives in 32-bit floats in the request's state slot, decays and step sizes are made here from
 // the projected values.  The tokens of a request are visited one after the other and every sum
-// has a fixed order.  The diagonal recurrence cuts long portions into runs that are walked at the
-// same time (recurrence_runs_kernel), so how a prompt was cut into steps changes a token's result by
-// the rounding of 32-bit sums; the other recurrences, and its short portions, give the same bits.
+// has a fixed order, so a token's result is the same bits whatever else is in the step.  The diagonal
+// recurrence cuts long portions into runs that are walked at the same time (recurrence_runs_kernel):
+// whether and where follows from the portion's own length, so how a prompt was cut into steps changes
+// a token's result by the rounding of 32-bit sums, and the other portions of a step do not.  The other
+// recurrences, and short portions, give the same bits however a prompt was cut.
 //
 // Which rows of a step belong to which request is read on the device: either every row is a
 // request of its own (`single`: slot = row_slot[row]), or a table of (first row, end row) per
@@ -80,9 +82,10 @@ struct ScanArgs {
   // `unit`: q and k of every head are divided by sqrt(sum of squares + unit_floor) first
   const float* beta; int beta_stride;
   int unit; float unit_floor;
-  int parts, part_rows;                  // runs a request's rows are cut into, and their length
-  float* part_state;                     // [request of the step][run][H][V][K]
-  float* part_decay;                     // [request of the step][run][H][K] (one number with a scalar decay)
+  int long_rows, least_run;              // requests with so many rows (0: none) are cut into runs (run_rows)
+  int n_requests;
+  float* part_state;                     // [run of the step][H][V][K]
+  float* part_decay;                     // [run of the step][H][K] (one number with a scalar decay)
   int tail_only;        // only the last (rows of the request) % 4 rows: the others went in groups of four
 };
 
@@ -141,7 +144,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) linear_recurrence_kernel(const S
     first = a.seg[SEG * slot], end = a.seg[SEG * slot + 1];
   }
   if (a.tail_only) first = end - ((end - first) & 3);
-  if (end <= first) return;
+  if (end <= first || (a.long_rows > 0 && end - first >= a.long_rows)) return;     // (the latter in runs)
   const int K = a.K, V = a.V, g = h / (a.H / a.G);
   const int j0 = blockIdx.z * COLS;
   const int li = lane % L;
@@ -394,7 +397,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) linear_recurrence_kernel(const S
 // ---- long portions in runs.  The walk above is one chain per block: a token's shared-memory reads
 // and shuffles, some 450 cycles, with one or two warps per scheduler (a prompt of 2,048 tokens on 4
 // heads of 128 x 256: 64 blocks on 148 SMs, 436 us; on 32 heads of 128 x 64 492 us).  The recurrence is a
-// diagonal map, so a portion can be cut into runs of part_rows that are walked at the same time:
+// diagonal map, so a portion can be cut into runs that are walked at the same time:
 //   FOLD    each run but the last from a zero state, no outputs: what the run adds to the state,
 //           and the product of its decays;
 //   carry   (scan_carry_kernel) the states that enter the runs, one after the other;
@@ -422,6 +425,55 @@ __device__ __forceinline__ float pair_lo(pair_f32 v) { return __uint_as_float((u
 __device__ __forceinline__ float pair_hi(pair_f32 v) { return __uint_as_float((uint32_t)(v >> 32)); }
 
 constexpr int RUN_COLS = 8;      // columns per lane
+constexpr int MOST_RUNS = 32;    // of a portion
+
+// the rows of a run of a portion of so many
+__host__ __device__ __forceinline__ int run_rows(int rows, int least) {
+  const int even = (rows + 16 * MOST_RUNS - 1) / (16 * MOST_RUNS) * 16;
+  return even > least ? even : least;
+}
+
+// What a block of the kernels below works on: the runs of the step's long requests are numbered
+// through, in the order of the table, and so are those requests.  A whole warp asks for the request
+// that holds run `index` (or, BY_REQUEST, for request `index`); slot < 0: there is none.
+struct LongRequest {
+  int slot, first, rows;
+  int run0;              // number of its first run
+};
+template <bool BY_REQUEST>
+__device__ __forceinline__ LongRequest find_long(const ScanArgs& a, int index, int lane) {
+  LongRequest found = {-1, 0, 0, 0};
+  int runs_before = 0, requests_before = 0;
+  for (int base = 0; base < a.n_requests; base += 32) {
+    int slot = base + lane < a.n_requests ? a.seg[SEG * (base + lane) + 2] : -1, first = 0, rows = 0;
+    if (slot >= 0) first = a.seg[SEG * slot], rows = a.seg[SEG * slot + 1] - first;
+    const bool is_long = slot >= 0 && rows >= a.long_rows;
+    const unsigned longs = __ballot_sync(0xffffffffu, is_long);
+    if (longs == 0) continue;
+    const int length = run_rows(rows, a.least_run), runs = is_long ? (rows + length - 1) / length : 0;
+    int upto = runs;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const int my_run0 = runs_before + upto - runs;
+    const int my_request = requests_before + __popc(longs & ((1u << lane) - 1));
+    const bool here = is_long && (BY_REQUEST ? my_request == index : index >= my_run0 && index < my_run0 + runs);
+    const unsigned hit = __ballot_sync(0xffffffffu, here);
+    if (hit) {
+      const int from = __ffs(hit) - 1;
+      found.slot = __shfl_sync(0xffffffffu, slot, from);
+      found.first = __shfl_sync(0xffffffffu, first, from);
+      found.rows = __shfl_sync(0xffffffffu, rows, from);
+      found.run0 = __shfl_sync(0xffffffffu, my_run0, from);
+      return found;
+    }
+    runs_before += __shfl_sync(0xffffffffu, upto, 31);
+    requests_before += __popc(longs);
+  }
+  return found;
+}
 
 template <int L, int NF, bool VEC, bool FOLD>
 __global__ void __launch_bounds__(SCAN_THREADS) recurrence_runs_kernel(const ScanArgs a) {
@@ -438,15 +490,14 @@ __global__ void __launch_bounds__(SCAN_THREADS) recurrence_runs_kernel(const Sca
   pdl_trigger();
   pdl_wait();
   const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int request = blockIdx.x / a.parts, run = blockIdx.x - request * a.parts;
-  const int slot = a.seg[SEG * request + 2];
+  const LongRequest request = find_long<false>(a, blockIdx.x, lane);
+  const int slot = request.slot, length = run_rows(request.rows, a.least_run);
   if (slot < 0) return;
-  const int first = a.seg[SEG * slot] + run * a.part_rows;
-  int end = a.seg[SEG * slot + 1];
-  if (end <= first) return;
-  const bool last_run = end - first <= a.part_rows;
+  const int first = request.first + (blockIdx.x - request.run0) * length;
+  int end = request.first + request.rows;
+  const bool last_run = end - first <= length;
   if (FOLD && last_run) return;
-  if (!last_run) end = first + a.part_rows;
+  if (!last_run) end = first + length;
   const int K = a.K, V = a.V, g = h / (a.H / a.G);
   const int j0 = blockIdx.z * COLS;
   const int li = lane % L;
@@ -656,18 +707,18 @@ __global__ void __launch_bounds__(SCAN_THREADS) recurrence_runs_kernel(const Sca
 __global__ void __launch_bounds__(256) scan_carry_kernel(const ScanArgs a, int per_channel) {
   pdl_trigger();
   pdl_wait();
-  const int slot = a.seg[SEG * blockIdx.y + 2];
+  const LongRequest request = find_long<true>(a, blockIdx.y, threadIdx.x & 31);
+  const int slot = request.slot, length = run_rows(request.rows, a.least_run);
   if (slot < 0) return;
-  const int rows = a.seg[SEG * slot + 1] - a.seg[SEG * slot];
-  const int runs = (rows + a.part_rows - 1) / a.part_rows;
+  const int runs = (request.rows + length - 1) / length;
   const long long size = (long long)a.H * a.V * a.K;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= size) return;
   const int h = (int)(i / ((long long)a.V * a.K)), ch = (int)(i % a.K);
   float s = a.state[(size_t)slot * a.state_stride + i];
-  float* part = a.part_state + (size_t)blockIdx.y * a.parts * size + i;
-  const float* decay = per_channel ? a.part_decay + ((size_t)blockIdx.y * a.parts * a.H + h) * a.K + ch
-                                   : a.part_decay + (size_t)blockIdx.y * a.parts * a.H + h;
+  float* part = a.part_state + (size_t)request.run0 * size + i;
+  const float* decay = per_channel ? a.part_decay + ((size_t)request.run0 * a.H + h) * a.K + ch
+                                   : a.part_decay + (size_t)request.run0 * a.H + h;
   const size_t step = (size_t)a.H * (per_channel ? a.K : 1);
   for (int r = 0; r < runs; r += 4) {      // four runs' loads are under way together
     float add[4], keep[4];
@@ -686,21 +737,21 @@ __global__ void __launch_bounds__(256) scan_carry_kernel(const ScanArgs a, int p
 }
 
 template <int L, int NF, bool VEC>
-int launch_runs(const ScanArgs& a, int n_requests, cudaStream_t stream) {
+int launch_runs(const ScanArgs& a, int n_long, int n_runs, cudaStream_t stream) {
   constexpr int COLS = RUN_COLS * (32 / L) * (SCAN_THREADS / 32);
-  const dim3 grid(n_requests * a.parts, a.H, (a.V + COLS - 1) / COLS);
+  const dim3 grid(n_runs, a.H, (a.V + COLS - 1) / COLS);
   int rc = launch_pdl(recurrence_runs_kernel<L, NF, VEC, true>, grid, SCAN_THREADS, 0, stream, a);
   if (rc) return rc;
   next_launch_plain();      // (blocks that wait would take the fold's places)
   const long long size = (long long)a.H * a.V * a.K;
-  rc = launch_pdl(scan_carry_kernel, dim3((unsigned)((size + 255) / 256), n_requests), 256, 0, stream, a, (int)VEC);
+  rc = launch_pdl(scan_carry_kernel, dim3((unsigned)((size + 255) / 256), n_long), 256, 0, stream, a, (int)VEC);
   if (rc) return rc;
   return launch_pdl(recurrence_runs_kernel<L, NF, VEC, false>, grid, SCAN_THREADS, 0, stream, a);
 }
 
-static int run_in_runs(const ScanArgs& a, int n_requests, cudaStream_t stream) {
+static int run_in_runs(const ScanArgs& a, int n_long, int n_runs, cudaStream_t stream) {
   const bool scalar = a.kind == DECAY_RATE_STEP || a.kind == DECAY_SCALAR_INPUT;
-#define RUNS(L, NF) return scalar ? launch_runs<L, NF, false>(a, n_requests, stream) : launch_runs<L, NF, true>(a, n_requests, stream)
+#define RUNS(L, NF) return scalar ? launch_runs<L, NF, false>(a, n_long, n_runs, stream) : launch_runs<L, NF, true>(a, n_long, n_runs, stream)
   if (a.K <= 32) RUNS(8, 1);
   if (a.K <= 64) RUNS(16, 1);
   if (a.K <= 128) RUNS(32, 1);
@@ -1473,17 +1524,20 @@ static int run_scan(ScanArgs& a, int rows, int n_requests, cudaStream_t stream) 
 // channel fastest.  `ones`: v has V - 1 channels per head and the state's last column is fed the
 // constant 1, so that it holds the decayed sum of the keys alone and the last output channel is
 // its product with the query (the normaliser of a matrix memory).
-// parts > 1 (K up to 256): every request's rows are cut into runs of part_rows, at most `parts` of
-// them, which are walked at the same time; `work` holds n_requests * parts * H * (V + 1) * K floats.
+// n_long > 0 (K up to 256): so many requests have long_rows rows or more; they are cut into runs of
+// run_rows(rows, least_run) rows, n_runs in all, which are walked at the same time; `work` holds
+// n_runs * H * (V + 1) * K floats.
 LLM_EXPORT int llm_linear_recurrence(const float* q, int q_stride, const float* k, int k_stride, const float* v,
                                      int v_stride, const float* d, int d_stride, const float* d2, int ones,
                                      const float* p0, const float* p1, float c, float q_scale, float* state,
                                      long long state_stride, float* out, int out_stride, const int* seg,
                                      const int* row_slot, int rows, int n_requests, int single, int H, int G,
-                                     int K, int V, int kind, int parts, int part_rows, float* work,
-                                     cudaStream_t stream) {
+                                     int K, int V, int kind, int n_long, int long_rows, int least_run, int n_runs,
+                                     float* work, cudaStream_t stream) {
   if (rows <= 0) return 0;
-  if (parts > 1 && (single || !work || part_rows <= 0 || n_requests > 65535 || K > 256)) return LLM_ERR_ARGUMENT;
+  if (n_long > 0 && (single || !seg || !work || long_rows <= 0 || least_run <= 0 || n_runs < n_long || n_long > n_requests ||
+                     n_long > 65535 || K > 256))
+    return LLM_ERR_ARGUMENT;
   if (H <= 0 || G <= 0 || H % G || K <= 0 || V <= 0 || kind < 0 || kind > 3) return LLM_ERR_ARGUMENT;
   if (kind == DECAY_RATE_STEP && (!p0 || !p1)) return LLM_ERR_ARGUMENT;
   if (kind == DECAY_SCALAR_INPUT && !d2) return LLM_ERR_ARGUMENT;
@@ -1498,9 +1552,11 @@ LLM_EXPORT int llm_linear_recurrence(const float* q, int q_stride, const float* 
   a.seg = seg, a.row_slot = row_slot;
   a.single = single, a.H = H, a.G = G, a.K = K, a.V = V, a.kind = kind;
   a.beta = nullptr, a.beta_stride = 0, a.unit = 0, a.unit_floor = 0.f, a.tail_only = 0;
-  a.parts = parts > 1 ? parts : 1, a.part_rows = part_rows, a.part_state = work;
-  a.part_decay = parts > 1 ? work + (size_t)n_requests * parts * H * V * K : nullptr;
-  const int rc = parts > 1 ? run_in_runs(a, n_requests, stream) : run_scan(a, rows, n_requests, stream);
+  a.long_rows = n_long > 0 ? long_rows : 0, a.least_run = least_run, a.n_requests = n_requests, a.part_state = work;
+  a.part_decay = n_long > 0 ? work + (size_t)n_runs * H * V * K : nullptr;
+  int rc = 0;
+  if (n_long <= 0 || n_long < n_requests) rc = run_scan(a, rows, n_requests, stream);
+  if (rc == 0 && n_long > 0) rc = run_in_runs(a, n_long, n_runs, stream);
   if (!single) next_launch_plain();      // (whatever follows the walk of a portion)
   return rc;
 }
@@ -1535,7 +1591,7 @@ LLM_EXPORT int llm_delta_recurrence_grouped(const float* q, int q_stride, const 
   a.seg = seg, a.row_slot = row_slot;
   a.single = single, a.H = H, a.G = G, a.K = K, a.V = V, a.kind = kind;
   a.beta = beta, a.beta_stride = beta_stride, a.unit = unit ? 1 : 0, a.unit_floor = unit_floor, a.tail_only = 0;
-  a.parts = 1, a.part_rows = 0, a.part_state = a.part_decay = nullptr;
+  a.long_rows = a.least_run = a.n_requests = 0, a.part_state = a.part_decay = nullptr;
   // Portions of prompts with 68 to 256 key channels go four tokens at a time: what a group needs
   // is prepared once per head in parallel over the tokens, the walk takes a group per round, and
   // the token-by-token kernel takes the rows that are left (fewer than four a request).

@@ -9,7 +9,7 @@ from __future__ import annotations
 import contextlib
 import ctypes
 from ctypes import c_float, c_int, c_longlong, c_void_p
-from typing import Optional, Tuple
+from typing import List, Optional, Sequence, Tuple
 
 import torch
 
@@ -98,7 +98,7 @@ def _signatures():
         "llm_segment_table": [P, I, P, I, P],
         "llm_bias_sigmoid_pow": [P, P, I, I, F, P],
         "llm_linear_recurrence": [P, I, P, I, P, I, P, I, P, I, P, P, F, F, P, L, P, I, P, P, I, I,
-                                  I, I, I, I, I, I, I, I, P, P],
+                                  I, I, I, I, I, I, I, I, I, I, P, P],
         "llm_log_gate_scan": [P, P, I, P, P, F, P, L, P, I, P, P, I, I, I, I, P],
         "llm_memory_out_norm": [P, I, P, I, P, I, P, P, I, I, I, I, I, F, F, P],
         "llm_stream_step": [P, L, I, P, P, P, I, I, P, P, F, P, I, P, I, I, P],
@@ -499,7 +499,8 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, d: torc
                       rate_log: Optional[torch.Tensor] = None,
                       step_bias: Optional[torch.Tensor] = None, n_requests: int = 0,
                       input_weight: Optional[torch.Tensor] = None, ones: bool = False,
-                      work: Optional[torch.Tensor] = None) -> None:
+                      work: Optional[torch.Tensor] = None,
+                      portions: Sequence[int] = ()) -> None:
     """Per request and head ``S <- diag(a_t) S + k_t v_t^T``, ``o_t = S^T (q_scale q_t)`` over
     the rows of the step in order.  q, k float32 [rows, groups * key_dim], v and out float32
     [rows, heads * value_dim] (column slices of wider matrices are fine); head h uses group
@@ -514,9 +515,11 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, d: torc
     holds the decayed sum of the keys, and the last output channel its product with q).
     ``seg``: the table of :func:`segment_table` with ``n_requests`` the
     number of requests that have rows in the step, or None when every row is a request of its
-    own.  ``work`` (float32, at least :func:`recurrence_work_floats` elements): room for the
-    states between the runs that :func:`recurrence_runs` cuts long portions into; without it
-    every portion is walked as a whole.  The two ways differ by rounding only."""
+    own.  ``portions`` (how many rows each of those requests has, in any order) and ``work`` (float32,
+    at least :func:`recurrence_work_floats` elements: room for the states between runs): requests
+    with as many rows as :func:`recurrence_runs` cuts go in runs; without them every portion is
+    walked as a whole.  The two ways differ by rounding only, and which one a request goes, and how
+    it is cut, does not depend on the other requests."""
     _cuda(q, k, v, d, state, out, row_slot, seg, rate_log, step_bias, input_weight, work)
     assert work is None or (work.dtype == torch.float32 and work.is_contiguous())
     for t in (q, k, v, d, state, out):
@@ -525,49 +528,76 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, d: torc
     assert state.dim() == 2 and state.shape[1] >= heads * value_dim * key_dim
     if input_weight is not None:
         assert input_weight.dtype == torch.float32 and input_weight.stride(0) == d.stride(0)
-    parts, part_rows = 1, 0
+    cuts = []
     if work is not None and seg is not None:
-        parts, part_rows = recurrence_runs(rows, n_requests, heads, key_dim, value_dim)
-        need = recurrence_work_floats(rows, n_requests, heads, key_dim, value_dim)
+        assert len(portions) == n_requests and sum(portions) == rows
+        cuts = _long_cuts(portions, heads, key_dim, value_dim)
+        need = recurrence_work_floats(portions, heads, key_dim, value_dim)
         if work.numel() < need:
             raise KernelError(f"linear_recurrence: {need} floats of work are needed, "
                               f"{work.numel()} given")
+    long_rows, least_run = _run_limits(heads, key_dim, value_dim)
     _check(lib().llm_linear_recurrence(
         _ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(d), d.stride(0),
         _ptr(input_weight), int(ones), _ptr(rate_log), _ptr(step_bias), float(exponent), float(q_scale), _ptr(state),
         state.stride(0), _ptr(out), out.stride(0), _ptr(seg), _ptr(row_slot), rows,
-        int(n_requests), int(seg is None), heads, groups, key_dim, value_dim, kind, parts,
-        part_rows, _ptr(work) if parts > 1 else None, _stream()),
+        int(n_requests), int(seg is None), heads, groups, key_dim, value_dim, kind, len(cuts),
+        long_rows, least_run, sum(cuts), _ptr(work) if cuts else None, _stream()),
         f"linear_recurrence (key_dim {key_dim})")
     global launches
-    launches += 2 * int(parts > 1)      # the folds and the states between the runs
+    if cuts:          # folds, the states between runs and the runs, beside the walk of the others
+        launches += 2 + int(len(cuts) < n_requests)
 
 
-def recurrence_runs(rows: int, n_requests: int, heads: int, key_dim: int,
-                    value_dim: int) -> Tuple[int, int]:
-    """Into how many runs of how many rows the portions of a step's requests are cut for
-    :func:`linear_recurrence`, (1, 0) for none.  A block of the runs has 128, 64 or 32 value
-    channels of a head; portions are cut so that about 2,000 blocks run (three to four rounds).
-    The runs cost half as much arithmetic again: with up to 64 blocks to the whole walk (one or
-    two warps per scheduler) they pay from 192 rows a request on (4 heads of 128 x 256, 192 / 512 /
-    2,048 rows: 47 / 115 / 436 -> 42 / 50 / 124 us; 32 heads of 128 x 64: 53 / 129 / 492 -> 50 / 81 / 228),
-    with up to 128 from 1,024 rows on (16 heads of 128 x 256, 512 / 1,024 / 2,048 rows: 136 / 265 / 522
-    -> 130 / 218 / 402), beyond that not (128 heads of 128 x 64, 2,048 rows: 739 -> 775)."""
+def _run_limits(heads: int, key_dim: int, value_dim: int) -> Tuple[int, int]:
+    """(rows from which a portion is cut into runs, least rows of a run), (0, 0) for never.  A block
+    of the runs has 128, 64 or 32 value channels of a head; the runs cost half as much arithmetic
+    again as the whole walk, which pays while the walk's blocks leave the GPU idle.  Both numbers are of
+    the layer alone, so that a request's bits do not depend on its company; they are chosen so that
+    one portion gains and a step of 2,048 rows full of them does not lose much.  Whole walk -> runs in us,
+    one portion / portions that fill 2,048 rows:
+    32 blocks (4 heads of 128 x 256), from 256 rows: 256 rows 60 -> 41 / 97 -> 128, 512 113 -> 50 / 136 -> 128,
+    2,048 435 -> 121; (192 rows 48 -> 45 / 74 -> 105);
+    64 blocks (32 heads of 128 x 64), from 384 rows: 384 rows 99 -> 76 / 146 -> 179, 512 127 -> 80 / 191 -> 228,
+    1,024 248 -> 125 / 286 -> 228, 2,048 492 -> 232; (256 rows 68 -> 70 / 154 -> 224);
+    128 blocks (16 heads of 128 x 256), from 1,024 rows: 1,024 rows 265 -> 211 / 359 -> 402, 2,048 521 -> 400;
+    (512 rows 136 -> 130 / 285 -> 381);
+    more: never (128 heads of 128 x 64, 2,048 rows: 739 -> 775).
+    Shorter runs would serve one portion of few rows (64 blocks, 512 rows: 77 with runs of 32) and cost
+    a full step (291): every run brings its state from memory and takes it back."""
     columns = 128 if key_dim <= 32 else 64 if key_dim <= 64 else 32
-    blocks = max(1, n_requests) * heads * -(-value_dim // columns)
-    if key_dim > 256 or blocks > 128 or rows < (192 if blocks <= 64 else 1024) * n_requests:
+    blocks = heads * -(-value_dim // columns)
+    if key_dim > 256 or blocks > 128:
+        return 0, 0
+    return (256 if blocks <= 32 else 384 if blocks <= 64 else 1024), 32 * -(-blocks // 32)
+
+
+MOST_RUNS = 32           # of a portion
+
+
+def recurrence_runs(rows: int, heads: int, key_dim: int, value_dim: int) -> Tuple[int, int]:
+    """Into how many runs of how many rows :func:`linear_recurrence` cuts a request that has
+    ``rows`` rows in the step, (1, 0) when it walks them as a whole."""
+    long_rows, least_run = _run_limits(heads, key_dim, value_dim)
+    if long_rows == 0 or rows < long_rows:
         return 1, 0
-    parts = min(32, -(-2000 // blocks))
-    part_rows = max(32, -(-rows // (16 * parts)) * 16)
-    return -(-rows // part_rows), part_rows
+    length = max(least_run, 16 * -(-rows // (16 * MOST_RUNS)))
+    return -(-rows // length), length
 
 
-def recurrence_work_floats(rows: int, n_requests: int, heads: int, key_dim: int,
+def _long_cuts(portions: Sequence[int], heads: int, key_dim: int, value_dim: int) -> List[int]:
+    """Into how many runs each of the portions that are cut goes."""
+    long_rows, _ = _run_limits(heads, key_dim, value_dim)
+    return [recurrence_runs(n, heads, key_dim, value_dim)[0] for n in portions
+            if long_rows and n >= long_rows]
+
+
+def recurrence_work_floats(portions: Sequence[int], heads: int, key_dim: int,
                            value_dim: int) -> int:
-    """Elements of ``work`` with which :func:`linear_recurrence` cuts portions into runs, 0 when
-    it would not cut them."""
-    parts, _ = recurrence_runs(rows, n_requests, heads, key_dim, value_dim)
-    return n_requests * parts * heads * (value_dim + 1) * key_dim if parts > 1 else 0
+    """Elements of ``work`` with which :func:`linear_recurrence` cuts the long ones of these
+    portions into runs, 0 when none is cut."""
+    return (sum(_long_cuts(portions, heads, key_dim, value_dim))
+            * heads * (value_dim + 1) * key_dim)
 
 
 def bias_sigmoid_pow(z: torch.Tensor, bias: Optional[torch.Tensor], exponent: float) -> None:

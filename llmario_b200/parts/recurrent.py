@@ -67,13 +67,13 @@ def step_segments(ctx: StepContext) -> Optional[torch.Tensor]:
     return seg
 
 
-def _runs_work(ctx: StepContext, heads: int, key_dim: int, value_dim: int
-               ) -> Optional[torch.Tensor]:
-    """Room for the states between the runs of long portions (None: nothing is cut)."""
+def _runs(ctx: StepContext, heads: int, key_dim: int, value_dim: int) -> Dict[str, object]:
+    """The arguments with which long portions go in runs (none when no portion is cut)."""
     if ctx.rows == len(ctx.segments):
-        return None
-    n = kernels.recurrence_work_floats(ctx.rows, len(ctx.segments), heads, key_dim, value_dim)
-    return ctx.buffer("scan.work", (n,), torch.float32) if n else None
+        return {}
+    portions = [s.rows for s in ctx.segments]
+    n = kernels.recurrence_work_floats(portions, heads, key_dim, value_dim)
+    return dict(work=ctx.buffer("scan.work", (n,), torch.float32), portions=portions) if n else {}
 
 
 def _f32(t: torch.Tensor, device) -> torch.Tensor:
@@ -148,7 +148,7 @@ class GatedLinearAttention:
         kernels.linear_recurrence(
             proj[:, :self.col_k], proj[:, self.col_k:self.col_v], proj[:, self.col_v:self.col_g],
             z, state, o, ctx.row_slot, step_segments(ctx), H, H, K, V, kernels.DECAY_VECTOR,
-            q_scale=K ** -0.5, n_requests=len(ctx.segments), work=_runs_work(ctx, H, K, V))
+            q_scale=K ** -0.5, n_requests=len(ctx.segments), **_runs(ctx, H, K, V))
         gated = ctx.buffer("gla.gated", (rows, H * V))
         kernels.gated_group_norm(o, proj[:, self.col_g:self.col_a], self.norm_weight, gated,
                                  group=V, eps=self.eps, gate_first=False)
@@ -216,7 +216,7 @@ class StateSpaceMixer:
             xbc[:, self.inner + G * N:], xbc[:, self.inner:self.inner + G * N], xbc[:, :self.inner],
             proj[:, self.col_dt:self.col_dt + H], state, o, ctx.row_slot, seg, H, G, N, P,
             kernels.DECAY_RATE_STEP, rate_log=self.rate_log, step_bias=self.step_bias,
-            n_requests=len(ctx.segments), work=_runs_work(ctx, H, N, P))
+            n_requests=len(ctx.segments), **_runs(ctx, H, N, P))
         gated = ctx.buffer("ssm.gated", (rows, self.inner))
         kernels.gated_group_norm(o, proj[:, :self.inner], self.norm_weight, gated,
                                  group=self.inner // self.norm_groups, eps=self.eps,
@@ -280,7 +280,7 @@ class MatrixMemory:
             proj[:, :self.col_k], proj[:, self.col_k:self.col_v], proj[:, self.col_v:self.col_g],
             gates[:, :H], state, o, ctx.row_slot, seg, H, H, K, V + 1,
             kernels.DECAY_SCALAR_INPUT, q_scale=K ** -0.5, n_requests=len(ctx.segments),
-            input_weight=gates[:, H:2 * H], ones=True, work=_runs_work(ctx, H, K, V + 1))
+            input_weight=gates[:, H:2 * H], ones=True, **_runs(ctx, H, K, V + 1))
         gated = ctx.buffer("mlstm.gated", (rows, H * V))
         kernels.memory_out_norm(o, gates[:, 2 * H:], proj[:, self.col_g:self.col_i],
                                 self.norm_weight, gated, H, V, self.eps, self.floor)

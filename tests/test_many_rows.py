@@ -43,22 +43,24 @@ def test_gemm_float32(M, N, K, pad, accumulate):
 
 
 def test_runs_cover_the_rows_and_fit_their_work():
-    for rows in (1, 100, 192, 193, 1000, 2048, 8191):
-        for n in (1, 2, 7, 40):
-            for H, K, V in ((4, 128, 256), (32, 128, 64), (1, 30, 7), (16, 250, 33)):
-                parts, run = recurrence_runs(rows, n, H, K, V)
-                floats = recurrence_work_floats(rows, n, H, K, V)
-                if parts == 1:
-                    assert floats == 0
-                else:
-                    assert parts * run >= rows and (parts - 1) * run < rows and run % 16 == 0
-                    assert floats == n * parts * H * (V + 1) * K and floats < 2 ** 27
+    for rows in (1, 100, 255, 256, 383, 384, 1000, 1023, 1024, 2048, 8191):
+        for H, K, V in ((4, 128, 256), (32, 128, 64), (1, 30, 7), (16, 250, 33), (16, 128, 256), (128, 128, 64)):
+            parts, run = recurrence_runs(rows, H, K, V)
+            floats = recurrence_work_floats([rows, 1, 1], H, K, V)
+            if parts == 1:
+                assert floats == 0
+            else:
+                assert parts * run >= rows and (parts - 1) * run < rows and run % 16 == 0 and parts <= 32
+                assert floats == parts * H * (V + 1) * K and floats < 2 ** 27
+                assert recurrence_work_floats([rows, rows, 3], H, K, V) == 2 * floats
+    assert recurrence_runs(2048, 128, 128, 64) == (1, 0) and recurrence_runs(300, 4, 128, 256)[0] > 1
 
 
 @gpu
-@pytest.mark.parametrize("H,G,K,V,lengths", [(2, 1, 128, 64, [2048]), (4, 4, 128, 256, [193]), (3, 3, 30, 7, [500, 3, 1, 290]),
+@pytest.mark.parametrize("H,G,K,V,lengths", [(2, 1, 128, 64, [2048]), (4, 4, 128, 256, [257]), (3, 3, 30, 7, [500, 3, 1, 290]),
                                              (2, 2, 72, 20, [96, 480]), (1, 1, 256, 16, [320, 64]),
-                                             (2, 1, 200, 40, [288, 111])])
+                                             (2, 1, 200, 40, [288, 111]),
+                                             (1, 1, 8, 4, [1, 260] + [1] * 40 + [2, 511, 256, 255] + [3] * 30 + [777])])
 @pytest.mark.parametrize("kind", (0, 1, 2, 3))
 def test_recurrence_in_runs(kind, H, G, K, V, lengths):
     """Long portions in runs against the formula in float64 and against the whole walk, states that
@@ -67,7 +69,7 @@ def test_recurrence_in_runs(kind, H, G, K, V, lengths):
     if kind in (0, 1) and G != H:
         G = H
     rows, n_slots = sum(lengths), len(lengths) + 2
-    assert recurrence_runs(rows, len(lengths), H, K, V)[0] > 1
+    assert recurrence_runs(max(lengths), H, K, V)[0] > 1
     slots = list(range(n_slots - 1, n_slots - 1 - len(lengths), -1))
     row_slot = torch.tensor(sum(([s] * n for s, n in zip(slots, lengths)), []), dtype=torch.int32, device=DEV)
     seg = torch.empty(n_slots, 3, dtype=torch.int32, device=DEV)
@@ -87,10 +89,10 @@ def test_recurrence_in_runs(kind, H, G, K, V, lengths):
         out = torch.full((rows, H * V), float("nan"), device=DEV)
         kernels.linear_recurrence(q, k, v, d, state, out, row_slot, seg, H, G, K, V, kind, q_scale=0.5, exponent=0.25,
                                   rate_log=p0, step_bias=p1, n_requests=len(lengths), input_weight=d2, ones=kind == 3,
-                                  work=work)
+                                  work=work, portions=lengths)
         return state, out
 
-    work = torch.full((recurrence_work_floats(rows, len(lengths), H, K, V),), float("nan"), device=DEV)
+    work = torch.full((recurrence_work_floats(lengths, H, K, V),), float("nan"), device=DEV)
     state, out = go(work)
     state_w, out_w = go(None)
     S = start[:, :H * V * K].double().view(n_slots, H, V, K).clone()
@@ -124,6 +126,44 @@ def test_recurrence_in_runs(kind, H, G, K, V, lengths):
     assert err(got, S) <= 1.2 * err(whole, S) + 2 ** -22
     assert torch.equal(state[:, H * V * K:], start[:, H * V * K:])
     assert torch.equal(state[:2], start[:2])                  # slots without rows
+
+
+@gpu
+@pytest.mark.parametrize("H,K,V,lengths", [(4, 128, 256, [600, 1, 1, 255, 3, 256]), (32, 128, 64, [1, 2, 500, 384, 383]),
+                                           (16, 128, 256, [1, 1100]), (3, 30, 7, [300, 1, 256])])
+@pytest.mark.parametrize("kind", (0, 2))
+def test_a_request_gives_the_same_bits_alone_and_in_company(kind, H, K, V, lengths):
+    """Whether a portion goes in runs, and where it is cut, is its own: decoded tokens and short portions
+    beside long ones, and long ones beside others, give the bits that they give alone."""
+    from llmario_b200 import kernels
+    rows = sum(lengths)
+    q, k, v = rnd(rows, H * K, seed=1), rnd(rows, H * K, seed=2, scale=0.3), rnd(rows, H * V, seed=3)
+    d = torch.sigmoid(rnd(rows, H * K, seed=4) + 4) if kind == 0 else rnd(rows, H, seed=4)
+    p0, p1 = rnd(H, seed=6) - 2, rnd(H, seed=7)
+    start = rnd(len(lengths), H * V * K, seed=8)
+
+    def go(which):
+        at = [sum(lengths[:i]) for i in range(len(lengths))]
+        pick = sum((list(range(at[i], at[i] + lengths[i])) for i in which), [])
+        mine = [lengths[i] for i in which]
+        row_slot = torch.tensor(sum(([i] * lengths[i] for i in which), []), dtype=torch.int32, device=DEV)
+        seg = None
+        if any(n > 1 for n in mine):
+            seg = torch.empty(len(lengths), 3, dtype=torch.int32, device=DEV)
+            kernels.segment_table(row_slot, seg)
+        state, out = start.clone(), torch.full((len(pick), H * V), float("nan"), device=DEV)
+        work = torch.full((recurrence_work_floats(mine, H, K, V),), float("nan"), device=DEV)
+        kernels.linear_recurrence(q[pick], k[pick], v[pick], d[pick], state, out, row_slot, seg, H, H, K, V, kind,
+                                  q_scale=0.5, rate_log=p0, step_bias=p1, n_requests=len(which),
+                                  work=work if len(work) else None, portions=mine)
+        return state, out
+
+    state, out = go(range(len(lengths)))
+    for i, n in enumerate(lengths):
+        state_i, out_i = go([i])
+        at = sum(lengths[:i])
+        assert torch.equal(out_i, out[at:at + n]), (i, n)
+        assert torch.equal(state_i[i], state[i]), (i, n)
 
 
 @gpu
