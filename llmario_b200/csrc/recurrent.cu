@@ -23,6 +23,8 @@
 // single tokens can be recorded and replayed.
 #include "common.cuh"
 
+#include <limits.h>
+
 namespace {
 
 // The table has three integers per request slot s: (first row, row after the last) of the rows
@@ -82,7 +84,7 @@ struct ScanArgs {
   // `unit`: q and k of every head are divided by sqrt(sum of squares + unit_floor) first
   const float* beta; int beta_stride;
   int unit; float unit_floor;
-  int long_rows, least_run;              // requests with so many rows (0: none) are cut into runs (run_rows)
+  int whole_rows, least_run;             // requests with more rows are cut into runs (run_rows)
   int n_requests;
   float* part_state;                     // [run of the step][H][V][K]
   float* part_decay;                     // [run of the step][H][K] (one number with a scalar decay)
@@ -142,9 +144,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) linear_recurrence_kernel(const S
     slot = a.seg[SEG * blockIdx.x + 2];
     if (slot < 0) return;
     first = a.seg[SEG * slot], end = a.seg[SEG * slot + 1];
+    if (!DELTA && end - first > a.whole_rows) return;      // (it goes in runs)
   }
   if (a.tail_only) first = end - ((end - first) & 3);
-  if (end <= first || (a.long_rows > 0 && end - first >= a.long_rows)) return;     // (the latter in runs)
+  if (end <= first) return;
   const int K = a.K, V = a.V, g = h / (a.H / a.G);
   const int j0 = blockIdx.z * COLS;
   const int li = lane % L;
@@ -447,7 +450,7 @@ __device__ __forceinline__ LongRequest find_long(const ScanArgs& a, int index, i
   for (int base = 0; base < a.n_requests; base += 32) {
     int slot = base + lane < a.n_requests ? a.seg[SEG * (base + lane) + 2] : -1, first = 0, rows = 0;
     if (slot >= 0) first = a.seg[SEG * slot], rows = a.seg[SEG * slot + 1] - first;
-    const bool is_long = slot >= 0 && rows >= a.long_rows;
+    const bool is_long = slot >= 0 && rows > a.whole_rows;
     const unsigned longs = __ballot_sync(0xffffffffu, is_long);
     if (longs == 0) continue;
     const int length = run_rows(rows, a.least_run), runs = is_long ? (rows + length - 1) / length : 0;
@@ -1552,7 +1555,7 @@ LLM_EXPORT int llm_linear_recurrence(const float* q, int q_stride, const float* 
   a.seg = seg, a.row_slot = row_slot;
   a.single = single, a.H = H, a.G = G, a.K = K, a.V = V, a.kind = kind;
   a.beta = nullptr, a.beta_stride = 0, a.unit = 0, a.unit_floor = 0.f, a.tail_only = 0;
-  a.long_rows = n_long > 0 ? long_rows : 0, a.least_run = least_run, a.n_requests = n_requests, a.part_state = work;
+  a.whole_rows = n_long > 0 ? long_rows - 1 : INT_MAX, a.least_run = least_run, a.n_requests = n_requests, a.part_state = work;
   a.part_decay = n_long > 0 ? work + (size_t)n_runs * H * V * K : nullptr;
   int rc = 0;
   if (n_long <= 0 || n_long < n_requests) rc = run_scan(a, rows, n_requests, stream);
@@ -1591,7 +1594,7 @@ LLM_EXPORT int llm_delta_recurrence_grouped(const float* q, int q_stride, const 
   a.seg = seg, a.row_slot = row_slot;
   a.single = single, a.H = H, a.G = G, a.K = K, a.V = V, a.kind = kind;
   a.beta = beta, a.beta_stride = beta_stride, a.unit = unit ? 1 : 0, a.unit_floor = unit_floor, a.tail_only = 0;
-  a.long_rows = a.least_run = a.n_requests = 0, a.part_state = a.part_decay = nullptr;
+  a.whole_rows = INT_MAX, a.least_run = a.n_requests = 0, a.part_state = a.part_decay = nullptr;
   // Portions of prompts with 68 to 256 key channels go four tokens at a time: what a group needs
   // is prepared once per head in parallel over the tokens, the walk takes a group per round, and
   // the token-by-token kernel takes the rows that are left (fewer than four a request).
