@@ -437,3 +437,20 @@ def test_linear_takes_wider_operands_at_few_rows(rows):
     assert bool(((out[:rows, :96].double() - ref).abs() <= bound).all())
     assert not out[rows:].any() and not out[:, 96:].any()
     kernels.check_tc_status(torch.device(DEV))
+
+
+@gpu
+@pytest.mark.parametrize("T,N,K,splits", [(1, 16384, 512, 2), (8, 16388, 512, 2), (3, 1028, 1024, 4), (40, 4096, 512, 2),
+                                          (1300, 512, 512, 2)])
+def test_the_output_of_a_cut_product_is_cleared_first(T, N, K, splits):
+    """Few wide rows in pieces, many rows in turn, columns that are not whole pieces; nothing beside the
+    output is touched."""
+    from llmario_b200 import kernels
+    a, w = rnd(T, K, dtype=torch.bfloat16, seed=1), rnd(N, K, dtype=torch.bfloat16, seed=2)
+    wide = torch.full((T, N + 8), 7.0, device=DEV)
+    kernels.gemm_tcgen05(a, w, wide[:, :N], 0, splits=splits, bn=64)
+    ref = a.double() @ w.double().T
+    bound = (K + 10) * 2 ** -23 * (a.abs().double() @ w.abs().double().T)
+    assert bool(((wide[:, :N].double() - ref).abs() <= bound).all())
+    assert bool((wide[:, N:] == 7.0).all())
+    kernels.check_tc_status(torch.device(DEV))
