@@ -30,7 +30,7 @@
 #include "tcgen05.cuh"
 
 int llm_zero_f32(float* p, int rows, int cols, int ld, cudaStream_t stream);   // elementwise.cu
-int llm_pair_store_way(int T, int N, int K, int splits);                       // gemm_tcgen05_pair.cu
+extern "C" int llm_pair_store_way(int T, int N, int K, int splits);            // gemm_tcgen05_pair.cu
 int llm_gemm_tcgen05_pair(const void* X, const void* W, void* C, int c_dtype, int T, int N, int K, int lda,
                           int ldw, int ldc, int mode, int half, float limit, int ranges, int* status, cudaStream_t stream);
 int llm_gemm_tcgen05_persistent(const void* X, const void* W, void* C, int c_dtype, int T, int N, int K,

@@ -31,7 +31,8 @@
 // turn) meets it before tensor memory is freed.  No load is multicast.
 #include "tcgen05.cuh"
 
-extern int g_llm_pair_ksplits;
+int g_llm_pair = 1;           // 0: the dispatcher keeps to the one-CTA kernels (for comparisons)
+int g_llm_pair_ksplits = 0;   // > 0: this many ranges of K in the adding epilogue (for measurements)
 
 namespace {
 
@@ -485,26 +486,65 @@ int cheapest_cut(int m_tiles, int T, int nkb, int pairs) {
   return ksplits;
 }
 
+int pair_sm_count() {
+  static int sm_count = 0;
+  if (!sm_count) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
+    if (sm_count <= 0) sm_count = 148;
+  }
+  return sm_count;
+}
+
+template <int STAGES, int EPI, typename TC, int FORM>
+constexpr int pair_smem() {
+  return (int)sizeof(PairStorage<STAGES, gated_epilogue(EPI) ? 64 : TILE_M, TC, FORM == GROUPED_TILES>) + 1024;
+}
+
+// As many pairs as the device holds at once (an SM without a free neighbour stays empty), at most one
+// per two SMs; negative: a CUDA error, 0: no pair of this kernel fits.
+template <int STAGES, int EPI, typename TC, int FORM>
+int resident_pairs() {
+  static int pairs = 0;
+  if (pairs) return pairs;
+  auto kernel = gemm_pair_kernel<STAGES, EPI, TC, FORM>;
+  constexpr int smem = pair_smem<STAGES, EPI, TC, FORM>();
+  static_assert(smem <= 227 * 1024, "the stages and output chunks fit one SM");
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return -(int)e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(192);
+  cfg.gridDim = dim3(pair_sm_count() & ~1);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  return pairs = n < pair_sm_count() / 2 ? n : pair_sm_count() / 2;
+}
+
 template <int STAGES, int EPI, typename TC, int FORM>
 int launch_form(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mxs, const CUtensorMap& mc, int T, int N,
-           int K, int half, int sm_count, int* status, cudaStream_t stream, float act_limit = 0.f,
+           int K, int half, int* status, cudaStream_t stream, float act_limit = 0.f,
            const Grouping& grouping = Grouping(), int ranges = 0) {
   constexpr bool GATED = gated_epilogue(EPI), GROUPED = FORM == GROUPED_TILES;
   constexpr int FEAT = GATED ? 64 : TILE_M;
   auto kernel = gemm_pair_kernel<STAGES, EPI, TC, FORM>;
-  constexpr int smem = (int)sizeof(PairStorage<STAGES, FEAT, TC, GROUPED>) + 1024;
-  static_assert(smem <= 227 * 1024, "the stages and output chunks fit one SM");
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  const int most = resident_pairs<STAGES, EPI, TC, FORM>();
+  if (most <= 0) return most < 0 ? -most : LLM_ERR_UNSUPPORTED;
   const int limit = GATED ? half : N;
   const int m_tiles = (limit + 2 * FEAT - 1) / (2 * FEAT), n_tiles = GROUPED ? grouping.n_small : (T + BN - 1) / BN;
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(192);
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = pair_smem<STAGES, EPI, TC, FORM>();
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -514,26 +554,14 @@ int launch_form(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap&
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  // as many pairs as the device holds at once (an SM without a free neighbour stays empty)
-  static int resident_pairs = 0;
-  if (!resident_pairs) {
-    cfg.gridDim = dim3(sm_count & ~1);
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
-      (void)cudaGetLastError();
-      return LLM_ERR_UNSUPPORTED;
-    }
-    resident_pairs = n < sm_count / 2 ? n : sm_count / 2;
-  }
   int ksplits = 1;
   if (EPI == EPI_ACCUM) {
     const int nkb = (K + TILE_K - 1) / TILE_K;
-    ksplits = ranges > 0 ? ranges : cheapest_cut(m_tiles, T, nkb, resident_pairs);
+    ksplits = ranges > 0 ? ranges : cheapest_cut(m_tiles, T, nkb, most);
     if (g_llm_pair_ksplits > 0 && nkb / g_llm_pair_ksplits >= 1) ksplits = g_llm_pair_ksplits;
   }
   const int works = m_tiles * n_tiles * ksplits;
-  const int pairs = works < resident_pairs ? works : resident_pairs;
+  const int pairs = works < most ? works : most;
   cfg.gridDim = dim3(2 * pairs);
   // directly behind the rotation kernel the pair kernel starts only when that kernel is done
   cfg.numAttrs = (g_llm_pdl && !g_llm_after_rotation) ? 2 : 1;
@@ -544,15 +572,15 @@ int launch_form(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap&
 
 template <int STAGES, int EPI, typename TC>
 int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mxs, const CUtensorMap& mc, int T, int N,
-           int K, int half, int sm_count, int* status, cudaStream_t stream, float act_limit = 0.f, int ranges = 0) {
+           int K, int half, int* status, cudaStream_t stream, float act_limit = 0.f, int ranges = 0) {
   Grouping g = Grouping();
   g.k_up = ranges > 0;
   if (short_tail(T)) {
     g.in_order = tail_in_order(N, K);
-    return launch_form<STAGES, EPI, TC, LAST_TOKENS>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream, act_limit, g,
+    return launch_form<STAGES, EPI, TC, LAST_TOKENS>(mw, mx, mxs, mc, T, N, K, half, status, stream, act_limit, g,
                                                      ranges);
   }
-  return launch_form<STAGES, EPI, TC, WHOLE_TILES>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream, act_limit, g,
+  return launch_form<STAGES, EPI, TC, WHOLE_TILES>(mw, mx, mxs, mc, T, N, K, half, status, stream, act_limit, g,
                                                    ranges);
 }
 }  // namespace
@@ -569,8 +597,10 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mxs,
 // (rows x N x K) 39.6 -> 27.4 us (ranges of K), 777 x 4,096 x 1,024 29.7 -> 20.5 (two sums; one sum 19.5,
 // two ranges added in memory 26.6), 1,501 x 4,096 x 4,096 70.5 -> 57.3 (two ranges; one sum 56.3, two sums
 // 61.5); 513 x 1,024 x 1,024 stays on lone CTAs (15.4 against 18.4 on pairs).
-int llm_pair_store_way(int T, int N, int K, int splits) {
-  const int pairs = 74, nkb = (K + TILE_K - 1) / TILE_K;
+LLM_EXPORT int llm_pair_store_way(int T, int N, int K, int splits) {
+  const int pairs = g_llm_pair ? resident_pairs<5, EPI_STORE, float, WHOLE_TILES>() : 0;
+  if (pairs <= 0) return 2;
+  const int nkb = (K + TILE_K - 1) / TILE_K;
   const int m_tiles = (N + 2 * TILE_M - 1) / (2 * TILE_M);
   const double clear = (2.5 + (double)T * N * 4 / 3e6) / 0.39;
   // (two sums leave no accumulator for the next tile: every round but the last waits for its epilogue)
@@ -579,7 +609,7 @@ int llm_pair_store_way(int T, int N, int K, int splits) {
   const int s = splits == 2 ? 2 : cheapest_cut(m_tiles, T, nkb, pairs);
   const double cut = s == 1 ? 1e30 : rounds_cost(N, K, T, pairs, s);
   const long long lone = (long long)((N + TILE_M - 1) / TILE_M) * ((T + 127) / 128) * splits;
-  const double alone = (double)((lone + 4 * pairs - 1) / (4 * pairs)) * (1.4 * nkb / splits + 6.0) + clear;
+  const double alone = (double)((lone + 2 * pair_sm_count() - 1) / (2 * pair_sm_count())) * (1.4 * nkb / splits + 6.0) + clear;
   if (alone < whole && alone < cut + clear) return 2;
   return cut + clear < whole ? 1 : 0;
 }
@@ -588,50 +618,37 @@ int llm_pair_store_way(int T, int N, int K, int splits) {
 // split but in mode 1, in `ranges` ranges or, for 0, as many as are soonest, and in mode 0 with 32-bit C
 // as two sums for ranges = 2; the gated form only with interleaved rows).  Returns LLM_ERR_UNSUPPORTED when the output
 // cannot be written by TMA or the mode is not one of these: the caller then uses the one-CTA kernel.
-int g_llm_pair = 1;   // 0: the dispatcher keeps to the one-CTA kernels (for comparisons)
-int g_llm_pair_ksplits = 0;   // > 0: this many ranges of K in the adding epilogue (for measurements)
 LLM_EXPORT void llm_set_pair_ksplits(int n) { g_llm_pair_ksplits = n; }
 LLM_EXPORT void llm_set_pair(int on) { g_llm_pair = on ? 1 : 0; }
-
-static int pair_sm_count() {
-  static int sm_count = 0;
-  if (!sm_count) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-    if (sm_count <= 0) sm_count = 148;
-  }
-  return sm_count;
-}
 
 int llm_gemm_tcgen05_pair(const void* X, const void* W, void* C, int c_dtype, int T, int N, int K, int lda,
                           int ldw, int ldc, int mode, int half, float limit, int ranges, int* status, cudaStream_t stream) {
   if (!g_llm_pair) return LLM_ERR_UNSUPPORTED;
-  const int sm_count = pair_sm_count();
   if (mode != 0 && mode != 1 && mode != 3 && mode != 4) return LLM_ERR_UNSUPPORTED;
   const int esize = c_dtype == LLM_F32 ? 4 : 2;
   if (((uintptr_t)C & 15) || ((size_t)ldc * esize) % 16) return LLM_ERR_UNSUPPORTED;
   CUtensorMap mw, mx, mxs, mc;
   if (!llm_tensor_map(W, N, K, ldw, TILE_M, TILE_K, 0, &mw)) return LLM_ERR_UNSUPPORTED;
   if (!llm_tensor_map(X, T, K, lda, HALF_N, TILE_K, 0, &mx)) return LLM_ERR_UNSUPPORTED;
-  if (!llm_tensor_map(X, T, K, lda, HALF_N / 2, TILE_K, 0, &mxs)) return LLM_ERR_UNSUPPORTED;
+  mxs = mx;      // (read for narrow last tokens alone)
+  if (short_tail(T) && !llm_tensor_map(X, T, K, lda, HALF_N / 2, TILE_K, 0, &mxs)) return LLM_ERR_UNSUPPORTED;
   const int out_cols = mode >= 3 ? half : N;
   if (!llm_tensor_map(C, T, out_cols, ldc, CH, mode >= 3 ? 64 : TILE_M, c_dtype == LLM_F32 ? 2 : 1, &mc))
     return LLM_ERR_UNSUPPORTED;
   if (mode == 0) {
     if (c_dtype == LLM_F32 && ranges == 2)
-      return launch<5, EPI_TWO_SUMS, float>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream);
-    if (c_dtype == LLM_F32) return launch<5, EPI_STORE, float>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream);
-    if (c_dtype == LLM_BF16) return launch<6, EPI_STORE, bf16>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream);
+      return launch<5, EPI_TWO_SUMS, float>(mw, mx, mxs, mc, T, N, K, half, status, stream);
+    if (c_dtype == LLM_F32) return launch<5, EPI_STORE, float>(mw, mx, mxs, mc, T, N, K, half, status, stream);
+    if (c_dtype == LLM_BF16) return launch<6, EPI_STORE, bf16>(mw, mx, mxs, mc, T, N, K, half, status, stream);
   } else if (mode == 1) {
-    if (c_dtype == LLM_F32) return launch<5, EPI_ACCUM, float>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream, 0.f, ranges);
+    if (c_dtype == LLM_F32) return launch<5, EPI_ACCUM, float>(mw, mx, mxs, mc, T, N, K, half, status, stream, 0.f, ranges);
   } else {
     if (N != 2 * half || half % 16) return LLM_ERR_ARGUMENT;
     if (mode == 4)
-      return c_dtype == LLM_BF16 ? launch<6, EPI_CLAMPED, bf16>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream, limit)
+      return c_dtype == LLM_BF16 ? launch<6, EPI_CLAMPED, bf16>(mw, mx, mxs, mc, T, N, K, half, status, stream, limit)
                                  : LLM_ERR_UNSUPPORTED;
-    if (c_dtype == LLM_BF16) return launch<6, EPI_GATED, bf16>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream);
-    if (c_dtype == LLM_F32) return launch<6, EPI_GATED, float>(mw, mx, mxs, mc, T, N, K, half, sm_count, status, stream);
+    if (c_dtype == LLM_BF16) return launch<6, EPI_GATED, bf16>(mw, mx, mxs, mc, T, N, K, half, status, stream);
+    if (c_dtype == LLM_F32) return launch<6, EPI_GATED, float>(mw, mx, mxs, mc, T, N, K, half, status, stream);
   }
   return LLM_ERR_UNSUPPORTED;
 }
@@ -661,9 +678,8 @@ LLM_EXPORT int llm_gemm_tcgen05_grouped_pair(const void* X, const void* W, void*
   if (!llm_tensor_map(X, T, K, lda, HALF_N / 2, TILE_K, 0, &mxs)) return LLM_ERR_UNSUPPORTED;
   if (!llm_tensor_map(C, T, gated ? half : N, ldc, CH, gated ? 64 : TILE_M, c_dtype == LLM_F32 ? 2 : 1, &mc))
     return LLM_ERR_UNSUPPORTED;
-  const int sms = pair_sm_count();
-  if (mode == 0) return launch_form<5, EPI_STORE, float, GROUPED_TILES>(mw, mx, mxs, mc, T, N, K, half, sms, status, stream, 0.f, g);
-  if (mode == 3) return launch_form<6, EPI_GATED, bf16, GROUPED_TILES>(mw, mx, mxs, mc, T, N, K, half, sms, status, stream, 0.f, g);
-  if (mode == 4) return launch_form<6, EPI_CLAMPED, bf16, GROUPED_TILES>(mw, mx, mxs, mc, T, N, K, half, sms, status, stream, limit, g);
-  return launch_form<6, EPI_RELU2, bf16, GROUPED_TILES>(mw, mx, mxs, mc, T, N, K, half, sms, status, stream, 0.f, g);
+  if (mode == 0) return launch_form<5, EPI_STORE, float, GROUPED_TILES>(mw, mx, mxs, mc, T, N, K, half, status, stream, 0.f, g);
+  if (mode == 3) return launch_form<6, EPI_GATED, bf16, GROUPED_TILES>(mw, mx, mxs, mc, T, N, K, half, status, stream, 0.f, g);
+  if (mode == 4) return launch_form<6, EPI_CLAMPED, bf16, GROUPED_TILES>(mw, mx, mxs, mc, T, N, K, half, status, stream, limit, g);
+  return launch_form<6, EPI_RELU2, bf16, GROUPED_TILES>(mw, mx, mxs, mc, T, N, K, half, status, stream, 0.f, g);
 }

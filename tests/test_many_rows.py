@@ -454,3 +454,18 @@ def test_the_output_of_a_cut_product_is_cleared_first(T, N, K, splits):
     assert bool(((wide[:, :N].double() - ref).abs() <= bound).all())
     assert bool((wide[:, N:] == 7.0).all())
     kernels.check_tc_status(torch.device(DEV))
+
+
+@gpu
+def test_the_choice_of_pairs_knows_when_they_are_off():
+    """A product of many rows is not prepared for CTA pairs that will not run: its output is then
+    cleared only where the lone CTAs add into it."""
+    from llmario_b200 import kernels
+    way = kernels.lib().llm_pair_store_way
+    sizes = [(777, 4096, 1024, 2), (2048, 1024, 3072, 5), (1501, 4096, 4096, 2), (513, 1024, 1024, 4)]
+    assert [way(*s) for s in sizes] == [0, 1, 1, 2]
+    kernels.use_cta_pairs(False)
+    try:
+        assert [way(*s) for s in sizes] == [2] * 4
+    finally:
+        kernels.use_cta_pairs(True)
