@@ -527,6 +527,23 @@ __global__ void __launch_bounds__(WARPS * 32) attention_outside_kernel(
 }
 }  // namespace
 
+// Prompts in 32-bit: blocks of consecutive tokens by tiles, the rest by the kernel of one warp
+// per (row, head), which leaves those out: two launches.  Both find the blocks on the device, from
+// row_slot and row_pos, so no list of items is needed; a caller that knows that every row is a request of
+// its own (`single`) gets the second kernel alone, and so do steps of fewer than 16 rows (16 rows of
+// one prompt: 19 us row by row, 23 by tiles; 64: 43 and 28).  `more`: a sink, kept first keys or pooled
+// blocks.
+LLM_EXPORT int llm_attention_generic_launches(const void* q, const void* out, const void* k_cache, const void* v_cache,
+                                              int dtype, long long page_stride, int rows, int Hq, int Hkv, int hd, int vd,
+                                              int more, int single) {
+  const int group = Hkv > 0 ? Hq / Hkv : 0;
+  const bool tiled = dtype == LLM_F32 && !single && !more && (vd <= 0 || vd == hd) && (hd == 64 || hd == 128) &&
+                     (group == 1 || group == 2 || group == 4 || group == 8) && rows >= 16 && Hkv <= 65535 &&
+                     page_stride % 8 == 0 && (((uintptr_t)k_cache | (uintptr_t)v_cache) & 31) == 0 &&
+                     (((uintptr_t)q | (uintptr_t)out) & 15) == 0;
+  return tiled ? 2 : 1;
+}
+
 static int attention_generic(const void* q, void* out, const void* k_cache, const void* v_cache, int dtype,
                              long long page_stride, const int* block_table, int table_stride, const int* row_slot,
                              const int* row_pos, int rows, int Hq, int Hkv, int hd, int page_size, float scale,
@@ -547,15 +564,9 @@ static int attention_generic(const void* q, void* out, const void* k_cache, cons
                     ((p_page_stride % 8) == 0 && (((uintptr_t)pk_cache | (uintptr_t)pv_cache) & 31) == 0));
   const long long items = (long long)rows * Hq;
   const int blocks = (int)((items + WARPS - 1) / WARPS);
-  // Prompts in 32-bit: blocks of consecutive tokens by tiles, the rest by the kernel of one warp
-  // per (row, head), which leaves those out.  Both find the blocks on the device, from row_slot and
-  // row_pos, so no list of items is needed; a caller that knows that every row is a request of its
-  // own (`single`) gets the second kernel alone, and so do steps of fewer than 16 rows (16 rows of
-  // one prompt: 19 us row by row, 23 by tiles; 64: 43 and 28).
   const int group = Hq / Hkv;
-  if (dtype == LLM_F32 && vec && !single && vd == hd && (hd == 64 || hd == 128) && !sink && keep_first == 0 &&
-      pk_cache == nullptr && (group == 1 || group == 2 || group == 4 || group == 8) && rows >= 16 && Hkv <= 65535 &&
-      (((uintptr_t)q | (uintptr_t)out) & 15) == 0) {
+  if (llm_attention_generic_launches(q, out, k_cache, v_cache, dtype, page_stride, rows, Hq, Hkv, hd, vd,
+                                     sink || keep_first || pk_cache, single) == 2) {
     int rc = LLM_ERR_UNSUPPORTED;
 #define TILED(D, G)                                                                                              \
   do {                                                                                                           \

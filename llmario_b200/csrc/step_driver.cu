@@ -61,6 +61,8 @@ int llm_attention_generic(const void* q, void* out, const void* k_cache, const v
                           const int* row_slot, const int* row_pos, int rows, int Hq, int Hkv, int hd,
                           int page_size, float scale, int window, const float* sink, int vd,
                           cudaStream_t stream);
+int llm_attention_generic_launches(const void* q, const void* out, const void* k_cache, const void* v_cache, int dtype,
+                          long long page_stride, int rows, int Hq, int Hkv, int hd, int vd, int more, int single);
 int llm_attention_generic_single(const void* q, void* out, const void* k_cache, const void* v_cache, int dtype,
                           long long page_stride, const int* block_table, int table_stride,
                           const int* row_slot, const int* row_pos, int rows, int Hq, int Hkv, int hd,
@@ -643,11 +645,15 @@ struct Run {
                                              c.page_size, L.scale, window, L.sink, L.value_dim, L.keep_first,
                                              L.pool > 0 ? L.pool_k : nullptr, L.pool_v, L.pool_page_stride,
                                              L.pool_table, L.pool_table_stride, L.pool, stream), K_GENERIC);
-    if (plain || (L.sink != nullptr && !tc))
+    if (plain || (L.sink != nullptr && !tc)) {
+      const int n = llm_attention_generic_launches(q, out, c.k, c.v, st.dtype, c.page_stride, st.rows, Hq, Hkv, hd,
+                                                   L.value_dim, L.sink != nullptr, st.all_single);
+      launches += n - 1, g_counts[K_GENERIC] += n - 1;
       return check((st.all_single ? llm_attention_generic_single : llm_attention_generic)(
                        q, out, c.k, c.v, st.dtype, c.page_stride, c.block_table, c.table_stride, st.row_slot,
                        st.row_pos, st.rows, Hq, Hkv, hd, c.page_size, L.scale, window, L.sink, L.value_dim, stream),
                    K_GENERIC);
+    }
     const float* sink = L.sink;
     float *extra_o = nullptr, *extra_ml = nullptr;
     if (outside) {

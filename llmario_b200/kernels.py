@@ -54,6 +54,7 @@ def _signatures():
                                    I, F, I, I, I, P],
         "llm_rope_table": [P, P, P, I, I, F, P],
         "llm_attention_generic": [P, P, P, P, I, L, P, I, P, P, I, I, I, I, I, F, I, P, I, P],
+        "llm_attention_generic_launches": [P, P, P, P, I, L, I, I, I, I, I, I, I],
         "llm_attention_generic_ext": [P, P, P, P, I, L, P, I, P, P, I, I, I, I, I, F, I, P, I, I, P,
                                       P, L, P, I, I, P],
         "llm_attention_latent_ok": [I, I, I],
@@ -383,6 +384,10 @@ def attention_generic(q: torch.Tensor, out: torch.Tensor, k_cache: torch.Tensor,
         head_dim, page_size, float(scale), int(window or 0), _ptr(sink), int(value_dim),
         _stream()),
         f"attention (head_dim {head_dim})")
+    global launches
+    launches += lib().llm_attention_generic_launches(
+        _ptr(q), _ptr(out), _ptr(k_cache), _ptr(v_cache), _dt(q), page_stride, rows, num_heads,
+        num_kv_heads, head_dim, int(value_dim), int(sink is not None), 0) - 1
 
 
 def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor,

@@ -469,3 +469,33 @@ def test_the_choice_of_pairs_knows_when_they_are_off():
         assert [way(*s) for s in sizes] == [2] * 4
     finally:
         kernels.use_cta_pairs(True)
+
+
+@gpu
+def test_launches_of_the_generic_attention_are_counted():
+    """A prompt in 32-bit takes two kernels per layer, as many decoded tokens one, and the counts say so."""
+    from llmario_b200 import Model, ModelRunner, StepEntry, driver, kernels
+    from llmario_b200.config import Qwen3Config
+    from llmario_b200.weights import random_tensors
+    cfg = Qwen3Config.from_dict(dict(
+        architectures=["Qwen3ForCausalLM"], model_type="qwen3", max_position_embeddings=512, num_hidden_layers=3,
+        hidden_size=64, num_attention_heads=4, num_key_value_heads=2, head_dim=64, intermediate_size=128,
+        vocab_size=256, rope_theta=10000.0, rms_norm_eps=1e-6, tie_word_embeddings=True, torch_dtype="float32"))
+    spec = cfg.to_spec()
+    model = Model(spec, random_tensors(spec, 1, torch.float32, DEV), torch.float32, DEV)
+    runner = ModelRunner(model, page_size=16, n_pages=64, max_requests=20, max_context=64, use_graphs=False)
+
+    def counted(entries):
+        runner.step(entries)
+        torch.cuda.synchronize()
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            was, generic = kernels.launches, driver.kernel_counts()["generic"]
+            runner.step(entries)
+            torch.cuda.synchronize()
+            said = kernels.launches - was, driver.kernel_counts()["generic"] - generic
+        names = [e.name for e in prof.events() if "attention" in e.name]
+        return said[1], len(names)
+
+    assert counted([StepEntry("a", list(range(24)), [23])]) == (6, 6)
+    entries = [StepEntry(i, [i + 1], [0]) for i in range(17)]
+    assert counted(entries) == (3, 3)
