@@ -147,3 +147,39 @@ def test_host_time_of_a_mixed_step():
     assert times[True] * 2 <= times[False], times
     print(f"host time of a mixed step: python {times[False] * 1e3:.2f} ms, "
           f"native {times[True] * 1e3:.2f} ms")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", (1, 2, 3, 4))
+def test_few_rows_through_the_row_product(rows):
+    """A decode step of one to four rows with the products for few rows and small matrices (the norms
+    made inside them) and without: the kernels are the ones asked for, the logits agree within what
+    16-bit activations show between two correct orders of their sums."""
+    from llmario_b200 import Model, ModelRunner, StepEntry, driver, kernels
+    from llmario_b200.config import Qwen3Config
+    from llmario_b200.weights import random_tensors
+    layers = 3
+    spec = Qwen3Config.from_dict(dict(
+        architectures=["Qwen3ForCausalLM"], model_type="qwen3", max_position_embeddings=512, num_hidden_layers=layers,
+        hidden_size=1024, num_attention_heads=4, num_key_value_heads=2, head_dim=128, intermediate_size=768,
+        vocab_size=512, rope_theta=10000.0, rms_norm_eps=1e-6, tie_word_embeddings=True,
+        torch_dtype="bfloat16")).to_spec()
+    model = Model(spec, random_tensors(spec, 1, torch.bfloat16, "cuda:0"), torch.bfloat16, "cuda:0")
+    switch = kernels.lib().llm_set_row_product
+    got = {}
+    for most in (4, 0):
+        runner = ModelRunner(model, page_size=16, n_pages=64, max_requests=8, max_context=128, use_graphs=False)
+        for i in range(rows):
+            runner.step([StepEntry(i, [(7 * i + j) % 512 for j in range(20 + 3 * i)], [])])
+        switch(most)
+        try:
+            before = driver.kernel_counts()
+            got[most] = runner.step([StepEntry(i, [100 + i], [0]) for i in range(rows)]).double().cpu()
+            ran = {k: v - before[k] for k, v in driver.kernel_counts().items()}
+        finally:
+            switch(4)
+        # q/k/v with its norm, the output projection, gate and up with their norm, the way down
+        assert ran["row_product"] == (4 * layers if most else 0)
+        assert ran["norm"] == (0 if most else 2 * layers)
+    kernels.check_tc_status(torch.device("cuda:0"))
+    assert float((got[4] - got[0]).norm() / got[0].norm()) < 1e-2
