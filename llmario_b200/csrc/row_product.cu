@@ -12,17 +12,23 @@
 // that every warp keeps in registers, so that no barrier follows), the dot products from shared
 // memory, five shuffles and a store: 2.6 to 4.5 us with the norm inside, a decode step of one request
 // (28 layers of Qwen3-0.6B sizes) 935 -> 698 us.  No atomics: an output is one warp's sum.
-// Limits: K 1,024 or 2,048, or 3,072 for one row, so that the rows fit a warp's registers beside a
-// second CTA, and slices of at most 100 KB, so that the slices of two kernels of the chain fit an SM
-// and the next one's copies overlap this one's work.  What has more values of h (up to four rows of
-// up to 4,096) keeps them in shared memory, a warp per row making them, behind one barrier: a step of
-// three or four requests (14 layers) 507 -> 478 us.  With room for eight rows the dot products took
-// longer than the chain saved (six or eight requests: 511 -> 631 us), so those stay on tcgen05.
+// Limits: K up to 3,072 for one row and up to 2,048 for two, so that the rows fit a warp's registers
+// beside a second CTA, and slices of at most 100 KB, so that the slices of two kernels of the chain fit
+// an SM and the next one's copies overlap this one's work.  All else, up to four rows of up to 4,096,
+// keeps h in shared memory, a warp per row making it, behind one barrier: a step of three or four
+// requests (14 layers) 507 -> 478 us.  So does the norm of two rows, which every warp would make for
+// both.  Links of a chain K -> K, in shared memory -> in registers, K 512 / 1,024 / 1,536 / 2,048 / 2,560: one
+// row's norm 2.9 / 3.5 / 5.0 / 5.8 / 8.2 -> 2.3 / 2.9 / 3.7 / 4.3 / 5.7 us, one row 1.9 / 2.5 / 4.5 / 5.0 / 7.2
+// -> 1.3 / 1.6 / 2.5 / 3.0 / 4.0, two rows' norm 2.8 / 3.2 / 4.8 / 5.3 / 8.3 -> 3.0 / 3.8 / 5.5 / 9.1 / -, two rows
+// - / 2.5 / - / 4.9 / - -> - / 1.9 / - / 3.4 / -.  With room for eight rows the dot products took longer than the
+// chain saved (six or eight requests: 511 -> 631 us), so those stay on tcgen05.
 #include "common.cuh"
 
 namespace {
 constexpr int RP_WARPS = 8, RP_ROWS = 4;       // warps; weight rows a warp multiplies at a time
-constexpr int RP_SLICE = 100 * 1024, RP_SHARED = 112 * 1024;
+// most bytes of a slice; of a slice and h, so that two CTAs fit an SM (two rows of up to 2,048: 16 KB beside
+// any slice)
+constexpr int RP_SLICE = 100 * 1024, RP_SHARED = 112 * 1024, RP_SHARED_2 = RP_SLICE + 16 * 1024;
 constexpr int RP_MAX = 4;                      // rows
 enum RowMode : int { ROW_STORE = 0, ROW_ADD = 1, ROW_GATED = 2 };
 
@@ -355,8 +361,11 @@ template <int KC, int R>
 int rp_mode(const void* x, int ldx, const float* norm_w, float eps, const void* W, void* out, int ldc, int N, int per,
             int mode, int* status, cudaStream_t stream) {
 #define RP(M)                                                                                                       \
-  return norm_w ? rp_launch<KC, R, M, true>(x, ldx, norm_w, eps, W, out, ldc, N, per, status, stream)               \
-                : rp_launch<KC, R, M, false>(x, ldx, norm_w, eps, W, out, ldc, N, per, status, stream)
+  do {                                                                                                              \
+    if (!norm_w) return rp_launch<KC, R, M, false>(x, ldx, norm_w, eps, W, out, ldc, N, per, status, stream);       \
+    if constexpr (R == 1) return rp_launch<KC, R, M, true>(x, ldx, norm_w, eps, W, out, ldc, N, per, status, stream); \
+    return LLM_ERR_UNSUPPORTED;                                                                                     \
+  } while (0)
   if (mode == ROW_STORE) RP(ROW_STORE);
   if (mode == ROW_ADD) RP(ROW_ADD);
   RP(ROW_GATED);
@@ -366,7 +375,7 @@ int rp_shared(const void* x, int ldx, const float* norm_w, float eps, const void
               int K, int per, int mode, int* status, cudaStream_t stream) {
   const int smem = (RP_MAX * K + per * (mode == ROW_GATED ? 2 : 1) * K) * 2;
   auto go = [&](auto kernel) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RP_SHARED);
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RP_SHARED_2);
     if (e != cudaSuccess) return (int)e;
     return launch_pdl(kernel, (N + per - 1) / per, RP_WARPS * 32, smem, stream, x, ldx, norm_w, eps, (const bf16*)W, out,
                       ldc, rows, N, K, per, status);
@@ -376,18 +385,18 @@ int rp_shared(const void* x, int ldx, const float* norm_w, float eps, const void
   return norm_w ? go(row_product_shared_kernel<ROW_GATED, true>) : go(row_product_shared_kernel<ROW_GATED, false>);
 }
 
-// whether the rows fit a warp's registers
-bool rp_in_registers(int rows, int K) { return rows <= 2 && (K == 1024 || K == 2048 || (K == 3072 && rows == 1)); }
+// whether the rows go to a warp's registers
+bool rp_in_registers(int rows, int K, bool norm) { return (rows == 1 && K <= 3072) || (rows == 2 && K <= 2048 && !norm); }
 }  // namespace
 
-// Whether llm_row_product takes these sizes: rows x K values of h in registers, N (gated: features)
-// outputs whose weights fit the SMs' slices.
+// Whether llm_row_product takes these sizes: rows x K values of h in registers or in shared memory, N
+// (gated: features) outputs whose weights fit the SMs' slices.
 LLM_EXPORT int llm_row_product_ok(int rows, int N, int K, int gated) {
   if (rows < 1 || rows > RP_MAX || N < 1 || K < 256 || K > 4096 || K % 256) return 0;
   const int per = (N + rp_sm_count() - 1) / rp_sm_count();
   const long long slice = (long long)per * (gated ? 2 : 1) * K * 2;
-  if (rp_in_registers(rows, K)) return slice <= RP_SLICE;
-  return slice <= RP_SLICE && slice + RP_MAX * K * 2 <= RP_SHARED;
+  if (slice > RP_SLICE) return 0;
+  return rp_in_registers(rows, K, false) || slice + RP_MAX * K * 2 <= RP_SHARED;
 }
 
 // mode 0: out f32 = h W^T; 1: out f32 += h W^T; 2: out bf16 = silu(gate) * up, W interleaved, N features
@@ -400,16 +409,17 @@ LLM_EXPORT int llm_row_product(const void* x, int ldx, const float* norm_w, floa
   if (!llm_row_product_ok(rows, N, K, mode == ROW_GATED) || (mode == ROW_GATED && N % 16)) return LLM_ERR_UNSUPPORTED;
   if ((((uintptr_t)x | (uintptr_t)W | (uintptr_t)norm_w) & 15) || ldx % (norm_w ? 4 : 8)) return LLM_ERR_UNSUPPORTED;
   const int per = (N + rp_sm_count() - 1) / rp_sm_count();
-  if (!rp_in_registers(rows, K))
+  if (!rp_in_registers(rows, K, norm_w != nullptr))
     return rp_shared(x, ldx, norm_w, eps, W, out, ldc, rows, N, K, per, mode, status, stream);
 #define RP_GO(KC, R) return rp_mode<KC, R>(x, ldx, norm_w, eps, W, out, ldc, N, per, mode, status, stream)
+#define RP_ROWS_1(KC) case KC * 8 + 1: RP_GO(KC, 1);
+#define RP_ROWS_2(KC) case KC * 8 + 1: RP_GO(KC, 1); case KC * 8 + 2: RP_GO(KC, 2);
   switch (K / 256 * 8 + rows) {
-    case 4 * 8 + 1: RP_GO(4, 1);
-    case 4 * 8 + 2: RP_GO(4, 2);
-    case 8 * 8 + 1: RP_GO(8, 1);
-    case 8 * 8 + 2: RP_GO(8, 2);
-    case 12 * 8 + 1: RP_GO(12, 1);
+    RP_ROWS_2(1) RP_ROWS_2(2) RP_ROWS_2(3) RP_ROWS_2(4) RP_ROWS_2(5) RP_ROWS_2(6) RP_ROWS_2(7) RP_ROWS_2(8)
+    RP_ROWS_1(9) RP_ROWS_1(10) RP_ROWS_1(11) RP_ROWS_1(12)
   }
+#undef RP_ROWS_1
+#undef RP_ROWS_2
 #undef RP_GO
   return LLM_ERR_UNSUPPORTED;
 }

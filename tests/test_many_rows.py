@@ -344,12 +344,15 @@ def test_grouped_products_on_cta_pairs(counts, N, K, bn):
 @gpu
 @pytest.mark.parametrize("rows", (1, 2, 3, 4))
 @pytest.mark.parametrize("N,K", [(1024, 2048), (4096, 1024), (1024, 3072), (148, 1024), (7, 2048), (3056, 1024), (640, 256),
-                                 (96, 4096)])
+                                 (96, 4096), (200, 768), (1000, 1536), (300, 2304), (3600, 2048)])
 def test_row_product(rows, N, K):
     """One to four rows through a small matrix (held in registers or in shared memory): stored, added,
     gated, of 16-bit rows and of the norm of 32-bit rows; fewer outputs than SMs, slices that do not
     come out even, strided rows."""
     from llmario_b200 import kernels
+    if (N, K) == (3600, 2048) and rows > 2:      # (slices of 100 KB: no room for more rows beside them)
+        assert not kernels.row_product_ok(rows, N, K)
+        return
     assert kernels.row_product_ok(rows, N, K)
     x = rnd(rows, K + 8, seed=1)[:, :K]
     h = rnd(rows, K + 8, dtype=torch.bfloat16, seed=2)[:, :K]
