@@ -448,10 +448,14 @@ __global__ void __launch_bounds__(192, 1) gemm_pair_kernel(
 }
 
 // The last tokens of a T that is not a multiple of 256 make shorter items where they are at most half a
-// tile and there are fewer than four whole ones: beyond that the padding saved is less than what the
-// variant with a width read at run time loses.  Four layers of Qwen3-8B widths, padded -> narrow, 520 /
-// 600 / 800 tokens: 1,231 / 1,252 / 1,625 -> 1,183 / 1,187 / 1,543 us; 1,100 / 2,100: 1,849 / 3,022 -> 1,858 /
-// 3,044; 1,500 / 3,000 (220 and 184 left over): 2,161 / 4,133 -> 2,230 / 4,238.
+// tile and there are fewer than four whole ones.  A pair's time for a tile falls with its tokens only
+// where the box of tokens does too (up to 128: see load_w), and the variant with a width read at run time
+// loses about 1 % on the whole tiles, which four or more of them make more than the padding.  The four
+// products of a layer, padded -> narrow, us: Qwen3-0.6B widths 600 / 840 tokens 60 -> 58 / 67 -> 64, 4B 163 ->
+// 156 / 194 -> 192, 8B 220 -> 218 / 322 -> 321 (its matrices of 100 and 200 MB follow their tiles, see below:
+// 780 tokens 311 -> 317, 896 329 -> 324).  Tried wider: with 129 to 255 tokens left 0.6B widths 641 / 720 / 900 /
+// 1,020 tokens 563 / 566 / 648 / 661 -> 597 / 580 / 634 / 667 (twelve layers), beyond four tiles 1,280 and
+// 2,060 789 / 908 -> 790 / 911: nothing.
 bool short_tail(int T) { return T < 4 * BN && T % BN != 0 && T % BN <= BN / 2; }
 // Dealt last, the short items even out the pairs, but they meet every weight a second time: fine
 // while the weights stay in the L2 (some 48 MB), else they follow their tiles (600 tokens 1,199 ->
