@@ -20,7 +20,7 @@ import sys
 from typing import Any, Dict, List
 
 from .pemolorn import _View, pemolorn_config
-from .vunasun import SIZES, _rates, _time
+from .vunasun import SIZES, _rates, _time, runs_of
 
 
 def pavatar_config(preset: Dict[str, Any], layers: int, vocab: int = 32768):
@@ -154,13 +154,13 @@ def kernel_table(width: int = 4096, tokens: int = 2048, batch: int = 64, heads: 
         state.zero_()
         us = _time(lambda: kernels.linear_recurrence(
             q, k, v, step, state, o, row_slot, seg, H, G, K, V, kernels.DECAY_RATE_STEP,
-            rate_log=rate, step_bias=bias, n_requests=live), flush=flush)
+            rate_log=rate, step_bias=bias, n_requests=live, **runs_of(rows, single, H, K, V)), flush=flush)
         rec(f"linear recurrence, a decay per head, the state-space mixer's ({label})", us,
             io + rows * H * 4, flops=4.0 * cells)
         state.zero_()
         us = _time(lambda: kernels.linear_recurrence(
             q, k, v, decay, state, o, row_slot, seg, H, G, K, V, kernels.DECAY_VECTOR,
-            q_scale=K ** -0.5, n_requests=live), flush=flush)
+            q_scale=K ** -0.5, n_requests=live, **runs_of(rows, single, H, K, V)), flush=flush)
         rec(f"linear recurrence, a decay per key channel, gated linear attention's ({label})", us,
             io + rows * H * K * 4, flops=4.0 * cells)
         # ---- the decay per key channel from the projected step

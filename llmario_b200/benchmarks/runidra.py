@@ -18,7 +18,7 @@ import json
 import sys
 from typing import Any, Dict, List
 
-from .vunasun import SIZES, _rates, _time
+from .vunasun import SIZES, _rates, _time, prompt_note, runs_of
 
 
 def runidra_config(preset: Dict[str, Any], layers: int, vocab: int = 32768, window: int = 1024):
@@ -130,10 +130,10 @@ def kernel_table(width: int = 4096, tokens: int = 2048, batch: int = 64, heads: 
         us = _time(lambda: kernels.linear_recurrence(
             proj[:, :H * K], proj[:, H * K:2 * H * K], proj[:, 2 * H * K:2 * H * K + H * V], gates[:, :H],
             state, o, row_slot, seg, H, H, K, V + 1, kernels.DECAY_SCALAR_INPUT, q_scale=K ** -0.5,
-            n_requests=1, input_weight=gates[:, H:2 * H], ones=True), flush=flush)
+            n_requests=1, input_weight=gates[:, H:2 * H], ones=True, **runs_of(rows, single, H, K, V + 1)), flush=flush)
         moved = rows * (2 * H * K + 2 * H * V) * 4 + 2 * live * H * (V + 1) * K * 4
         rec(f"linear_recurrence, matrix memory ({label})", us, moved,
-            note="a prompt is one request: its tokens are walked in order" if not single else "")
+            note="" if single else prompt_note(rows, H, K, V + 1))
         gated = torch.empty(rows, H * V, dtype=torch.bfloat16, device=dev)
         wv = f32(H * V)
         us = _time(lambda: kernels.memory_out_norm(o, gates[:, 2 * H:], proj[:, 2 * H * K + H * V:ci], wv, gated,

@@ -125,6 +125,23 @@ def compare(sizes: List[str], layers: int, batch: int = 8, prompt_len: int = 102
 
 
 # ---------------------------------------------------------------------------------------------
+def runs_of(rows: int, single: bool, heads: int, key_dim: int, value_dim: int) -> Dict[str, Any]:
+    """The arguments with which the recurrence cuts one prompt into runs, as the model has it do."""
+    import torch
+
+    from .. import kernels
+    floats = 0 if single else kernels.recurrence_work_floats([rows], heads, key_dim, value_dim)
+    return dict(work=torch.empty(floats, dtype=torch.float32, device="cuda:0"),
+                portions=[rows]) if floats else {}
+
+
+def prompt_note(rows: int, heads: int, key_dim: int, value_dim: int) -> str:
+    from .. import kernels
+    parts, length = kernels.recurrence_runs(rows, heads, key_dim, value_dim)
+    return "one request, its tokens walked in order" if parts == 1 else \
+        f"one request in {parts} runs of {length} tokens: folded, then walked at the same time"
+
+
 def _time(fn, reps: int = 20, flush=None) -> float:
     """Median microseconds of ``fn`` timed with CUDA events, the L2 flushed before every run."""
     import torch
@@ -186,11 +203,12 @@ def kernel_table(width: int = 4096, tokens: int = 2048, batch: int = 64) -> List
         o = torch.empty(rows, H * V, dtype=torch.float32, device=dev)
         us = _time(lambda: kernels.linear_recurrence(
             proj[:, :H * K], proj[:, H * K:2 * H * K], proj[:, 2 * H * K:2 * H * K + H * V], z, state, o,
-            row_slot, seg, H, H, K, V, kernels.DECAY_VECTOR, q_scale=K ** -0.5, n_requests=1), flush=flush)
+            row_slot, seg, H, H, K, V, kernels.DECAY_VECTOR, q_scale=K ** -0.5, n_requests=1,
+            **runs_of(rows, single, H, K, V)), flush=flush)
         live = rows if single else 1
         moved = rows * (3 * H * K + 2 * H * V) * 4 + 2 * live * H * V * K * 4
         rec(f"linear_recurrence gla ({label})", us, moved,
-            "a prompt is one request: its tokens are walked in order" if not single else "")
+            "" if single else prompt_note(rows, H, K, V))
         gated = torch.empty(rows, H * V, dtype=torch.bfloat16, device=dev)
         w = f32(V)
         us = _time(lambda: kernels.gated_group_norm(o, proj[:, 2 * H * K + H * V:2 * H * K + 2 * H * V], w, gated,
@@ -210,10 +228,10 @@ def kernel_table(width: int = 4096, tokens: int = 2048, batch: int = 64) -> List
         a_log, dtb = f32(H2) * 0.1, f32(H2) * 0.1
         us = _time(lambda: kernels.linear_recurrence(
             xbc[:, inner + N:], xbc[:, inner:inner + N], xbc[:, :inner], proj2[:, 2 * inner + 2 * N:], st2, o2,
-            row_slot, seg, H2, G, N, P, kernels.DECAY_RATE_STEP, rate_log=a_log, step_bias=dtb, n_requests=1),
-            flush=flush)
+            row_slot, seg, H2, G, N, P, kernels.DECAY_RATE_STEP, rate_log=a_log, step_bias=dtb, n_requests=1,
+            **runs_of(rows, single, H2, N, P)), flush=flush)
         moved = rows * (2 * N + 2 * inner + H2) * 4 + 2 * live * H2 * P * N * 4
-        rec(f"linear_recurrence mamba2 ({label})", us, moved)
+        rec(f"linear_recurrence mamba2 ({label})", us, moved, "" if single else prompt_note(rows, H2, N, P))
         g2 = torch.empty(rows, inner, dtype=torch.bfloat16, device=dev)
         w2, skip = f32(inner), f32(H2)
         us = _time(lambda: kernels.gated_group_norm(o2, proj2[:, :inner], w2, g2, inner, 1e-6, True, skip=skip,

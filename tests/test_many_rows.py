@@ -121,9 +121,9 @@ def test_recurrence_in_runs(kind, H, G, K, V, lengths):
     err = lambda x, y: float((x.double() - y).norm() / y.norm())  # noqa: E731
     e_out, e_whole = err(out, ref.view(rows, -1)), err(out_w, ref.view(rows, -1))
     got, whole = (t[:, :H * V * K].reshape(S.shape) for t in (state, state_w))
-    # 32-bit sums: the runs may not be further off than the whole walk by more than a rounding
-    assert e_out <= 1.2 * e_whole + 2 ** -22 and e_out < 1e-5
-    assert err(got, S) <= 1.2 * err(whole, S) + 2 ** -22
+    # A state gets one rounding more per run (the carry's) among those of hundreds of tokens: the runs are
+    # no further off than the whole walk, but for a quarter of a rounding in the norm
+    assert e_out <= e_whole + 2 ** -26 and err(got, S) <= err(whole, S) + 2 ** -26 and e_out < 1e-6
     assert torch.equal(state[:, H * V * K:], start[:, H * V * K:])
     assert torch.equal(state[:2], start[:2])                  # slots without rows
 
@@ -502,3 +502,85 @@ def test_launches_of_the_generic_attention_are_counted():
     assert counted([StepEntry("a", list(range(24)), [23])]) == (6, 6)
     entries = [StepEntry(i, [i + 1], [0]) for i in range(17)]
     assert counted(entries) == (3, 3)
+
+
+@gpu
+@pytest.mark.parametrize("activation,weight_on,identity,shared", [
+    ("silu", "output", 0, False), ("silu", "output", 2, True), ("clamped_swish", "input", 0, False),
+    ("clamped_swish", "output", 0, True), ("relu_squared", "output", 0, False)])
+@pytest.mark.parametrize("rows,E,top,width,ff", [(520, 8, 2, 264, 272), (700, 5, 1, 128, 80), (1501, 4, 3, 64, 144)])
+def test_routed_experts_of_many_rows(rows, E, top, width, ff, activation, weight_on, identity, shared):
+    """The whole feed-forward with enough tokens per expert for the products on CTA pairs: the bits of
+    the one-CTA products (one expert nearly without tokens, one with many), and the formula in float64."""
+    from llmario_b200 import kernels
+    from llmario_b200.config.spec import PartSpec
+    from llmario_b200.parts.base import Segment, StepContext, Workspace, build_part
+    assert kernels.moe_pairs(rows * top, E)
+    b16 = lambda *s, seed: rnd(*s, dtype=torch.bfloat16, scale=s[-1] ** -0.5, seed=seed)  # noqa: E731
+    gated = activation != "relu_squared"
+    w = {"r": rnd(E + identity, width, scale=2 * width ** -0.5, seed=1)}
+    names = {"router": ["r"]}
+    for e in range(E):
+        for k, shape in ((("gate", (ff, width)),) if gated else ()) + (("up", (ff, width)), ("down", (width, ff))):
+            w[f"{k}{e}"] = b16(*shape, seed=10 * e + len(k))
+            names[f"{k}{e}"] = [f"{k}{e}"]
+    bias = torch.zeros(E + identity, device=DEV)
+    bias[0], bias[1] = -3.0, 2.0
+    w["b"], names["router_bias"] = bias, ["b"]
+    params = dict(hidden_size=width, intermediate_size=ff, experts=E, top=top, identity=identity, activation=activation,
+                  weight_on=weight_on, limit=0.7, scores="softmax_all" if identity else "softmax_chosen", tensors=names)
+    if shared:
+        for k, shape in (("gate", (32, width)), ("up", (32, width)), ("down", (width, 32))):
+            w["s" + k] = b16(*shape, seed=99 + len(k))
+        params["shared"] = PartSpec("swiglu", dict(hidden_size=width, intermediate_size=32,
+                                                   tensors={k: ["s" + k] for k in ("gate", "up", "down")}))
+    part = build_part("feed_forward", PartSpec("moe", params), w, torch.bfloat16, DEV)
+    h = rnd(rows, width, dtype=torch.bfloat16, seed=3)
+    x0 = rnd(rows, width, seed=4)
+    ints = torch.zeros(rows, dtype=torch.int32, device=DEV)
+
+    def forward():
+        ctx = StepContext(rows=rows, tokens=ints, row_pos=ints, row_slot=ints, segments=[Segment("r", 0, 0, rows, 0)],
+                          dtype=torch.bfloat16, device=torch.device(DEV), workspace=Workspace(torch.device(DEV)),
+                          cache=None)
+        x = x0.clone()
+        part.forward(ctx, h, x)
+        return x, ctx.buffer("moe.ids", (rows, top), torch.int32).clone(), \
+            ctx.buffer("moe.weights", (rows, top), torch.float32).clone()
+
+    got, ids, wts = forward()
+    kernels.use_cta_pairs(False)
+    try:
+        lone, _, _ = forward()
+    finally:
+        kernels.use_cta_pairs(True)
+    assert torch.equal(got, lone)
+    kernels.check_tc_status(torch.device(DEV))
+    hd, want = h.double(), x0.double()
+    r16 = lambda t: t.to(torch.bfloat16).double()  # noqa: E731
+
+    def act(z, e, s=1.0):
+        up = z @ w[f"up{e}"].double().T * s
+        if not gated:
+            return r16(up.clamp(min=0) ** 2)
+        g = z @ w[f"gate{e}"].double().T * s
+        if activation == "silu":
+            return r16(g * torch.sigmoid(g) * up)
+        g, up = g.clamp(max=0.7), up.clamp(-0.7, 0.7)
+        return r16(g * torch.sigmoid(1.702 * g) * (up + 1))
+
+    for k in range(top):
+        for e in range(E + identity):
+            at = (ids[:, k] == e).nonzero()[:, 0]
+            f = wts[at, k].double()[:, None]
+            if e >= E:
+                want[at] += f * hd[at]
+            elif weight_on == "input":
+                want[at] += act(hd[at], e, f) @ w[f"down{e}"].double().T
+            else:
+                want[at] += f * (act(hd[at], e) @ w[f"down{e}"].double().T)
+    if shared:
+        g = hd @ w["sgate"].double().T
+        want += r16(g * torch.sigmoid(g) * (hd @ w["sup"].double().T)) @ w["sdown"].double().T
+    # activations are rounded to 8 bits of mantissa on both sides: a rounding may fall the other way
+    assert float((got.double() - want).norm() / (want - x0.double()).norm()) < 2 ** -9

@@ -410,6 +410,27 @@ def test_mixed_batches_and_reused_slots(name, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("name", ("mix", "experts"))
+def test_a_request_alone_and_in_company_gives_the_same_bits(name):
+    """Long portions (which recurrences walk in runs), a short one and a decoded token in one step, each
+    against the same request in a step of its own, in 32-bit."""
+    parts = {"a": (tokens_for(name, 301, 1), 1), "b": (tokens_for(name, 23, 2), 22), "c": (tokens_for(name, 420, 3), 17),
+             "d": (tokens_for(name, 41, 4), 1)}      # (tokens, how many of them come in an earlier step)
+
+    def go(which):
+        runner = runner_for(name, "float32", page_size=16, cache_tokens=1024, max_requests=4)
+        for r in which:
+            run_steps(runner, [[(r, parts[r][0][:parts[r][1]], [])]])
+        return run_steps(runner, [[(r, parts[r][0][n:], range(len(parts[r][0]) - n))
+                                   for r, n in ((r, parts[r][1]) for r in which)]])
+
+    together = go("abcd")
+    for r in parts:
+        alone = go(r)[r]
+        assert all(np.array_equal(alone[p], together[r][p]) for p in alone) and len(alone)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("name", ("latent_tc", "mix", "experts", "experts_tc"))
 def test_a_long_prompt_over_many_windows_and_the_engine_page(name, dtype):
