@@ -85,7 +85,7 @@ struct ScanArgs {
   const float* beta; int beta_stride;
   int unit; float unit_floor;
   int whole_rows, least_run;             // requests with more rows are cut into runs (run_rows)
-  int n_requests;
+  int n_requests, n_runs;                // requests of the step; runs that there is room for
   float* part_state;                     // [run of the step][H][V][K]
   float* part_decay;                     // [run of the step][H][K] (one number with a scalar decay)
   int tail_only;        // only the last (rows of the request) % 4 rows: the others went in groups of four
@@ -713,7 +713,7 @@ __global__ void __launch_bounds__(256) scan_carry_kernel(const ScanArgs a, int p
   const LongRequest request = find_long<true>(a, blockIdx.y, threadIdx.x & 31);
   const int slot = request.slot, length = run_rows(request.rows, a.least_run);
   if (slot < 0) return;
-  const int runs = (request.rows + length - 1) / length;
+  const int runs = min((request.rows + length - 1) / length, a.n_runs - request.run0);
   const long long size = (long long)a.H * a.V * a.K;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= size) return;
@@ -1555,7 +1555,8 @@ LLM_EXPORT int llm_linear_recurrence(const float* q, int q_stride, const float* 
   a.seg = seg, a.row_slot = row_slot;
   a.single = single, a.H = H, a.G = G, a.K = K, a.V = V, a.kind = kind;
   a.beta = nullptr, a.beta_stride = 0, a.unit = 0, a.unit_floor = 0.f, a.tail_only = 0;
-  a.whole_rows = n_long > 0 ? long_rows - 1 : INT_MAX, a.least_run = least_run, a.n_requests = n_requests, a.part_state = work;
+  a.whole_rows = n_long > 0 ? long_rows - 1 : INT_MAX, a.least_run = least_run, a.n_requests = n_requests, a.n_runs = n_runs;
+  a.part_state = work;
   a.part_decay = n_long > 0 ? work + (size_t)n_runs * H * V * K : nullptr;
   int rc = 0;
   if (n_long <= 0 || n_long < n_requests) rc = run_scan(a, rows, n_requests, stream);
@@ -1594,7 +1595,7 @@ LLM_EXPORT int llm_delta_recurrence_grouped(const float* q, int q_stride, const 
   a.seg = seg, a.row_slot = row_slot;
   a.single = single, a.H = H, a.G = G, a.K = K, a.V = V, a.kind = kind;
   a.beta = beta, a.beta_stride = beta_stride, a.unit = unit ? 1 : 0, a.unit_floor = unit_floor, a.tail_only = 0;
-  a.whole_rows = INT_MAX, a.least_run = a.n_requests = 0, a.part_state = a.part_decay = nullptr;
+  a.whole_rows = INT_MAX, a.least_run = a.n_requests = a.n_runs = 0, a.part_state = a.part_decay = nullptr;
   // Portions of prompts with 68 to 256 key channels go four tokens at a time: what a group needs
   // is prepared once per head in parallel over the tokens, the walk takes a group per round, and
   // the token-by-token kernel takes the rows that are left (fewer than four a request).
