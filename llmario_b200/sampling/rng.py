@@ -79,6 +79,5 @@ def next_uniforms(streams: Sequence[Optional[Xoshiro256StarStar]], out: int) -> 
     where = array("Q", at)
     _native().llm_rng_uniforms(where.buffer_info()[0], len(at), out)
     if 0 in at:
-        for i, r in enumerate(streams):
-            if r is not None and not at[i]:
-                ctypes.c_double.from_address(out + 8 * i).value = r.next_f64()
+        for i in [i for i, a in enumerate(at) if not a and streams[i] is not None]:
+            ctypes.c_double.from_address(out + 8 * i).value = streams[i].next_f64()

@@ -111,12 +111,18 @@ class DeviceSampler:
             # draw may be prepared while the copy for the one before it is still queued)
             self._host = [torch.empty(c * 10, dtype=torch.float32, pin_memory=True)
                           for _ in range(2)]
+            self._host_np = [h.numpy() for h in self._host]
             self._host_key = [None, None]
             self._host_event = [None, None]
             self._dev = torch.empty(c * 10, dtype=torch.float32, device=self.device)
             self._dev_key = None
+            d = self._dev      # (its parts are taken once: a draw of few rows is host time)
+            self._options = (d[0:c], d[6 * c:7 * c].view(torch.int32), d[c:2 * c], d[2 * c:3 * c],
+                             d[8 * c:10 * c].view(torch.float64))
+            self._penalties = (d[3 * c:4 * c], d[4 * c:5 * c], d[5 * c:6 * c])
             # [status words | tokens]: one copy brings both to the host
             self._out = torch.zeros(STATUS_WORDS + c, dtype=torch.int32, device=self.device)
+            self._out_parts = (self._out[STATUS_WORDS:], self._out[:STATUS_WORDS])
             # two host copies in turn: a draw may be launched before the one before it is read
             self._out_host = [torch.empty(STATUS_WORDS + c, dtype=torch.int32, pin_memory=True)
                               for _ in range(2)]
@@ -150,16 +156,22 @@ class DeviceSampler:
         still running and this row's input is the token it draws."""
         rows = logits.shape[0]
         assert rows == len(samplers) and logits.dtype == torch.float32 and rows > 0
+        params = [s.params for s in samplers]
         tri: List[int] = []
-        src: List[int] = [-1] * rows
-        for r, s in enumerate(samplers):
-            if s.params.penalties_active:
-                unknown = inflight is not None and inflight[r] >= 0
-                if unknown:
-                    src[r] = int(inflight[r])
-                for tok, cnt in (s.counts_before_unknown() if unknown else s.counts).items():
-                    tri += (r, tok, cnt)
-        any_unknown = any(x >= 0 for x in src)
+        src: List[int] = []
+        any_unknown = False
+        # (the plain attributes first: a property costs a call, for every row of every draw)
+        for r in [r for r, p in enumerate(params)
+                  if (p.repeat_penalty != 1.0 or p.frequency_penalty != 0.0
+                      or p.presence_penalty != 0.0) and p.penalties_active]:
+            s = samplers[r]
+            unknown = inflight is not None and inflight[r] >= 0
+            if unknown:
+                src = src or [-1] * rows
+                src[r] = int(inflight[r])
+                any_unknown = True
+            for tok, cnt in (s.counts_before_unknown() if unknown else s.counts).items():
+                tri += (r, tok, cnt)
         # (the tokens of the draw before, taken before the buffers may be replaced by larger ones)
         drawn = self.device_tokens if any_unknown else None
         self._buffers(rows, len(tri) // 3 + (rows if any_unknown else 0))
@@ -167,17 +179,16 @@ class DeviceSampler:
         # the options of a row change only when the set of requests changes; the uniforms
         # change with every draw (greedy rows draw nothing)
         key = [s.serial for s in samplers]
-        any_draw = any(not s.params.greedy for s in samplers)
+        any_draw = any(not p.greedy for p in params)
         if key != self._dev_key or any_draw:
             i = self._flip
             if self._host_event[i] is not None:
                 self._host_event[i].synchronize()
-            h = self._host[i].numpy()
+            h = self._host_np[i]
             if key != self._host_key[i]:
                 f = h[:6 * c].reshape(6, c)
                 k = h[6 * c:7 * c].view(np.int32)
-                for r, s in enumerate(samplers):
-                    p = s.params
+                for r, p in enumerate(params):
                     f[0, r], f[1, r], f[2, r] = p.temperature, p.top_p, p.min_p
                     f[3, r], f[4, r], f[5, r] = (p.repeat_penalty, p.frequency_penalty,
                                                  p.presence_penalty)
@@ -185,7 +196,7 @@ class DeviceSampler:
                 self._host_key[i] = key
             # (greedy rows do not advance their streams; samplers with a next_uniform of their own
             # are asked)
-            streams = [None if s.params.greedy else s.rng for s in samplers]
+            streams = [None if p.temperature <= 0.0 else s.rng for p, s in zip(params, samplers)]
             own = [r for r, s in enumerate(samplers)
                    if type(s) is not RequestSampler or "next_uniform" in s.__dict__]
             for r in own:
@@ -198,7 +209,6 @@ class DeviceSampler:
             self._host_event[i] = torch.cuda.Event()
             self._host_event[i].record()
             self._dev_key = key
-        d = self._dev
         if tri or any_unknown:
             n = len(tri) // 3
             # the rows' sources of tokens in flight travel behind the triples
@@ -210,13 +220,10 @@ class DeviceSampler:
             self.h2d_bytes += 4 * len(words)
             self._tri_event = torch.cuda.Event()
             self._tri_event.record()
-            kernels.apply_penalties(logits, self._tri_dev, n, d[3 * c:4 * c], d[4 * c:5 * c],
-                                    d[5 * c:6 * c],
+            kernels.apply_penalties(logits, self._tri_dev, n, *self._penalties,
                                     self._tri_dev[3 * n:3 * n + rows] if any_unknown else None,
                                     drawn)
-        kernels.sample(logits, d[0:c], d[6 * c:7 * c].view(torch.int32), d[c:2 * c],
-                       d[2 * c:3 * c], d[8 * c:10 * c].view(torch.float64),
-                       self._out[STATUS_WORDS:], self._out[:STATUS_WORDS])
+        kernels.sample(logits, *self._options, *self._out_parts)
         host = self._out_host[self._flip]
         self._flip ^= 1
         n = STATUS_WORDS + rows
