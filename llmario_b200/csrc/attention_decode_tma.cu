@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(32, 4) flash_decode_tma_kernel(
     float* __restrict__ part_o, float* __restrict__ part_ml, const int* __restrict__ block_table,
     int table_stride, const int* __restrict__ items, const int* __restrict__ row_slot,
     const int* __restrict__ row_pos, int Hq, int Hkv, int page_size, int n_slots, int slot,
-    float scale_log2, int window, int splits, int* __restrict__ status, const Fused fu) {
+    float scale_log2, int window, int splits, int* __restrict__ status, const Fused fu, int beside) {
   constexpr int KS = HD / 16, MT = KT / 16, DM = HD / 16;
   constexpr int TILE_BYTES = KT * HD * 2;            // one K or V tile
   extern __shared__ uint8_t raw[];
@@ -123,7 +123,11 @@ __global__ void __launch_bounds__(32, 4) flash_decode_tma_kernel(
   int early = 0;          // tiles asked for before the wait: those wholly below the new positions
   for (; early < STAGES && tb0 + early < tb1 && (tb0 + early + 1) * KT <= it.pos_start; ++early)
     load_tile(tb0 + early, early);
-  pdl_wait();
+  // beside: the kernel ahead is the prompt attention of the same step, which writes nothing that is
+  // read here and lets this kernel start only when its own wait is over, so that everything before it
+  // is complete.  This kernel then runs beside it and waits for its end at its own end instead: what
+  // comes next may rely on both.
+  if (!beside) pdl_wait();
   for (int i = early; i < STAGES && tb0 + i < tb1; ++i) load_tile(tb0 + i, i);
 
   int cpos[2], clo[2];
@@ -392,6 +396,7 @@ __global__ void __launch_bounds__(32, 4) flash_decode_tma_kernel(
   }
   if (!alive) {   // let the loads that are still in flight land before the shared memory goes
     for (int i = 0; i < STAGES; ++i) mbar_wait(&full[i], 0), mbar_wait(&full[i], 1);
+    if (beside) pdl_wait();
     return;
   }
 
@@ -425,6 +430,7 @@ __global__ void __launch_bounds__(32, 4) flash_decode_tma_kernel(
       }
     }
   }
+  if (beside) pdl_wait();
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -772,7 +778,7 @@ template <int HD, bool FUSED>
 int launch(const CUtensorMap& map, const bf16* q, bf16* out, float* part_o, float* part_ml, const int* table,
            int table_stride, const int* items, const int* row_slot, const int* row_pos, int n_items, int Hq,
            int Hkv, int page_size, int n_slots, int slot, float scale, int window, int splits, int* status,
-           const Fused& fu, cudaStream_t s) {
+           const Fused& fu, int beside, cudaStream_t s) {
   constexpr int KT = DECODE_KT, STAGES = DECODE_STAGES;
   auto kernel = flash_decode_tma_kernel<HD, KT, STAGES, FUSED>;
   constexpr int smem = 2 * STAGES * KT * HD * 2 + STAGES * 8 + 1024;
@@ -785,7 +791,7 @@ int launch(const CUtensorMap& map, const bf16* q, bf16* out, float* part_o, floa
   dim3 grid(n_items, Hkv, splits);
   return launch_pdl(kernel, grid, 32, smem, s, map, q, out, part_o, part_ml, table, table_stride, items,
                     row_slot, row_pos, Hq, Hkv, page_size, n_slots, slot, scale * 1.4426950408889634f, window,
-                    splits, status, fu);
+                    splits, status, fu, beside);
 }
 
 int check_and_map(const void* storage, long long n_pages, int n_slots, int slot, int Hq, int Hkv, int hd,
@@ -810,13 +816,13 @@ int check_and_map(const void* storage, long long n_pages, int n_slots, int slot,
 
 // storage: the group's whole cache [n_pages][n_slots][2][Hkv][page_size][hd] bfloat16, contiguous;
 // slot: the cache slot of this layer call.  page_size: a power of two.
-// Other arguments as llm_attention_decode.
-LLM_EXPORT int llm_attention_decode_tma(const void* q, void* out, float* part_o, float* part_ml,
-                                        const void* storage, long long n_pages, int n_slots, int slot,
-                                        const int* block_table, int table_stride, const int* items,
-                                        const int* row_slot, const int* row_pos, int n_items, int Hq,
-                                        int Hkv, int hd, int page_size, float scale, int window,
-                                        int splits, int* status, cudaStream_t stream) {
+// Other arguments as llm_attention_decode.  beside: the kernel launched before this one is
+// llm_attention_tcgen05 for other rows of the same step, and the two may run side by side.
+int llm_attention_decode_tma_beside(const void* q, void* out, float* part_o, float* part_ml, const void* storage,
+                                    long long n_pages, int n_slots, int slot, const int* block_table,
+                                    int table_stride, const int* items, const int* row_slot, const int* row_pos,
+                                    int n_items, int Hq, int Hkv, int hd, int page_size, float scale, int window,
+                                    int splits, int beside, int* status, cudaStream_t stream) {
   if (n_items <= 0) return 0;
   CUtensorMap map;
   if (int e = check_and_map(storage, n_pages, n_slots, slot, Hq, Hkv, hd, page_size, splits, part_o, part_ml, &map))
@@ -825,10 +831,21 @@ LLM_EXPORT int llm_attention_decode_tma(const void* q, void* out, float* part_o,
 #define GO(HD)                                                                                          \
   return launch<HD, false>(map, (const bf16*)q, (bf16*)out, part_o, part_ml, block_table, table_stride,  \
                            items, row_slot, row_pos, n_items, Hq, Hkv, page_size, (int)n_slots, slot, scale, \
-                           window, splits, status, none, stream)
+                           window, splits, status, none, beside, stream)
   if (hd == 128) GO(128);
   GO(64);
 #undef GO
+}
+
+LLM_EXPORT int llm_attention_decode_tma(const void* q, void* out, float* part_o, float* part_ml,
+                                        const void* storage, long long n_pages, int n_slots, int slot,
+                                        const int* block_table, int table_stride, const int* items,
+                                        const int* row_slot, const int* row_pos, int n_items, int Hq,
+                                        int Hkv, int hd, int page_size, float scale, int window,
+                                        int splits, int* status, cudaStream_t stream) {
+  return llm_attention_decode_tma_beside(q, out, part_o, part_ml, storage, n_pages, n_slots, slot, block_table,
+                                         table_stride, items, row_slot, row_pos, n_items, Hq, Hkv, hd, page_size,
+                                         scale, window, splits, 0, status, stream);
 }
 
 // The persistent form for steps of single new tokens (see flash_decode_persistent_kernel): rows
@@ -890,7 +907,7 @@ LLM_EXPORT int llm_attention_decode_fused(float* proj, int proj_stride, void* ou
 #define GO(HD)                                                                                          \
   return launch<HD, true>(map, nullptr, (bf16*)out, part_o, part_ml, block_table, table_stride, nullptr,  \
                           row_slot, row_pos, rows, Hq, Hkv, page_size, (int)n_slots, slot, scale, window,   \
-                          splits, status, fu, stream)
+                          splits, status, fu, 0, stream)
   if (hd == 128) GO(128);
   GO(64);
 #undef GO

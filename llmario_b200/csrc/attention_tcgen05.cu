@@ -110,14 +110,16 @@ __global__ void __launch_bounds__(320, 1) attention_tcgen05_kernel(
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
-  // only now may the next kernel of the stream be scheduled: every CTA of this one that is
-  // running holds its tensor memory, so a successor that also allocates some cannot starve it
-  pdl_trigger();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ the Q tile
     if (lane == 0) {
       pdl_wait();
+      // only now may the next kernel of the stream be scheduled.  Every CTA of this one that is
+      // running holds its tensor memory, so a successor that also allocates some cannot starve it;
+      // and whatever came before this kernel is complete, so that decode attention for other rows of
+      // the step may run beside it without a wait of its own (attention_decode_tma.cu).
+      pdl_trigger();
       mbar_expect_tx(&sm.q_full, ROWS * HD * 2);
 #pragma unroll
       for (int h = 0; h < HALVES; ++h)
@@ -551,13 +553,12 @@ __global__ void __launch_bounds__(320, 1) attention_tcgen05_persistent_kernel(
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sm.tmem_base;
-  pdl_trigger();          // after the allocation, as in the kernel above
-
 
   if (warp == 0) {
     // ------------------------------------------------------------------ loads
     if (lane == 0) {
       pdl_wait();
+      pdl_trigger();          // after the allocation and the wait, as in the kernel above
       const int R = page_size < KT ? page_size : KT;
       bool ok = true;
       uint32_t T = 0;           // key tiles asked for so far, over all work items

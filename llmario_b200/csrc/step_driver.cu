@@ -30,6 +30,11 @@
 #include "step_driver.h"
 
 // ---- the kernels' own entry points (defined in the other files of this library)
+int llm_attention_decode_tma_beside(const void* q, void* out, float* part_o, float* part_ml, const void* storage,
+                                    long long n_pages, int n_slots, int slot, const int* block_table,
+                                    int table_stride, const int* items, const int* row_slot, const int* row_pos,
+                                    int n_items, int Hq, int Hkv, int hd, int page_size, float scale, int window,
+                                    int splits, int beside, int* status, cudaStream_t stream);
 extern "C" {
 int llm_rms_norm(const float* x, const float* w, void* y, int out_dtype, const int* rows_index, int rows,
                  int width, float eps, cudaStream_t stream);
@@ -78,11 +83,6 @@ int llm_attention_decode(const void* q, void* out, float* part_o, float* part_ml
                          int table_stride, const int* items, const int* row_slot, const int* row_pos,
                          int n_items, int Hq, int Hkv, int hd, int page_size, float scale, int window,
                          int splits, cudaStream_t stream);
-int llm_attention_decode_tma(const void* q, void* out, float* part_o, float* part_ml, const void* storage,
-                             long long n_pages, int n_slots, int slot, const int* block_table,
-                             int table_stride, const int* items, const int* row_slot, const int* row_pos,
-                             int n_items, int Hq, int Hkv, int hd, int page_size, float scale, int window,
-                             int splits, int* status, cudaStream_t stream);
 int llm_attention_decode_persistent(const void* q, float* part_o, float* part_ml, const void* storage,
                                     long long n_pages, int n_slots, int slot, const int* block_table,
                                     int table_stride, const int* row_slot, const int* row_pos, int rows, int Hq,
@@ -678,13 +678,15 @@ struct Run {
     int rc = plan_for(group, (x2 ? 256 : tc ? 128 : 64) / group, &plan, merged);
     if (rc) return rc;
     const int reach = reach_of(window, st.max_pos);
-    if (plan->n_small) {
-      const bool tma = group <= 8 && decode_tma_ok(c, hd);
-      int splits = plan->small_single
-                       ? llm_decode_splits(plan->n_small, Hkv, reach, (tma ? DECODE_TMA_CTAS_PER_SM : 6) * sm_count(),
-                                           tma ? DECODE_TMA_TILE : 32)
-                       : 1;
-      if (merged && splits < 2) splits = 2;      // the sink and the outside part join in the merge
+    const bool tma = group <= 8 && decode_tma_ok(c, hd);
+    int splits = plan->small_single && plan->n_small
+                     ? llm_decode_splits(plan->n_small, Hkv, reach, (tma ? DECODE_TMA_CTAS_PER_SM : 6) * sm_count(),
+                                         tma ? DECODE_TMA_TILE : 32)
+                     : 1;
+    if (merged && splits < 2) splits = 2;      // the sink and the outside part join in the merge
+    // the short items: decoded tokens (beside: behind the prompt attention and at the same time)
+    auto short_items = [&](bool beside) -> int {
+      int rc;
       float *part_o, *part_ml;
       const int resident = DECODE_TMA_CTAS_PER_SM * sm_count();
       if (g_persistent_decode && !merged && tma && plan->small == nullptr && st.rows <= PERSISTENT_MAX_ROWS &&
@@ -704,10 +706,10 @@ struct Run {
       rc = parts(splits, L, &part_o, &part_ml);
       if (rc) return rc;
       if (tma)
-        rc = check(llm_attention_decode_tma(q, out, part_o, part_ml, c.storage, c.n_pages, c.n_slots, c.slot,
-                                            c.block_table, c.table_stride, plan->small, st.row_slot,
-                                            st.row_pos, plan->n_small, Hq, Hkv, hd, ps, L.scale, window,
-                                            splits, st.status, stream), K_DECODE_TMA);
+        rc = check(llm_attention_decode_tma_beside(q, out, part_o, part_ml, c.storage, c.n_pages, c.n_slots, c.slot,
+                                                   c.block_table, c.table_stride, plan->small, st.row_slot,
+                                                   st.row_pos, plan->n_small, Hq, Hkv, hd, ps, L.scale, window,
+                                                   splits, beside ? 1 : 0, st.status, stream), K_DECODE_TMA);
       else if (group <= 8)
         rc = check(llm_attention_decode(q, out, part_o, part_ml, c.k, c.v, c.page_stride, c.block_table,
                                         c.table_stride, plan->small, st.row_slot, st.row_pos, plan->n_small,
@@ -722,52 +724,69 @@ struct Run {
                                              splits, nullptr, 0, sink, extra_o, extra_ml, stream), K_MERGE);
         if (rc) return rc;
       }
-    }
-    if (plan->n_large && x2)
-      return check(llm_attention_tcgen05_x2(q, out, st.rows, c.k, c.v, c.page_stride, c.n_pages,
-                                            c.block_table, c.table_stride, plan->large, plan->n_large, Hq, Hkv,
-                                            hd, ps, L.scale, window, st.status, stream), K_TCGEN05_X2);
-    if (plan->n_large && tc) {
-      const int persistent = reach <= PERSISTENT_ATTENTION_MAX_KEYS ? 1 : 0;
-      const int* direct = plan->large;
-      int n_direct = plan->n_large;
-      if (g_gather && ps < 32 && GATHER_PAGE % ps == 0 && !plan->large_host.empty()) {
-        // pages too small for TMA boxes: long portions read gathered copies of their requests' keys
-        const GatherPlan* gp = nullptr;
-        rc = gather_for(*plan, ps, window, &gp);
-        if (rc) return rc;
-        if (gp->n_requests) {
-          const int D = GATHER_PAGE;
-          const long long stride = 2LL * Hkv * D * hd;
-          void* scratch = nullptr;
-          rc = buffer(B_GATHER, (size_t)gp->scratch_pages * stride * 2, &scratch);
+      return 0;
+    };
+    auto long_items = [&]() -> int {
+      if (plan->n_large && x2)
+        return check(llm_attention_tcgen05_x2(q, out, st.rows, c.k, c.v, c.page_stride, c.n_pages,
+                                              c.block_table, c.table_stride, plan->large, plan->n_large, Hq, Hkv,
+                                              hd, ps, L.scale, window, st.status, stream), K_TCGEN05_X2);
+      if (plan->n_large && tc) {
+        const int persistent = reach <= PERSISTENT_ATTENTION_MAX_KEYS ? 1 : 0;
+        const int* direct = plan->large;
+        int n_direct = plan->n_large;
+        if (g_gather && ps < 32 && GATHER_PAGE % ps == 0 && !plan->large_host.empty()) {
+          // pages too small for TMA boxes: long portions read gathered copies of their requests' keys
+          const GatherPlan* gp = nullptr;
+          int rc = gather_for(*plan, ps, window, &gp);
           if (rc) return rc;
-          bf16* ks = (bf16*)scratch;
-          bf16* vs = ks + (size_t)Hkv * D * hd;
-          rc = check(llm_kv_gather(c.k, c.v, c.page_stride, c.block_table, c.table_stride, ps, ks, vs, stride, D,
-                                   Hkv, hd, LLM_BF16, gp->list, gp->n_requests, gp->total_chunks, stream),
-                     K_KV_GATHER);
-          if (rc) return rc;
-          rc = check(llm_attention_tcgen05_extra(q, out, st.rows, ks, vs, stride, gp->scratch_pages, gp->table,
-                                                 gp->table_stride, gp->gathered, gp->n_gathered, Hq, Hkv, hd, D,
-                                                 L.scale, window, persistent, st.status, sink, extra_o, extra_ml,
-                                                 stream), K_TCGEN05);
-          if (rc) return rc;
-          direct = gp->direct;
-          n_direct = gp->n_direct;
+          if (gp->n_requests) {
+            const int D = GATHER_PAGE;
+            const long long stride = 2LL * Hkv * D * hd;
+            void* scratch = nullptr;
+            rc = buffer(B_GATHER, (size_t)gp->scratch_pages * stride * 2, &scratch);
+            if (rc) return rc;
+            bf16* ks = (bf16*)scratch;
+            bf16* vs = ks + (size_t)Hkv * D * hd;
+            rc = check(llm_kv_gather(c.k, c.v, c.page_stride, c.block_table, c.table_stride, ps, ks, vs, stride, D,
+                                     Hkv, hd, LLM_BF16, gp->list, gp->n_requests, gp->total_chunks, stream),
+                       K_KV_GATHER);
+            if (rc) return rc;
+            rc = check(llm_attention_tcgen05_extra(q, out, st.rows, ks, vs, stride, gp->scratch_pages, gp->table,
+                                                   gp->table_stride, gp->gathered, gp->n_gathered, Hq, Hkv, hd, D,
+                                                   L.scale, window, persistent, st.status, sink, extra_o, extra_ml,
+                                                   stream), K_TCGEN05);
+            if (rc) return rc;
+            direct = gp->direct;
+            n_direct = gp->n_direct;
+          }
         }
+        if (n_direct == 0) return 0;
+        return check(llm_attention_tcgen05_extra(q, out, st.rows, c.k, c.v, c.page_stride,
+                                                 c.storage != nullptr ? c.n_pages : 0, c.block_table, c.table_stride,
+                                                 direct, n_direct, Hq, Hkv, hd, ps, L.scale, window, persistent,
+                                                 st.status, sink, extra_o, extra_ml, stream), K_TCGEN05);
       }
-      if (n_direct == 0) return 0;
-      return check(llm_attention_tcgen05_extra(q, out, st.rows, c.k, c.v, c.page_stride,
-                                               c.storage != nullptr ? c.n_pages : 0, c.block_table, c.table_stride,
-                                               direct, n_direct, Hq, Hkv, hd, ps, L.scale, window, persistent,
-                                               st.status, sink, extra_o, extra_ml, stream), K_TCGEN05);
+      if (plan->n_large)
+        return check(llm_attention_flash(q, out, nullptr, nullptr, c.k, c.v, c.page_stride, c.block_table,
+                                         c.table_stride, plan->large, nullptr, nullptr, plan->n_large, 64, Hq,
+                                         Hkv, hd, ps, L.scale, window, 1, stream), K_FLASH);
+      return 0;
+    };
+    // Decoded tokens beside portions of prompts: the prompt attention of a small step leaves SMs idle (a
+    // CTA has an SM to itself: 13 items of 64 tokens on 8 KV heads are 104 of them), and decode attention
+    // does not depend on it, so it comes second and starts beside it.  Only with a merge behind it, which
+    // keeps a kernel between these CTAs and the product on CTA pairs.  (28 layers of Qwen3-0.6B sizes, 24
+    // tokens at 450 to 1,350 keys beside 753 rows of four portions: 3,083 -> 2,895 us a step.)
+    if (plan->n_small && plan->n_large && tc && !x2 && tma && splits > 1) {
+      rc = long_items();
+      return rc ? rc : short_items(true);
     }
-    if (plan->n_large)
-      return check(llm_attention_flash(q, out, nullptr, nullptr, c.k, c.v, c.page_stride, c.block_table,
-                                       c.table_stride, plan->large, nullptr, nullptr, plan->n_large, 64, Hq,
-                                       Hkv, hd, ps, L.scale, window, 1, stream), K_FLASH);
-    return 0;
+    if (plan->n_small) {
+      rc = short_items(false);
+      if (rc) return rc;
+    }
+    return long_items();
   }
 
   // the mixer: projections, per-head norm, rotation, cache write, attention, output projection
