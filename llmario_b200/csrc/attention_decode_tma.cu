@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(32, 4) flash_decode_tma_kernel(
   // read here and lets this kernel start only when its own wait is over, so that everything before it
   // is complete.  This kernel then runs beside it and waits for its end at its own end instead: what
   // comes next may rely on both.
-  if (!beside) pdl_wait();
+  if (FUSED || !beside) pdl_wait();
   for (int i = early; i < STAGES && tb0 + i < tb1; ++i) load_tile(tb0 + i, i);
 
   int cpos[2], clo[2];
@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(32, 4) flash_decode_tma_kernel(
   }
   if (!alive) {   // let the loads that are still in flight land before the shared memory goes
     for (int i = 0; i < STAGES; ++i) mbar_wait(&full[i], 0), mbar_wait(&full[i], 1);
-    if (beside) pdl_wait();
+    if (!FUSED && beside) pdl_wait();
     return;
   }
 
@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(32, 4) flash_decode_tma_kernel(
       }
     }
   }
-  if (beside) pdl_wait();
+  if (!FUSED && beside) pdl_wait();
 }
 
 // ---------------------------------------------------------------------------------------------
