@@ -149,3 +149,25 @@ static inline int launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
   cfg.numAttrs = g_llm_pdl && !plain ? 1 : 0;
   return (int)cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
+
+// The walk of a thread over [rows][n4] pieces of four columns, a stride of the whole grid at a time:
+// f(piece, column piece).  The column is carried along: the remainder of a 64-bit index by a width that
+// is known at run time costs more than a pass over 32-bit values has time for.
+template <typename F>
+__device__ __forceinline__ void for_each_piece(unsigned total4, unsigned n4, F f) {
+  const unsigned stride = gridDim.x * blockDim.x, wrap = stride % n4;
+  unsigned i = blockIdx.x * blockDim.x + threadIdx.x, c = i % n4;
+  for (; i < total4; i += stride) {
+    f(i, c);
+    c += wrap;
+    if (c >= n4) c -= n4;
+  }
+}
+// whether a contiguous matrix of `total` values, n to a row, goes by pieces of four
+static inline bool in_pieces(long long total, int n, const void* a, const void* b) {
+  return n % 4 == 0 && (((uintptr_t)a | (uintptr_t)b) & 15) == 0 && total / 4 < (1LL << 31);
+}
+static inline int piece_blocks(long long total) {
+  const long long want = (total / 4 + 255) / 256;
+  return (int)(want < 148 * 8 ? want : 148 * 8);
+}

@@ -800,6 +800,35 @@ __global__ void rate_decay_kernel(float* __restrict__ z, const float* __restrict
   }
 }
 
+// The same two by pieces of four columns (of one group in the second: `per` a multiple of four).  1,501
+// rows of 4,096: the second 31 -> 17 us.
+__global__ void __launch_bounds__(256) bias_sigmoid_pow_vec_kernel(float4* __restrict__ z, const float4* __restrict__ b,
+                                                                   unsigned total4, unsigned n4, float c) {
+  pdl_trigger();
+  pdl_wait();
+  for_each_piece(total4, n4, [&](unsigned i, unsigned col) {
+    float4 v = z[i];
+    const float4 w = b ? __ldg(b + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+    v.x = expf(-c * softplus_f(-(v.x + w.x))), v.y = expf(-c * softplus_f(-(v.y + w.y)));
+    v.z = expf(-c * softplus_f(-(v.z + w.z))), v.w = expf(-c * softplus_f(-(v.w + w.w)));
+    z[i] = v;
+  });
+}
+__global__ void __launch_bounds__(256) rate_decay_vec_kernel(float4* __restrict__ z, const float* __restrict__ rate_log,
+                                                             const float4* __restrict__ b, unsigned total4, unsigned n4,
+                                                             unsigned per4) {
+  pdl_trigger();
+  pdl_wait();
+  for_each_piece(total4, n4, [&](unsigned i, unsigned col) {
+    float4 v = z[i];
+    const float4 w = b ? __ldg(b + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float rate = -expf(__ldg(rate_log + col / per4));
+    v.x = expf(rate * softplus_f(v.x + w.x)), v.y = expf(rate * softplus_f(v.y + w.y));
+    v.z = expf(rate * softplus_f(v.z + w.z)), v.w = expf(rate * softplus_f(v.w + w.w));
+    z[i] = v;
+  });
+}
+
 // ---- short causal convolution per channel, bias, silu
 // out[r][c] = silu(b[c] + sum_{j < taps} w[c][taps - 1 - j] * in(r, j, c)); in(r, j, c) is the input
 // of channel c, j tokens before row r: a row of this step when the request has that many rows in
@@ -1644,6 +1673,9 @@ LLM_EXPORT int llm_rate_decay(float* z, const float* rate_log, const float* bias
   const long long total = (long long)rows * n;
   if (total <= 0) return 0;
   if (per <= 0 || !rate_log) return LLM_ERR_ARGUMENT;
+  if (per % 4 == 0 && in_pieces(total, n, z, bias))
+    return launch_pdl(rate_decay_vec_kernel, piece_blocks(total), 256, 0, stream, (float4*)z, rate_log, (const float4*)bias,
+                      (unsigned)(total / 4), (unsigned)(n / 4), (unsigned)(per / 4));
   const int blocks = (int)((total + 255) / 256 < 2368 ? (total + 255) / 256 : 2368);
   return launch_pdl(rate_decay_kernel, blocks, 256, 0, stream, z, rate_log, bias, total, n, per);
 }
@@ -1651,6 +1683,9 @@ LLM_EXPORT int llm_rate_decay(float* z, const float* rate_log, const float* bias
 LLM_EXPORT int llm_bias_sigmoid_pow(float* z, const float* b, int rows, int n, float c, cudaStream_t stream) {
   const long long total = (long long)rows * n;
   if (total <= 0) return 0;
+  if (in_pieces(total, n, z, b))
+    return launch_pdl(bias_sigmoid_pow_vec_kernel, piece_blocks(total), 256, 0, stream, (float4*)z, (const float4*)b,
+                      (unsigned)(total / 4), (unsigned)(n / 4), c);
   const int blocks = (int)((total + 255) / 256 < 2368 ? (total + 255) / 256 : 2368);
   return launch_pdl(bias_sigmoid_pow_kernel, blocks, 256, 0, stream, z, b, total, n, c);
 }
