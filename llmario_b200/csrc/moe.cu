@@ -157,14 +157,26 @@ __global__ void __launch_bounds__(256) moe_router_kernel(const T* __restrict__ h
   const int r0 = blockIdx.x * R, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   const bool wide = (width & 3) == 0 && ((uintptr_t)w & 15) == 0;
   if (sizeof(T) == 2 && (width & 7) == 0 && ((uintptr_t)h & 15) == 0) {
-    for (int i = threadIdx.x * 8; i < R * width; i += blockDim.x * 8) {     // (a piece stays inside its row)
-      const uint4 u = r0 + i / width < rows ? *reinterpret_cast<const uint4*>(h + (size_t)r0 * width + i)
-                                            : make_uint4(0, 0, 0, 0);
-      float4* dst = reinterpret_cast<float4*>(h_s + i);
-      dst[0] = make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
-                           __uint_as_float(u.y & 0xffff0000u));
-      dst[1] = make_float4(__uint_as_float(u.z << 16), __uint_as_float(u.z & 0xffff0000u), __uint_as_float(u.w << 16),
-                           __uint_as_float(u.w & 0xffff0000u));
+    // (the block's rows lie one behind the other: those that exist end at `there`; four pieces are in
+    // flight before the first is put down: 1,501 rows of 4,096 with eight experts 22 -> 19 us)
+    const int there = min(R, rows - r0) * width;
+    for (int i0 = threadIdx.x * 8; i0 < R * width; i0 += 4 * blockDim.x * 8) {
+      uint4 u[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int i = i0 + j * blockDim.x * 8;
+        u[j] = i < there ? *reinterpret_cast<const uint4*>(h + (size_t)r0 * width + i) : make_uint4(0, 0, 0, 0);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int i = i0 + j * blockDim.x * 8;
+        if (i >= R * width) break;
+        float4* dst = reinterpret_cast<float4*>(h_s + i);
+        dst[0] = make_float4(__uint_as_float(u[j].x << 16), __uint_as_float(u[j].x & 0xffff0000u),
+                             __uint_as_float(u[j].y << 16), __uint_as_float(u[j].y & 0xffff0000u));
+        dst[1] = make_float4(__uint_as_float(u[j].z << 16), __uint_as_float(u[j].z & 0xffff0000u),
+                             __uint_as_float(u[j].w << 16), __uint_as_float(u[j].w & 0xffff0000u));
+      }
     }
   } else
   for (int i = threadIdx.x; i < R * width; i += blockDim.x) {
@@ -178,9 +190,9 @@ __global__ void __launch_bounds__(256) moe_router_kernel(const T* __restrict__ h
 #pragma unroll
     for (int rr = 0; rr < R; ++rr) acc[rr] = 0.f;
     if (wide) {
-#pragma unroll 4
+#pragma unroll 8
       for (int i = lane * 4; i < width; i += 128) {
-        const float4 a = *reinterpret_cast<const float4*>(we + i);
+        const float4 a = __ldg(reinterpret_cast<const float4*>(we + i));
 #pragma unroll
         for (int rr = 0; rr < R; ++rr) {
           const float4 x = *reinterpret_cast<const float4*>(h_s + (size_t)rr * width + i);
