@@ -274,25 +274,44 @@ __global__ void merge_kernel(const float* __restrict__ part_o, const float* __re
   if (clear)      // the head's queries in the projection buffer, which every part has read by now
     for (int d = threadIdx.x; d < HD; d += blockDim.x)
       clear[(size_t)row * clear_stride + blockIdx.y * HD + d] = 0.f;
+  // The loads of eight parts are in flight together, those of the first eight before anything is asked of
+  // them: with a load behind the question whether its part has keys, each part cost the way to the L2
+  // and back.
+  constexpr int AHEAD = 8;
+  float mz[AHEAD], lz[AHEAD], v[AHEAD];
+  auto ask = [&](int z0, int d) {
+#pragma unroll
+    for (int j = 0; j < AHEAD; ++j)
+      if (z0 + j < splits) {
+        const size_t part = rowhead * splits + z0 + j;
+        mz[j] = part_ml[part * 2], lz[j] = part_ml[part * 2 + 1], v[j] = part_o[part * HD + d];
+      }
+  };
+  ask(0, threadIdx.x);      // (HD threads)
   // (the parts' maxima are base-2 logarithms: scores times scale times log2 e)
   const float sk = sink ? sink[blockIdx.y] * 1.4426950408889634f : -INFINITY;
   float mstar = sk;
+#pragma unroll 8
   for (int z = 0; z < splits; ++z) mstar = fmaxf(mstar, part_ml[(rowhead * splits + z) * 2]);
   const float me = extra_ml ? extra_ml[rowhead * 2] : -INFINITY;
   mstar = fmaxf(mstar, me);
-  for (int d = threadIdx.x; d < HD; d += blockDim.x) {
+  {
+    const int d = threadIdx.x;
     float acc = 0.f, lsum = sink ? exp2f(sk - mstar) : 0.f;
     if (me != -INFINITY) {
       const float w = exp2f(me - mstar);
       acc = w * extra_o[rowhead * HD + d];
       lsum += w * extra_ml[rowhead * 2 + 1];
     }
-    for (int z = 0; z < splits; ++z) {
-      const float mz = part_ml[(rowhead * splits + z) * 2];
-      if (mz == -INFINITY) continue;      // a part without keys: what lies in its place is not read
-      const float w = exp2f(mz - mstar);
-      acc += w * part_o[(rowhead * splits + z) * HD + d];
-      lsum += w * part_ml[(rowhead * splits + z) * 2 + 1];
+    for (int z0 = 0; z0 < splits; z0 += AHEAD) {
+      if (z0 > 0) ask(z0, d);
+#pragma unroll
+      for (int j = 0; j < AHEAD; ++j)
+        if (z0 + j < splits && mz[j] != -INFINITY) {      // (a part without keys: what lies in its place is not used)
+          const float w = exp2f(mz[j] - mstar);
+          acc += w * v[j];
+          lsum += w * lz[j];
+        }
     }
     out[rowhead * HD + d] = __float2bfloat16_rn(acc / lsum);
   }
